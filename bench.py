@@ -673,9 +673,8 @@ def gam3_section(neoxc, kw=None):
 
 
 def gam2_section(neoxc, small=False):
-    """The gam_2 build (GM2ICR / GM2sICR, k_md.cu) in FP64 and in the mixed
-    precision (FP32 tables, FP64 Boys function, seeds and sums, items above
-    the recompute threshold re-evaluated in FP64), timed as a one-iteration
+    """The gam_2 build (GM2ICR / GM2sICR, k_gam2.cu; FP64 with and without the
+    mixed-precision option, which gam_2 accepts), timed as a one-iteration
     XCHF SCF of a two-electron system (no gam_3: the gam_2 build dominates;
     the one-body, GAM_1 and GAM_ee builds and one Fock build are included).
     System: the first configuration's seeded basis with 2 electrons, or with

@@ -417,9 +417,8 @@ int neoxc_dev_gam4_fock_factored_tc(void* stream, int64_t ne, int64_t np,
  * NEOXC_SCF_MIXED (no reference counterpart) evaluates the gam_3 primitive
  * integrals with FP32 McMurchie-Davidson recursions (FP64 Boys function,
  * FP64 sums over primitives and geminal pairs); everything else stays FP64.
- * NEOXC_SCF_MIXED_GAM2 does the same for the gam_2 primitive items, with
- * dynamic precision: an item whose FP32 contribution exceeds the threshold
- * of neoxc_set_mixed_threshold is re-evaluated in FP64 (gam_1 is FP64).
+ * NEOXC_SCF_MIXED_GAM2 is accepted and changes nothing: the gam_2 build is
+ * FP64 (faster than its earlier FP32-first form; gam_1 is FP64 as well).
  *   DE (in: initial electronic density, e.g. from guessCE; out: converged)
  *   DP (in: initial nuclear density unless NEOXC_SCF_GUESS_PROT; out)
  *   E_init[16], E_final[16]: energy slots 0 E_total 1 E_nuc 2 E_ecore
@@ -434,8 +433,7 @@ int neoxc_dev_gam4_fock_factored_tc(void* stream, int64_t ne, int64_t np,
 #define NEOXC_SCF_DIIS 2           /* Pulay DIIS on the electronic Fock (new) */
 #define NEOXC_SCF_GAM4_ELEMENT 4   /* element-wise GAM4_DSCF for gam_4     */
 #define NEOXC_SCF_MIXED 8          /* gam_3 MD integrals in FP32 (new)     */
-#define NEOXC_SCF_MIXED_GAM2 16    /* gam_2 MD integrals in FP32, the large
-                                      items in FP64 (new) */
+#define NEOXC_SCF_MIXED_GAM2 16    /* accepted; gam_2 is FP64 either way (new) */
 #define NEOXC_SCF_GUESS_ELEC 32    /* DE (XCHF: guess_elec, xcscf.f:660) or
                                       DAE, DBE (XCUHF: guess_A_elec) from the
                                       electronic core Hamiltonian */
@@ -460,14 +458,10 @@ int neoxc_xchf_scf(int64_t nelec, int64_t nucst, int64_t nebf, int64_t npebf,
                    double* E_final, double* history, int64_t* niter,
                    int64_t* converged);
 
-/* Dynamic-precision threshold of the mixed gam_2 build (NEOXC_SCF_MIXED_GAM2
- * in every entry point that takes it; no reference counterpart).  Each
- * primitive item is first evaluated with the FP32 tables (FP64 Boys
- * function, seeds and sums); an item whose contribution to a contracted
- * gam_2 element exceeds tau in magnitude is re-evaluated entirely in FP64.
- * tau = 0 re-evaluates every item, INFINITY none.  Default 1e-5.
- * Process-wide; NEOXC_ERR_ARG for tau < 0 or NaN.  neoxc_get_mixed_threshold
- * returns the current value. */
+/* Threshold of the former dynamic-precision gam_2 build (no reference
+ * counterpart): the contribution above which an item had to be FP64.  Every
+ * item is FP64 now, so any value is satisfied; it is checked, kept and read
+ * back.  Default 1e-5.  Process-wide; NEOXC_ERR_ARG for tau < 0 or NaN. */
 int neoxc_set_mixed_threshold(double tau);
 double neoxc_get_mixed_threshold(void);
 

@@ -283,11 +283,22 @@ int stage_system(SysUpload& u, cudaStream_t s, int64_t nebf, int64_t npebf,
     RC(upload(u.g3i, g3i.data(), sizeof(int) * g3i.size(), s));
     u.d.g3_nket = nket;
     u.d.g3_ntile = ok ? ntile : 0;
+    u.d.g3_ntile_all = ntile;
+    u.d.g3_max_prim = 0;
+    for (int P = 0; P < nPe; P++) u.d.g3_max_prim = std::max(u.d.g3_max_prim, kofs[P + 1] - kofs[P]);
     u.d.g3i = u.g3i.as<int>();
     RC(dalloc(u.g3rec, sizeof(double) * g3_record_doubles(nket, (int)npbf), s));
     u.d.g3rec = u.g3rec.as<double>();
     CU(launch_g3_records(u.d, const_cast<double*>(u.d.g3rec), s));
   }
+  return NEOXC_OK;
+}
+
+// Both gam_2 tensors of a staged system, with the build's scratch.
+int build_gam2(const DevSystem& d, int rx, double* x1, double* x2, cudaStream_t s) {
+  DBuf scr;
+  RC(dalloc(scr, sizeof(double) * gam2_scratch_doubles(d, rx, d.npbf * (d.npbf + 1) / 2), s));
+  CU(launch_gam2_build(d, rx, scr.as<double>(), x1, x2, s));
   return NEOXC_OK;
 }
 
@@ -446,9 +457,7 @@ static int gam2_common(int rx, int64_t nebf, int64_t npebf, int64_t npbf,
   DBuf d1, d2;
   RC(dalloc(d1, sizeof(double) * ng2, s));
   RC(dalloc(d2, sizeof(double) * ng2, s));
-  CU(launch_gam2_raw(u.d, rx, d1.as<double>(), d2.as<double>(), s));
-  CU(launch_gam2_symmetrize((int)nebf, (int)npbf, rx, d1.as<double>(),
-                            d2.as<double>(), s));
+  RC(build_gam2(u.d, rx, d1.as<double>(), d2.as<double>(), s));
   CU(cudaMemcpyAsync(out1, d1.p, sizeof(double) * ng2, cudaMemcpyDeviceToHost, s));
   CU(cudaMemcpyAsync(out2, d2.p, sizeof(double) * ng2, cudaMemcpyDeviceToHost, s));
   return finish(s);
@@ -706,13 +715,17 @@ int neoxc_gam3_ic1_batch(const neoxc_xchf_job* jobs, int64_t njobs, int64_t opti
   return rc;
 }
 
+// Kept and read back only: the gam_2 build is FP64 throughout, so no item
+// falls below the threshold's precision whatever its value.
+static std::atomic<double> g_mixed_tau{1.0e-5};
+
 int neoxc_set_mixed_threshold(double tau) {
   if (!(tau >= 0.0)) return set_err(NEOXC_ERR_ARG, "mixed threshold: tau >= 0");
-  set_mixed_recompute_tau(tau);
+  g_mixed_tau.store(tau);
   return NEOXC_OK;
 }
 
-double neoxc_get_mixed_threshold(void) { return mixed_recompute_tau(); }
+double neoxc_get_mixed_threshold(void) { return g_mixed_tau.load(); }
 
 int64_t neoxc_gam3_batch_tuning(char* buf, int64_t len) {
   std::string out = "[";
@@ -1245,13 +1258,20 @@ static int gam2_dscf_dev(const SysUpload& u, cudaStream_t s, const double* dde,
   double* pv = part.as<double>();
   double* ps = pv + npart;
   double* ftmp = ps + npart;
-  for (int64_t pp = 0; pp < (int64_t)np * np; pp++) {
-    CU(launch_gam2_raw_range(u.d, 0, pp * n4, n4, s1.as<double>(),
-                             s2.as<double>(), s));
-    CU(launch_gam2_symmetrize(ne, 1, 0, s1.as<double>(), s2.as<double>(), s));
-    CU(launch_eg2_partials(ne, np, pp, 1, dde, s1.as<double>(),
-                           s2.as<double>(), pv, ps, s));
-  }
+  // the slices of (ip,jp) and (jp,ip) are the same: build it once
+  DBuf scr;
+  RC(dalloc(scr, sizeof(double) * gam2_scratch_doubles(u.d, 0, 1), s));
+  CU(launch_gam2_prepare(u.d, scr.as<double>(), s));
+  for (int ip = 0; ip < np; ip++)
+    for (int jp = 0; jp <= ip; jp++) {
+      CU(launch_gam2_slice(u.d, ip * (ip + 1) / 2 + jp, scr.as<double>(), s1.as<double>(),
+                           s2.as<double>(), s));
+      CU(launch_eg2_partials(ne, np, (int64_t)ip * np + jp, 1, dde, s1.as<double>(),
+                             s2.as<double>(), pv, ps, s));
+      if (ip != jp)
+        CU(launch_eg2_partials(ne, np, (int64_t)jp * np + ip, 1, dde, s1.as<double>(),
+                               s2.as<double>(), pv, ps, s));
+    }
   CU(launch_fock_reduce(ne, np, ne, pv, dde, ddp, 2.0, 1, dfe, dfp, ftmp, dE, s));
   CU(launch_fock_reduce(ne, np, ne, ps, dde, ddp, 1.0, 1, dse, dsp,
                         ftmp + np * np, dS, s));
@@ -1691,7 +1711,6 @@ static int xchf_scf_on(cudaStream_t s, int64_t nelec, int64_t nucst, int64_t neb
   RC(need(!((options & NEOXC_SCF_SOSCF) && (options & NEOXC_SCF_DIIS)),
           "NEOXC_SCF_SOSCF and NEOXC_SCF_DIIS are exclusive"));
   const int mixed = (options & NEOXC_SCF_MIXED) ? 1 : 0;
-  const int mixed_gam2 = (options & NEOXC_SCF_MIXED_GAM2) ? 1 : 0;
   if (nebf > kScfMaxN || npbf > kScfMaxN)
     return set_err(NEOXC_ERR_UNSUPPORTED, "XCHF SCF: nebf, npbf <= %d", kScfMaxN);
   const bool elem4 = (options & NEOXC_SCF_GAM4_ELEMENT) != 0;
@@ -1726,9 +1745,7 @@ static int xchf_scf_on(cudaStream_t s, int64_t nelec, int64_t nucst, int64_t neb
   CU(launch_gam1(u.d, G1.as<double>(), G1s.as<double>(), s, 0));
   CU(launch_gam_ee(u.d, Gee.as<double>(), s));
   if (nelec > 1) {
-    CU(launch_gam2_raw(u.d, 0, G2.as<double>(), G2s.as<double>(), s,
-                       mixed_gam2));
-    CU(launch_gam2_symmetrize(ne, np, 0, G2.as<double>(), G2s.as<double>(), s));
+    RC(build_gam2(u.d, 0, G2.as<double>(), G2s.as<double>(), s));
   }
   if (nelec > 2) {
     DBuf aux;
@@ -1943,7 +1960,24 @@ static size_t xchf_job_bytes(const neoxc_xchf_job& j, int64_t options) {
   const size_t ne = (size_t)j.nebf, np = (size_t)j.npbf;
   const size_t e2 = ne * ne, p2 = np * np;
   size_t d = 4 * e2 + 4 * p2 + 3 * e2 * p2 + e2 * e2 + 32 * (e2 + p2);
-  if (j.nelec > 1) d += 2 * e2 * e2 * p2 + eg2_partial_doubles((int)ne, (int)np);
+  if (j.nelec > 1) {
+    d += 2 * e2 * e2 * p2 + eg2_partial_doubles((int)ne, (int)np);
+    // the gam_2 build's scratch: primitive pairs of the canonical pairs
+    // (a range that stage_system will refuse counts as one primitive)
+    int64_t nket = 0, most = 1;
+    auto prims = [&](int64_t i) -> int64_t {
+      if (!j.KPESTR || !j.KPEEND) return 1;
+      const int64_t a = j.KPESTR[i], b = j.KPEEND[i];
+      return a >= 1 && b >= a && b <= j.npebf ? b - a + 1 : 1;
+    };
+    for (int64_t i = 0; i < j.nebf; i++)
+      for (int64_t k = 0; k <= i; k++) {
+        const int64_t n = prims(i) * prims(k);
+        nket += n;
+        most = std::max(most, n);
+      }
+    d += gam2_scratch_bound((int)ne, (int)np, (int)nket, (int)most, (int)j.ngtg1);
+  }
   if (j.nelec > 2) {
     d += e2 * e2 * e2 * p2 + gam3_aux_doubles((int)ne, (int)np) +
          eg3_partial_doubles((int)ne, (int)np);
@@ -2714,7 +2748,6 @@ int xcuhf_scf_on(cudaStream_t s, int64_t nelec, int64_t NAE, int64_t NBE, int64_
   if (nelec > 3 && !spin_smem_fits(4, (int)nebf))
     return set_err(NEOXC_ERR_UNSUPPORTED, "XCUHF SCF with OMG4: nebf <= 12");
   const int mixed = (options & NEOXC_SCF_MIXED) ? 1 : 0;
-  const int mixed_gam2 = (options & NEOXC_SCF_MIXED_GAM2) ? 1 : 0;
   const bool diis = (options & NEOXC_SCF_DIIS) != 0;
   SysUpload u;
   RC(stage_system(u, s, nebf, npebf, npbf, nat, ngtg1, pmass, cat, zan, bcoef1, gamma1,
@@ -2745,8 +2778,7 @@ int xcuhf_scf_on(cudaStream_t s, int64_t nelec, int64_t NAE, int64_t NBE, int64_
   CU(launch_gam1(u.d, G1.as<double>(), G1s.as<double>(), s, 0));
   CU(launch_gam_ee(u.d, Gee.as<double>(), s));
   if (nelec > 1) {
-    CU(launch_gam2_raw(u.d, 0, G2.as<double>(), G2s.as<double>(), s, mixed_gam2));
-    CU(launch_gam2_symmetrize(ne, np, 0, G2.as<double>(), G2s.as<double>(), s));
+    RC(build_gam2(u.d, 0, G2.as<double>(), G2s.as<double>(), s));
   }
   if (nelec > 2) {
     DBuf aux;
@@ -3026,8 +3058,7 @@ int rx_scf_on(cudaStream_t s, int64_t kind, int64_t NAE, int64_t NAalpE, int64_t
                         Hcp.as<double>(), s));
   CU(launch_gam1(u.d, G1.as<double>(), G1s.as<double>(), s, 0, 1));
   CU(launch_gam_ee(u.d, Gee.as<double>(), s));
-  CU(launch_gam2_raw(u.d, 1, G2.as<double>(), G2x.as<double>(), s));
-  CU(launch_gam2_symmetrize(ne, np, 1, G2.as<double>(), G2x.as<double>(), s));
+  RC(build_gam2(u.d, 1, G2.as<double>(), G2x.as<double>(), s));
   // SCF state
   DBuf dA, dB, dBE, dP, A0, B0, BE0, P0, CA, CBE, Ctmp, FA, FB, FP, FBE, ocb, en, info, st;
   for (DBuf* b : {&dA, &dB, &dBE, &A0, &B0, &BE0, &CA, &CBE, &Ctmp, &FA, &FB, &FBE})

@@ -36,7 +36,9 @@ struct DevSystem {
   // canonical order), kofs[nPe+1], tile_k[ntile+1], tile_P[ntile+1],
   // kperm[nket] (kets of each tile ordered by angular class); g3rec the
   // FP64 pair records of the kets and of the canonical nuclear pairs.
-  int g3_nket, g3_ntile;
+  // g3_ntile is 0 when a contracted pair has more primitive pairs than a tile
+  // holds (g3_max_prim of them); g3_ntile_all counts the tables' tiles anyway.
+  int g3_nket, g3_ntile, g3_ntile_all, g3_max_prim;
   const int* g3i;
   const double* g3rec;
 };
@@ -186,10 +188,19 @@ cudaError_t launch_eg2_partials(int ne, int np, long long ipjp0,
 
 // ---- integral builders (MD kernels) ------------------------------------
 cudaError_t launch_gam_ee(const DevSystem& sys, double* gee, cudaStream_t s);
-// tuples [t0, t0+ntup) of the packed index space, written from x[0]
-cudaError_t launch_gam2_raw_range(const DevSystem& sys, int rx, long long t0,
-                                  long long ntup, double* x1, double* x2,
-                                  cudaStream_t s, int fp32 = 0);
+// The symmetrised gam_2 tensors (k_gam2.cu), packed index_GAM_2PK: rx = 0
+// GM2ICR / GM2sICR, rx = 1 (RXCHF-ne) GM2ICR / GM2exICR.  scratch:
+// gam2_scratch_doubles of the same system (nPp_want = npbf(npbf+1)/2).
+size_t gam2_scratch_doubles(const DevSystem& sys, int rx, int nPp_want);
+// an upper bound of it from the sizes alone (rx = 0)
+size_t gam2_scratch_bound(int ne, int np, int nket, int max_prim, int ng);
+cudaError_t launch_gam2_build(const DevSystem& sys, int rx, double* scratch, double* x1,
+                              double* x2, cudaStream_t s);
+// The same for one canonical proton pair Pp = ip(ip+1)/2 + jp at a time (XCHF):
+// launch_gam2_prepare once, then slices of nebf^4; scratch sized with nPp_want = 1.
+cudaError_t launch_gam2_prepare(const DevSystem& sys, double* scratch, cudaStream_t s);
+cudaError_t launch_gam2_slice(const DevSystem& sys, int Pp, double* scratch, double* x1,
+                              double* x2, cudaStream_t s);
 // gam_3 raw tensor = W1(p,e1) GAM_ee(e2,e3) + W3(p,e1,e2) Hcore(e3) + R4,
 // R4 the contracted primitive sum of the four-particle terms, stored once
 // per pair-canonical tuple (k_gam3.cu).  aux (gam3_aux_doubles) holds
@@ -215,16 +226,6 @@ size_t g3_record_doubles(int nket, int np);
 cudaError_t launch_g3_records(const DevSystem& sys, double* rec, cudaStream_t s);
 constexpr int kG3MaxTileKets = 1024;
 constexpr double kScreenThreshold = 1.0e-12;   // NEOXC_SCF_SCREEN
-cudaError_t launch_gam2_raw(const DevSystem& sys, int rxchfne, double* x1,
-                            double* x2, cudaStream_t s, int fp32 = 0);
-// Dynamic precision of the mixed gam_2 build (process-wide): a primitive
-// item whose FP32 contribution to a contracted element exceeds this
-// magnitude is re-evaluated in FP64.
-constexpr double kMixedTauGam2 = 1.0e-5;
-void set_mixed_recompute_tau(double tau);
-double mixed_recompute_tau();
-cudaError_t launch_gam2_symmetrize(int ne, int np, int rxchfne, double* x1,
-                                   double* x2, cudaStream_t s);
 // Many systems of one angular class in one persistent launch: both passes of
 // the four-particle terms of every system go through one device work queue
 // (an atomic counter over items numbered system by system), each CTA taking

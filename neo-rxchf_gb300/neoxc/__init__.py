@@ -458,9 +458,8 @@ def xchf_scf(s: NeoSystem, DE, DP=None, nucst=None, maxit: int = 100,
     """xcscf.f XCHF RHF SCF on the GPU (plain Roothaan, or DIIS).  DE: initial
     electronic density, or None for the core-Hamiltonian guess (guess_elec);
     DP: initial nuclear density, or None for the core-Hamiltonian guess
-    (guess_prot).  mixed: False (all FP64), "gam3" (FP32 MD integrals for
-    gam_3), "gam2" (FP32 for gam_2, its large items in FP64: see
-    set_mixed_threshold), True (both).
+    (guess_prot).  mixed: False (all FP64), "gam3" or True (FP32 MD integrals
+    for gam_3), "gam2" (as False: gam_2 is FP64 in every mode).
     screen: skip gam_3 primitive (bra, ket) pairs whose Schwarz-type
     estimate is below 1e-12 (NEOXC_SCF_SCREEN).  soscf: the reference's
     second-order steps on the electronic orbitals (NEOXC_SCF_SOSCF; not with
@@ -555,8 +554,8 @@ def gam3_ic1_batch(systems, mixed: bool = False, screen: bool = False):
 
 
 def set_mixed_threshold(tau: float) -> None:
-    """neoxc_set_mixed_threshold: the contribution magnitude above which a
-    mixed gam_2 primitive item is re-evaluated in FP64 (0: all, inf: none)."""
+    """neoxc_set_mixed_threshold: the threshold of the former FP32-first gam_2
+    build, kept and read back (every gam_2 item is FP64)."""
     _check(lib().neoxc_set_mixed_threshold(float(tau)))
 
 
