@@ -1189,16 +1189,14 @@ static int gam3_dscf_dev(const SysUpload& u, cudaStream_t s, const double* dde,
   RC(dalloc(aux, sizeof(double) * gam3_aux_doubles(ne, np), s));
   CU(launch_gam3_aux(u.d, aux.as<double>(), s));
   CU(launch_gam3_pairs(u.d, aux.as<double>(), s, 0, 0.0));
+  CU(launch_eg3_weights(ne, dde, part.as<double>(), s));
   for (int64_t pp = 0; pp < (int64_t)np * np; pp++) {
     CU(launch_gam3_raw_range(u.d, aux.as<double>(), pp * n6, n6,
                              slice.as<double>(), s));
     CU(launch_gam3_symmetrize(ne, 1, slice.as<double>(), s));
-    CU(launch_eg3_partials(ne, np, pp, 1, dde, slice.as<double>(),
-                           part.as<double>(), s));
+    CU(launch_eg3_partials(ne, np, pp, 1, slice.as<double>(), part.as<double>(), s));
   }
-  const size_t nparts = (size_t)np * np * ne * ne * ne * ne;
-  CU(launch_fock_reduce(ne, np, ne * ne, part.as<double>(), dde, ddp, 3.0, 1,
-                        dfe, dfp, part.as<double>() + nparts, dE, s));
+  CU(launch_eg3_reduce(ne, np, part.as<double>(), dde, ddp, dfe, dfp, dE, s));
   return NEOXC_OK;
 }
 
@@ -1254,7 +1252,7 @@ static int gam2_dscf_dev(const SysUpload& u, cudaStream_t s, const double* dde,
   DBuf s1, s2, part;
   RC(dalloc(s1, sizeof(double) * n4, s));
   RC(dalloc(s2, sizeof(double) * n4, s));
-  RC(dalloc(part, sizeof(double) * (2 * npart + 2 * np * np), s));
+  RC(dalloc(part, sizeof(double) * (2 * npart + 2 * fock_reduce_doubles(ne, np)), s));
   double* pv = part.as<double>();
   double* ps = pv + npart;
   double* ftmp = ps + npart;
@@ -1274,7 +1272,7 @@ static int gam2_dscf_dev(const SysUpload& u, cudaStream_t s, const double* dde,
     }
   CU(launch_fock_reduce(ne, np, ne, pv, dde, ddp, 2.0, 1, dfe, dfp, ftmp, dE, s));
   CU(launch_fock_reduce(ne, np, ne, ps, dde, ddp, 1.0, 1, dse, dsp,
-                        ftmp + np * np, dS, s));
+                        ftmp + fock_reduce_doubles(ne, np), dS, s));
   return NEOXC_OK;
 }
 

@@ -11,6 +11,8 @@
 // shared memory, and partial sums are written per CTA and reduced by a
 // second, deterministic kernel (no floating-point atomics), so repeated
 // calls give bit-identical results.
+#include <algorithm>
+
 #include "neoxc_internal.h"
 
 namespace neoxc {
@@ -18,44 +20,76 @@ namespace neoxc {
 // part[((ipjp*ne + i1)*nsub + s)*ne + j1] -> Fock/energy.
 //   fe(i1,j1) (+)= fe_scale * sum_{ipjp} DP(ipjp) * sum_s part
 //   fp(ipjp)  (+)= sum_{i1,j1} DE(i1,j1) * sum_s part
-//   fp_tmp[ipjp] = DP(ipjp) * [that fp contribution]   (energy terms)
-__global__ void fock_reduce_kernel(int ne, int np, int nsub,
-                                   const double* __restrict__ part,
-                                   const double* __restrict__ DE,
-                                   const double* __restrict__ DP,
-                                   double fe_scale, int accumulate,
-                                   double* fe, double* fp, double* fp_tmp) {
+//   E = sum_{ipjp} DP(ipjp) * [that fp contribution]
+// Two kernels, both wide: the sub-block sums of every (ipjp, i1, j1) with
+// their share of fp, then the sums over ipjp.  (One thread per output walked
+// all of them in a row: 3.2 ms at ne = 12, np = 8, nsub = 144; now 10 us.)
+// A CTA of the first takes 1024 outputs of one ipjp, so that up to ne = 32
+// fp needs one partial per ipjp (the scratch size of the gam_4 calls).
+constexpr int kRedThreads = 128, kRedOut = 1024;
+
+__device__ __forceinline__ double block_add(double v, double* sw) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __syncthreads();
+  if (lane == 0) sw[w] = v;
+  __syncthreads();
+  double t = 0.0;
+  for (int k = 0; k < (int)(blockDim.x + 31) / 32; k++) t += sw[k];
+  return t;   // every thread gets the same value
+}
+
+// grid (ceil(ne^2 / kRedOut), np^2); the sums replace sub-block 0
+__global__ void __launch_bounds__(kRedThreads)
+fock_reduce_sub_kernel(int ne, int np, int nsub, double* __restrict__ part,
+                       const double* __restrict__ DE, double* __restrict__ fp_part) {
+  __shared__ double sw[kRedThreads / 32];
+  const int ipjp = blockIdx.y;
+  const int t0 = blockIdx.x * kRedOut, t1 = min(ne * ne, t0 + kRedOut);
+  double w = 0.0;
+  for (int t = t0 + threadIdx.x; t < t1; t += kRedThreads) {
+    const int i1 = t / ne, j1 = t - i1 * ne;
+    double* p = part + ((size_t)ipjp * ne + i1) * nsub * ne + j1;
+    double s = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < nsub; k++) s += p[(size_t)k * ne];
+    p[0] = s;
+    w = fma(DE[i1 + ne * j1], s, w);
+  }
+  const double sum = block_add(w, sw);
+  if (threadIdx.x == 0) fp_part[(size_t)ipjp * gridDim.x + blockIdx.x] = sum;
+}
+
+// CTAs 0..: a warp per (i1,j1), lanes over ipjp; the last CTA: fp and E
+__global__ void __launch_bounds__(kRedThreads)
+fock_reduce_out_kernel(int ne, int np, int nsub, int nfp, const double* __restrict__ part,
+                       const double* __restrict__ fp_part, const double* __restrict__ DP,
+                       double fe_scale, int accumulate, double* fe, double* fp, double* E) {
+  __shared__ double sw[kRedThreads / 32];
   const int n2 = ne * ne, p2 = np * np;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n2) {
-    int i1 = t / ne, j1 = t % ne;
-    double s = 0.0;
-    for (int ipjp = 0; ipjp < p2; ipjp++) {
-      int ip = ipjp / np, jp = ipjp % np;
-      double ss = 0.0;
-      for (int k = 0; k < nsub; k++)
-        ss += part[((size_t)(ipjp * ne + i1) * nsub + k) * ne + j1];
-      s = fma(DP[ip + np * jp], ss, s);
+  if (blockIdx.x == gridDim.x - 1) {
+    double e = 0.0;
+    for (int p = threadIdx.x; p < p2; p += kRedThreads) {
+      double s = 0.0;
+      for (int k = 0; k < nfp; k++) s += fp_part[(size_t)p * nfp + k];
+      const int f = p / np + np * (p % np);
+      if (fp) fp[f] = accumulate ? fp[f] + s : s;
+      e = fma(DP[f], s, e);
     }
-    if (fe) {
-      if (accumulate) fe[i1 + ne * j1] += fe_scale * s;
-      else fe[i1 + ne * j1] = fe_scale * s;
-    }
-  } else if (t < n2 + p2) {
-    int ipjp = t - n2, ip = ipjp / np, jp = ipjp % np;
-    double s = 0.0;
-    for (int i1 = 0; i1 < ne; i1++)
-      for (int j1 = 0; j1 < ne; j1++) {
-        double ss = 0.0;
-        for (int k = 0; k < nsub; k++)
-          ss += part[((size_t)(ipjp * ne + i1) * nsub + k) * ne + j1];
-        s = fma(DE[i1 + ne * j1], ss, s);
-      }
-    if (fp) {
-      if (accumulate) fp[ip + np * jp] += s;
-      else fp[ip + np * jp] = s;
-    }
-    fp_tmp[ipjp] = s * DP[ip + np * jp];
+    e = block_add(e, sw);
+    if (threadIdx.x == 0) *E = e;
+    return;
+  }
+  const int t = (int)((blockIdx.x * kRedThreads + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (t >= n2 || !fe) return;
+  const int i1 = t / ne, j1 = t - i1 * ne;
+  double s = 0.0;
+  for (int p = lane; p < p2; p += 32)
+    s = fma(DP[p / np + np * (p % np)], part[((size_t)p * ne + i1) * nsub * ne + j1], s);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0) {
+    const int f = i1 + ne * j1;
+    fe[f] = accumulate ? fe[f] + fe_scale * s : fe_scale * s;
   }
 }
 
@@ -73,72 +107,25 @@ __global__ void sum_vec_kernel(int n, const double* __restrict__ v,
   if (threadIdx.x == 0) *out = red[0];
 }
 
-cudaError_t launch_fock_reduce(int ne, int np, int nsub, const double* part,
+size_t fock_reduce_doubles(int ne, int np) {
+  return (size_t)np * np * (((size_t)ne * ne + kRedOut - 1) / kRedOut);
+}
+
+cudaError_t launch_fock_reduce(int ne, int np, int nsub, double* part,
                                const double* DE, const double* DP,
                                double fe_scale, int accumulate, double* fe,
-                               double* fp, double* fp_tmp, double* E,
+                               double* fp, double* fp_part, double* E,
                                cudaStream_t s) {
-  const int nout = ne * ne + np * np;
-  fock_reduce_kernel<<<(nout + 127) / 128, 128, 0, s>>>(
-      ne, np, nsub, part, DE, DP, fe_scale, accumulate, fe, fp, fp_tmp);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  sum_vec_kernel<<<1, 256, 0, s>>>(np * np, fp_tmp, E);
+  const int nfp = (ne * ne + kRedOut - 1) / kRedOut;
+  for (int p0 = 0; p0 < np * np; p0 += 65535)   // grid.y limit
+    fock_reduce_sub_kernel<<<dim3(nfp, std::min(np * np - p0, 65535)), kRedThreads, 0, s>>>(
+        ne, np, nsub, part + (size_t)p0 * ne * nsub * ne, DE, fp_part + (size_t)p0 * nfp);
+  fock_reduce_out_kernel<<<(ne * ne + 3) / 4 + 1, kRedThreads, 0, s>>>(
+      ne, np, nsub, nfp, part, fp_part, DP, fe_scale, accumulate, fe, fp, E);
   return cudaGetLastError();
 }
 
 namespace {
-
-// ---- EG3IC1 --------------------------------------------------------------
-// CTA per (ip,jp,i1,i2,i3): the ne^3 ket values G3(i1,x;i2,y;i3,z) are
-// staged in shared memory (one HBM read per element), then each thread
-// forms GAM3 for its (j1,j2,j3) from the six ket permutations.
-__global__ void __launch_bounds__(256)
-eg3_kernel(int ne, int np, const double* __restrict__ DE,
-           const double* __restrict__ g3, double* __restrict__ part,
-           long long ipjp0) {
-  extern __shared__ double sm[];
-  const int n2 = ne * ne, n3 = n2 * ne;
-  double* sG = sm;           // [x][y][z] = G3(i1,x,i2,y,i3,z)
-  double* sDE = sm + n3;
-  double* sred = sDE + n2;
-  int cta = blockIdx.x;
-  const int i3 = cta % ne; cta /= ne;
-  const int i2 = cta % ne; cta /= ne;
-  const int i1 = cta % ne; cta /= ne;
-  const long long ipjp = cta;   // relative to the slice g3 points at
-  for (int k = threadIdx.x; k < n2; k += blockDim.x) sDE[k] = DE[k];
-  // index_GAM_3PK(ip,jp,i1,x,i2,y,i3,z)-1 = z + ne*(i3 + ne*(y + ne*(i2 +
-  //   ne*(x + ne*(i1 + ne*ipjp)))))
-  for (int k = threadIdx.x; k < n3; k += blockDim.x) {
-    int x = k / n2, r = k - x * n2, y = r / ne, z = r - y * ne;
-    long long o = z + (long long)ne * (i3 + (long long)ne * (y + (long long)ne * (i2 +
-                  (long long)ne * (x + (long long)ne * (i1 + (long long)ne * ipjp)))));
-    sG[k] = __ldg(g3 + o);
-  }
-  __syncthreads();
-  const int lanes = blockDim.x / ne;
-  const int j1 = threadIdx.x % ne;
-  double acc = 0.0;
-  for (int q = threadIdx.x / ne; q < n2; q += lanes) {
-    const int j2 = q / ne, j3 = q - j2 * ne;
-#define G(a, b, c) sG[(a) * n2 + (b) * ne + (c)]
-    double o123 = G(j1, j2, j3), o213 = G(j2, j1, j3), o312 = G(j3, j1, j2);
-    double o132 = G(j1, j3, j2), o231 = G(j2, j3, j1), o321 = G(j3, j2, j1);
-#undef G
-    double g = 8.0 * o123 - 4.0 * o213 + 2.0 * o312 - 4.0 * o132 +
-               2.0 * o231 - 4.0 * o321;
-    g = g / 8.0;
-    acc = fma(sDE[i2 + ne * j2] * sDE[i3 + ne * j3], g, acc);
-  }
-  sred[threadIdx.x] = acc;
-  __syncthreads();
-  if ((int)threadIdx.x < ne) {
-    double s = 0.0;
-    for (int t = threadIdx.x; t < (int)blockDim.x; t += ne) s += sred[t];
-    part[((size_t)blockIdx.x + (size_t)ipjp0 * n3) * ne + threadIdx.x] = s;
-  }
-}
 
 // ---- EG2IC1 --------------------------------------------------------------
 // CTA per (ip,jp,i1,i2); thread per j1 (strided), loop over j2.
@@ -329,38 +316,39 @@ __global__ void index_fill_kernel(int kind, int ne, int np, long long count,
 }  // namespace
 
 size_t eg3_partial_doubles(int ne, int np) {
-  return (size_t)np * np * ne * ne * ne * ne + (size_t)np * np;
+  return rank3_weight_doubles(ne, 1) + (size_t)np * np * ne * ne * ne + fock_reduce_doubles(ne, np);
 }
 
-cudaError_t launch_eg3_partials(int ne, int np, long long ipjp0,
-                                long long nipjp, const double* DE,
-                                const double* g3_slice, double* part,
-                                cudaStream_t s) {
+cudaError_t launch_eg3_weights(int ne, const double* DE, double* scratch, cudaStream_t s) {
+  return launch_rank3_weights_closed(ne, DE, scratch, s);
+}
+
+cudaError_t launch_eg3_partials(int ne, int np, long long ipjp0, long long nipjp,
+                                const double* g3_slice, double* scratch, cudaStream_t s) {
   if (ne < 1 || ne > 20 || np < 1) return cudaErrorInvalidValue;
-  const int bs = ne * (256 / ne);
-  const size_t smem = sizeof(double) * ((size_t)ne * ne * ne + ne * ne + bs);
-  cudaError_t e = cudaFuncSetAttribute(eg3_kernel,
-      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  const long long grid = nipjp * ne * ne * ne;
-  eg3_kernel<<<(unsigned)grid, bs, smem, s>>>(ne, np, DE, g3_slice, part, ipjp0);
-  return cudaGetLastError();
+  double* part = scratch + rank3_weight_doubles(ne, 1) + (size_t)ipjp0 * ne * ne * ne;
+  return launch_rank3(ne, nipjp, 1, 1u, g3_slice, scratch, nullptr, nullptr, part, nullptr, s);
+}
+
+cudaError_t launch_eg3_reduce(int ne, int np, double* scratch, const double* DE, const double* DP,
+                              double* focke, double* fockp, double* E, cudaStream_t s) {
+  double* part = scratch + rank3_weight_doubles(ne, 1);
+  return launch_fock_reduce(ne, np, ne, part, DE, DP, 3.0, 1, focke, fockp,
+                            part + (size_t)np * np * ne * ne * ne, E, s);
 }
 
 cudaError_t launch_eg3ic1(int ne, int np, const double* DE, const double* DP,
                           const double* g3, double* scratch, double* focke,
                           double* fockp, double* E, cudaStream_t s) {
-  cudaError_t e = launch_eg3_partials(ne, np, 0, (long long)np * np, DE, g3,
-                                      scratch, s);
+  cudaError_t e = launch_eg3_weights(ne, DE, scratch, s);
   if (e != cudaSuccess) return e;
-  const long long grid = (long long)np * np * ne * ne * ne;
-  double* fp_tmp = scratch + (size_t)grid * ne;
-  return launch_fock_reduce(ne, np, ne * ne, scratch, DE, DP, 3.0, 1, focke,
-                            fockp, fp_tmp, E, s);
+  e = launch_eg3_partials(ne, np, 0, (long long)np * np, g3, scratch, s);
+  if (e != cudaSuccess) return e;
+  return launch_eg3_reduce(ne, np, scratch, DE, DP, focke, fockp, E, s);
 }
 
 size_t eg2_partial_doubles(int ne, int np) {
-  return 2 * (size_t)np * np * ne * ne * ne + 2 * (size_t)np * np;
+  return 2 * (size_t)np * np * ne * ne * ne + 2 * fock_reduce_doubles(ne, np);
 }
 
 cudaError_t launch_eg2ic1(int ne, int np, const double* DE, const double* DP,
@@ -380,7 +368,7 @@ cudaError_t launch_eg2ic1(int ne, int np, const double* DE, const double* DP,
   e = launch_fock_reduce(ne, np, ne, pv, DE, DP, 2.0, 1, FE, FP, ftmp, E, s);
   if (e != cudaSuccess) return e;
   return launch_fock_reduce(ne, np, ne, ps, DE, DP, 1.0, 0, SE, SP,
-                            ftmp + np * np, S, s);
+                            ftmp + fock_reduce_doubles(ne, np), S, s);
 }
 
 cudaError_t launch_eg2_partials(int ne, int np, long long ipjp0,

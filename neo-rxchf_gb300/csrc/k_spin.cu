@@ -80,27 +80,6 @@ __device__ inline void acc2(const S& g, int j1, int j2, double a2, double b2,
   if (fb & 2u) B = fma(a2, o12, B);
 }
 
-// K = 3: OMG6 (bit0), the two mixed pairs OMG12/OMG13 (bit1), OMG23 (bit2)
-template <typename S>
-__device__ inline void acc3(const S& g, const int* j, double a2, double b2,
-                            double a3, double b3, unsigned fa, unsigned fb,
-                            double& A, double& B) {
-  const int j1 = j[0], j2 = j[1], j3 = j[2];
-  const int k123[3] = {j1, j2, j3}, k213[3] = {j2, j1, j3}, k312[3] = {j3, j1, j2};
-  const int k132[3] = {j1, j3, j2}, k231[3] = {j2, j3, j1}, k321[3] = {j3, j2, j1};
-  const double g123 = g(k123), g213 = g(k213), g132 = g(k132), g321 = g(k321);
-  const unsigned f = fa | fb;
-  double o6 = 0.0;
-  if (f & 1u) o6 = g123 - g213 + g(k312) - g132 + g(k231) - g321;
-  const double o23 = g123 - g132, o12 = g123 - g213, o13 = g123 - g321;
-  if (fa & 1u) A = fma(a2 * a3, o6, A);
-  if (fa & 2u) A = fma(a2 * b3, o12, fma(b2 * a3, o13, A));
-  if (fa & 4u) A = fma(b2 * b3, o23, A);
-  if (fb & 1u) B = fma(b2 * b3, o6, B);
-  if (fb & 2u) B = fma(b2 * a3, o12, fma(a2 * b3, o13, B));
-  if (fb & 4u) B = fma(a2 * a3, o23, B);
-}
-
 // K = 4: the 24-term set (bit0), the three 6-term sets (bit1), the three
 // 4-term sets (bit2) and the last 6-term set (bit3) of calc_FAEOMG4.
 template <typename S>
@@ -151,8 +130,8 @@ __device__ inline void acc4(const S& g, const int* j, const double* a,
   if (fb & 8u) B = fma(a[0] * a[1] * a[2], bbb, B);
 }
 
-// CTA (ipjp, i1, i2) for rank 2, (ipjp, i1, i2, i3) for ranks 3 and 4 (rank
-// 4 loops over i4).  Outputs per CTA: part[(cta*nacc + a)*ne + j1]
+// CTA (ipjp, i1, i2) for rank 2, (ipjp, i1, i2, i3) for rank 4, which loops
+// over i4 (rank 3: k_rank3.cu).  Outputs per CTA: part[(cta*nacc + a)*ne + j1]
 // (a = 2*tensor + class; the electron Fock rows) and ppart[cta*2 + t] =
 // sum_j1 (DA(i1,j1) A_t[j1] + DB(i1,j1) B_t[j1]) (the proton terms).
 template <int K, bool SMEM>
@@ -247,8 +226,6 @@ spin_kernel(int ne, int np, const double* __restrict__ G,
         if constexpr (K == 2) {
           acc2(g[0], j1, j[1], a[0], b[0], fa, fb, accA[0], accB[0]);
           if (nten == 2) acc2(g[1], j1, j[1], a[0], b[0], fa, fb, accA[1], accB[1]);
-        } else if constexpr (K == 3) {
-          acc3(g[0], j, a[0], b[0], a[1], b[1], fa, fb, accA[0], accB[0]);
         } else {
           acc4(g[0], j, a, b, fa, fb, accA[0], accB[0]);
         }
@@ -464,7 +441,7 @@ cudaError_t launch_spin_kernel(int ne, int np, const double* G, const double* Gs
   cudaError_t e = cudaFuncSetAttribute(spin_kernel<K, SMEM>,
       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const long long grid = (long long)np * np * ne * ne * (K >= 3 ? ne : 1);
+  const long long grid = (long long)np * np * ne * ne * (K == 4 ? ne : 1);
   spin_kernel<K, SMEM><<<(unsigned)grid, bs, smem, s>>>(ne, np, G, Gs, DA, DB, fa,
                                                          fb, part, ppart);
   return cudaGetLastError();
@@ -474,8 +451,8 @@ cudaError_t launch_spin_kernel(int ne, int np, const double* G, const double* Gs
 
 size_t spin_scratch_doubles(int K, int ne, int np) {
   const int nacc = K == 2 ? 4 : 2;
-  const size_t ncta = (size_t)np * np * ne * ne * (K >= 3 ? ne : 1);
-  return ncta * nacc * ne + ncta * 2;
+  const size_t ncta = (size_t)np * np * ne * ne * (K == 4 ? ne : 1);
+  return ncta * nacc * ne + ncta * 2 + (K == 3 ? rank3_weight_doubles(ne, 2) : 0);
 }
 
 cudaError_t launch_spin_omg(int K, int ne, int np, const double* G, const double* Gs,
@@ -485,7 +462,7 @@ cudaError_t launch_spin_omg(int K, int ne, int np, const double* G, const double
   if (ne < 1 || ne > kSpinThreads || np < 1 || K < 2 || K > 4 || (K != 2 && Gs))
     return cudaErrorInvalidValue;
   const int nacc = (K == 2 && Gs) ? 4 : 2;
-  const size_t ncta = (size_t)np * np * ne * ne * (K >= 3 ? ne : 1);
+  const size_t ncta = (size_t)np * np * ne * ne * (K == 4 ? ne : 1);
   double* part = scratch;
   double* ppart = scratch + ncta * (K == 2 ? 4 : 2) * ne;
   cudaError_t e;
@@ -495,12 +472,16 @@ cudaError_t launch_spin_omg(int K, int ne, int np, const double* G, const double
              : launch_spin_kernel<2, false>(ne, np, G, Gs, DA, DB, fa, fb, part, ppart, s);
   else if (!fits)   // ranks 3 and 4 stage the whole ket block
     return cudaErrorInvalidValue;
-  else if (K == 3)
-    e = launch_spin_kernel<3, true>(ne, np, G, nullptr, DA, DB, fa, fb, part, ppart, s);
-  else
+  else if (K == 3) {
+    double* W = ppart + ncta * 2;
+    e = launch_rank3_weights_open(ne, DA, DB, fa, fb, W, s);
+    if (e != cudaSuccess) return e;
+    e = launch_rank3(ne, (long long)np * np, 2, (fa ? 1u : 0u) | (fb ? 2u : 0u), G, W, DA, DB,
+                     part, ppart, s);
+  } else
     e = launch_spin_kernel<4, true>(ne, np, G, nullptr, DA, DB, fa, fb, part, ppart, s);
   if (e != cudaSuccess) return e;
-  const int nsub = K == 2 ? ne : ne * ne;
+  const int nsub = K == 4 ? ne * ne : ne;
   const int ne_out = nacc * ne * ne;
   spin_reduce_e_kernel<<<(ne_out + 3) / 4, 128, 0, s>>>(ne, np, nacc, nsub, part, DP,
                                                         fe_out);

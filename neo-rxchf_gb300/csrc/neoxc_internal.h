@@ -55,11 +55,28 @@ int set_last_error(int code, const char* fmt, ...);
 //   part[((ipjp*ne + i1)*nsub + s)*ne + j1]:
 //   fe(i1,j1) (+)= fe_scale * sum_ipjp DP * sum_s part,
 //   fp(ipjp)  (+)= sum_{i1,j1} DE * sum_s part,  E = sum_ipjp DP * fp-part.
-cudaError_t launch_fock_reduce(int ne, int np, int nsub, const double* part,
+// part is overwritten; fp_part: fock_reduce_doubles (np^2 up to ne = 32).
+size_t fock_reduce_doubles(int ne, int np);
+cudaError_t launch_fock_reduce(int ne, int np, int nsub, double* part,
                                const double* DE, const double* DP,
                                double fe_scale, int accumulate, double* fe,
-                               double* fp, double* fp_tmp, double* E,
+                               double* fp, double* fp_part, double* E,
                                cudaStream_t s);
+
+// ---- stored rank-3 tensors (k_rank3.cu): EG3IC1, FAE / UFP_OMG3 -----------
+// Weight tables [class][slot][i2][i3][u][v] of the ket pair (u,v) left when
+// the Fock row's ket sits in `slot`, from the densities alone: closed shell
+// (EG3IC1, one class) or open shell (two classes, flag bits as below).
+size_t rank3_weight_doubles(int ne, int ncls);
+cudaError_t launch_rank3_weights_closed(int ne, const double* DE, double* W, cudaStream_t s);
+cudaError_t launch_rank3_weights_open(int ne, const double* DA, const double* DB, unsigned fa,
+                                      unsigned fb, double* W, cudaStream_t s);
+// part[((p*ne + i1)*ne + i2)*ncls + c][j1]; with DA / DB (two classes) also
+// ppart[2*((p*ne + i1)*ne + i2)] = sum_j1 (DA row_A + DB row_B).  used: bit c
+// set when class c has any nonzero weight (else its rows are zeros).
+cudaError_t launch_rank3(int ne, long long nipjp, int ncls, unsigned used, const double* g3,
+                         const double* W, const double* DA, const double* DB, double* part,
+                         double* ppart, cudaStream_t s);
 
 // ---- open-shell XCUHF contractions (k_spin.cu, xcuhf/xcuhf_omg*.f) ------
 // Rank K = 2 (GM2ICR, optional GM2sICR as Gs), 3 (GM3ICR) or 4 (OMG4_ICR).
@@ -176,10 +193,12 @@ cudaError_t launch_xcfock_correction(int ne, int np, double S_total,
 // Partial sums of one proton-pair slice [ipjp0, ipjp0+nipjp) of the
 // contraction; the slice pointer addresses the slice's first element and the
 // partials land at their global positions (direct-SCF slicing).
-cudaError_t launch_eg3_partials(int ne, int np, long long ipjp0,
-                                long long nipjp, const double* DE,
-                                const double* g3_slice, double* part,
-                                cudaStream_t s);
+// Call launch_eg3_weights once, the partials of every slice, then the reduce.
+cudaError_t launch_eg3_weights(int ne, const double* DE, double* scratch, cudaStream_t s);
+cudaError_t launch_eg3_partials(int ne, int np, long long ipjp0, long long nipjp,
+                                const double* g3_slice, double* scratch, cudaStream_t s);
+cudaError_t launch_eg3_reduce(int ne, int np, double* scratch, const double* DE, const double* DP,
+                              double* focke, double* fockp, double* E, cudaStream_t s);
 cudaError_t launch_eg2_partials(int ne, int np, long long ipjp0,
                                 long long nipjp, const double* DE,
                                 const double* g2_slice,
