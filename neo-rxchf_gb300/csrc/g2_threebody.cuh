@@ -29,24 +29,17 @@
 #pragma once
 #include "g3_fatbra.cuh"
 
-// Loops over directions and operators stay loops: unrolled, the routine
-// outgrows the instruction cache and the builder waits for instructions
-// instead of the FP64 pipe.
-#if defined(__CUDACC__)
-#define NX_LOOP _Pragma("unroll 1")
-#else
-#define NX_LOOP
-#endif
-
 namespace neoxc {
 namespace g2 {
 
+using g3::fold_line;
 using g3::kRC;
 using g3::kRE;
 using g3::kRLen;
 using g3::kRP;
 using g3::kRT;
 using g3::kRX;
+using g3::rsqrt64;
 
 // gradient record of a pair: EG[d][t], t <= 6, the Hermite coefficients of
 // (d phi_a / dx_d)(d phi_b / dx_d) in direction d
@@ -73,148 +66,19 @@ G3_HD void fill_gradient_record(const md::Prim& A, const md::Prim& B, double* ou
   for (int t = 3 * kGRow; t < kGLen; t++) out[t] = 0.0;
 }
 
-G3_HD double rsqrt64(double x) {
-#if defined(__CUDA_ARCH__)
-  return rsqrt(x);
-#else
-  return 1.0 / sqrt(x);
-#endif
-}
-
-// t! / ((2i-t)! (t-i)!), t, i <= 12 (zero unless i <= t <= 2i): the
-// coefficient of W[t] (2R)^(2i-t) in A[i]
-#define NX_HERMX_VALUES \
-    1, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
-    0, 1, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
-    0, 2, 1, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
-    0, 0, 6, 1, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
-    0, 0, 12, 12, 1, 0, 0, 0, 0, 0, 0, 0, 0, \
-    0, 0, 0, 60, 20, 1, 0, 0, 0, 0, 0, 0, 0, \
-    0, 0, 0, 120, 180, 30, 1, 0, 0, 0, 0, 0, 0, \
-    0, 0, 0, 0, 840, 420, 42, 1, 0, 0, 0, 0, 0, \
-    0, 0, 0, 0, 1680, 3360, 840, 56, 1, 0, 0, 0, 0, \
-    0, 0, 0, 0, 0, 15120, 10080, 1512, 72, 1, 0, 0, 0, \
-    0, 0, 0, 0, 0, 30240, 75600, 25200, 2520, 90, 1, 0, 0, \
-    0, 0, 0, 0, 0, 0, 332640, 277200, 55440, 3960, 110, 1, 0, \
-    0, 0, 0, 0, 0, 0, 665280, 1995840, 831600, 110880, 5940, 132, 1
-#if defined(__CUDACC__)
-static __device__ const double kHermXDev[13 * 13] = {NX_HERMX_VALUES};
-#endif
-static const double kHermXHost[13 * 13] = {NX_HERMX_VALUES};
-#undef NX_HERMX_VALUES
-G3_HD double hermx(int t, int i) {
-#if defined(__CUDA_ARCH__)
-  return __ldg(&kHermXDev[t * 13 + i]);
-#else
-  return kHermXHost[t * 13 + i];
-#endif
-}
-
-// A[i] = sum_t W[t] t! / ((2i-t)! (t-i)!) (2R)^(2i-t), i <= n: the factors of
-// (-alpha)^i F_i in d^t/dR^t of F_0(alpha R^2).  Orders up to 2 (most of
-// them) straight; beyond, Horner in 2R.
-G3_HD void hermite_powers(int n, const double* W, double R, double* A) {
-  A[0] = W[0];
-  if (n == 0) return;
-  const double x = R + R;
-  if (n == 1) {
-    A[1] = W[1] * x;
-    return;
-  }
-  if (n == 2) {
-    A[1] = fma(W[1], x, W[2] + W[2]);
-    A[2] = W[2] * x * x;
-    return;
-  }
-  double xp = 1.0;   // x^(2i - min(2i, n))
-  for (int i = 1; i <= n; i++) {
-    const int hi = 2 * i < n ? 2 * i : n;
-    double a = W[i];
-    for (int t = i + 1; t <= hi; t++) a = fma(a, x, W[t] * hermx(t, i));
-    if (2 * i > n) {
-      xp *= (2 * i == n + 1) ? x : x * x;
-      a *= xp;
-    }
-    A[i] = a;
-  }
-}
-
-// sum_m (-alpha)^m F_m(T) B[m], m <= L: boys_sum (md_math_body.cuh) over a
-// stored vector; for T > 20 the asymptotic F_m = F_0 prod (j - 1/2) / T by
-// Horner in -alpha / T.
-G3_HD double boys_dot(int L, double T, double alpha, const double* B) {
-  const double ma = -alpha;
-  if (!(T <= 20.0)) {
-    const double rs = rsqrt64(T);
-    const double q = ma * (rs * rs);
-    double s = B[L];
-    NX_LOOP
-    for (int m = L; m >= 1; m--) s = fma(s, q * ((double)m - 0.5), B[m - 1]);
-    return (0.88622692545275801365 * rs) * s;
-  }
-  return boys_sum(L, T, alpha, [&](int m) { return B[m]; });
-}
-
-// sum_m (-alpha)^m F_m(T) sum_{i+j+k=m} A_x[i] A_y[j] A_z[k]
+// sum_m F_m(T) sum_{i+j+k=m} A_x[i] A_y[j] A_z[k], T = alpha |R|^2
 template <int NT>
 G3_HD double coulomb_sum(const int* n, const double (*W)[NT + 1], const double* R, double T,
                          double alpha) {
-  double A[3][NT + 1];
+  const double z = -(alpha + alpha);
+  double B[3 * NT + 1], A[NT + 1];
+  g3::hermite_scaled(n[0], W[0], z * R[0], z, B);
   NX_LOOP
-  for (int d = 0; d < 3; d++) hermite_powers(n[d], W[d], R[d], A[d]);
-  const int nxy = n[0] + n[1], L = nxy + n[2];
-  double Bxy[2 * NT + 1], B[3 * NT + 1];
-  NX_LOOP
-  for (int m = 0; m <= nxy; m++) {
-    const int lo = m > n[1] ? m - n[1] : 0, hi = m < n[0] ? m : n[0];
-    double b = A[0][lo] * A[1][m - lo];
-    for (int i = lo + 1; i <= hi; i++) b = fma(A[0][i], A[1][m - i], b);
-    Bxy[m] = b;
+  for (int d = 1; d < 3; d++) {
+    g3::hermite_scaled(n[d], W[d], z * R[d], z, A);
+    g3::convolve(B, d == 1 ? n[0] : n[0] + n[1], A, n[d]);
   }
-  NX_LOOP
-  for (int m = 0; m <= L; m++) {
-    const int lo = m > n[2] ? m - n[2] : 0, hi = m < nxy ? m : nxy;
-    double b = Bxy[lo] * A[2][m - lo];
-    for (int i = lo + 1; i <= hi; i++) b = fma(Bxy[i], A[2][m - i], b);
-    B[m] = b;
-  }
-  return boys_dot(L, T, alpha, B);
-}
-
-// In place along one axis: v[x] <- sum_s v[s] E[s + x] C(s + x, x), s + x <= t.
-G3_HD void fold_line(double* v, int stride, int t, const double* E) {
-  const double v0 = v[0];
-  if (t == 0) {
-    v[0] = v0 * E[0];
-    return;
-  }
-  const double v1 = v[stride];
-  if (t == 1) {
-    v[0] = fma(v1, E[1], v0 * E[0]);
-    v[stride] = v0 * E[1];
-    return;
-  }
-  const double v2 = v[2 * stride];
-  if (t == 2) {
-    v[0] = fma(v2, E[2], fma(v1, E[1], v0 * E[0]));
-    v[stride] = fma(v1 + v1, E[2], v0 * E[1]);
-    v[2 * stride] = v0 * E[2];
-    return;
-  }
-  const double v3 = v[3 * stride];
-  if (t == 3) {
-    v[0] = fma(v3, E[3], fma(v2, E[2], fma(v1, E[1], v0 * E[0])));
-    v[stride] = fma(3.0 * v2, E[3], fma(v1 + v1, E[2], v0 * E[1]));
-    v[2 * stride] = fma(3.0 * v1, E[3], v0 * E[2]);
-    v[3 * stride] = v0 * E[3];
-    return;
-  }
-  const double v4 = v[4 * stride];
-  v[0] = fma(v4, E[4], fma(v3, E[3], fma(v2, E[2], fma(v1, E[1], v0 * E[0]))));
-  v[stride] = fma(4.0 * v3, E[4], fma(3.0 * v2, E[3], fma(v1 + v1, E[2], v0 * E[1])));
-  v[2 * stride] = fma(6.0 * v2, E[4], fma(3.0 * v1, E[3], v0 * E[2]));
-  v[3 * stride] = fma(4.0 * v1, E[4], v0 * E[3]);
-  v[4 * stride] = v0 * E[4];
+  return g3::boys_dot(n[0] + n[1] + n[2], T, B);
 }
 
 // One primitive triple and geminal pair.  FULL: *x1 = the Coulomb, nuclear
@@ -470,8 +334,8 @@ G3_HD double two_body_overlap(const double* r1, const double* rp, double g) {
 
 // Composite bra of pair densities A (kept) and B (integrated out with the
 // geminal exp(-g r_AB^2)): the charge density of A's particle dressed by B.
-template <class R, int MA, int MB, int NW>
-G3_HD void build_bra_pair(const double* ra, const double* rb, double g, g3::Bra<R, NW>& b) {
+template <int MA, int MB, int NW>
+G3_HD void build_bra_pair(const double* ra, const double* rb, double g, g3::Bra<double, NW>& b) {
   const double kPi = 3.14159265358979e+00;
   const double PA = ra[kRP], PB = rb[kRP];
   const double x = PB + g, rx = 1.0 / x;
@@ -493,7 +357,7 @@ G3_HD void build_bra_pair(const double* ra, const double* rb, double g, g3::Bra<
       fold_line(V + s * (tb + 1), 1, tb, rb + kRE + 5 * d);
     }
     for (int t = 0; t <= tb; t++) fold_line(V + t, tb + 1, ta, ra + kRE + 5 * d);
-    for (int k = 0; k <= NW; k++) b.W[d][k] = R(0);
+    for (int k = 0; k <= n; k++) b.W[d][k] = 0.0;
     double pa = 1.0;
     for (int s = 0; s <= ta; s++) {
       double p = pa;

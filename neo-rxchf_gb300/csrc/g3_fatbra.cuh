@@ -7,6 +7,7 @@
 // Boys function, the seeds (-alpha)^m F_m(T) and their sum are FP64 in both.
 #pragma once
 #include <math.h>
+#include <string.h>
 
 #include "md_math.cuh"
 
@@ -109,10 +110,45 @@ G3_HD void dgauss3t(int nk, const R* xi, const R (*c)[3], const R* X,
 #undef DD
 }
 
-G3_HD double binom_d(int n, int k) {
-  double r = 1.0;
-  for (int i = 1; i <= k; i++) r = r * (double)(n - k + i) / (double)i;
-  return r;
+// C(n, k), k <= n <= 4
+G3_HD int binom4(int n, int k) {
+  return k == 0 || k == n ? 1 : (n == 4 && k == 2 ? 6 : n);
+}
+
+// In place along one axis: v[x] <- sum_s v[s] E[s + x] C(s + x, x), s + x <= t.
+G3_HD void fold_line(double* v, int stride, int t, const double* E) {
+  const double v0 = v[0];
+  if (t == 0) {
+    v[0] = v0 * E[0];
+    return;
+  }
+  const double v1 = v[stride];
+  if (t == 1) {
+    v[0] = fma(v1, E[1], v0 * E[0]);
+    v[stride] = v0 * E[1];
+    return;
+  }
+  const double v2 = v[2 * stride];
+  if (t == 2) {
+    v[0] = fma(v2, E[2], fma(v1, E[1], v0 * E[0]));
+    v[stride] = fma(v1 + v1, E[2], v0 * E[1]);
+    v[2 * stride] = v0 * E[2];
+    return;
+  }
+  const double v3 = v[3 * stride];
+  if (t == 3) {
+    v[0] = fma(v3, E[3], fma(v2, E[2], fma(v1, E[1], v0 * E[0])));
+    v[stride] = fma(3.0 * v2, E[3], fma(v1 + v1, E[2], v0 * E[1]));
+    v[2 * stride] = fma(3.0 * v1, E[3], v0 * E[2]);
+    v[3 * stride] = v0 * E[3];
+    return;
+  }
+  const double v4 = v[4 * stride];
+  v[0] = fma(v4, E[4], fma(v3, E[3], fma(v2, E[2], fma(v1, E[1], v0 * E[0]))));
+  v[stride] = fma(4.0 * v3, E[4], fma(3.0 * v2, E[3], fma(v1 + v1, E[2], v0 * E[1])));
+  v[2 * stride] = fma(6.0 * v2, E[4], fma(3.0 * v1, E[3], v0 * E[2]));
+  v[3 * stride] = fma(4.0 * v1, E[4], v0 * E[3]);
+  v[4 * stride] = v0 * E[4];
 }
 
 // W'_d[x0+x1+x2] = sum E0[t0] E1[t1] E2[t2] sum_x C(t,x) cof^x D(t - x):
@@ -145,7 +181,7 @@ G3_HD void fold_bra(const double* r0, const double* r1, const double* r2, int nk
           for (int x0 = 0; x0 <= t0; x0++)
             for (int x1 = 0; x1 <= t1; x1++)
               for (int x2 = 0; x2 <= t2; x2++) {
-                const R cc = (R)(binom_d(t0, x0) * binom_d(t1, x1) * binom_d(t2, x2)) *
+                const R cc = (R)(binom4(t0, x0) * binom4(t1, x1) * binom4(t2, x2)) *
                              pw[0][x0] * pw[1][x1] * pw[2][x2] *
                              D[((t0 - x0) * X0 + (t1 - x1)) * X2 + (t2 - x2)];
                 b.W[d][x0 + x1 + x2] += e * cc;
@@ -153,6 +189,83 @@ G3_HD void fold_bra(const double* r0, const double* r1, const double* r2, int nk
         }
     b.N[d] = tl[0] + tl[1] + tl[2];
   }
+}
+
+// The same in FP64 with far fewer operations: one exponential for the three
+// directions (into *scale), and the sums over t one particle at a time.
+template <int LE, int LN, int NW>
+G3_HD void fold_bra(const double* r0, const double* r1, const double* r2, int nk,
+                    const double* xi, const double (*c)[3], const double* cof,
+                    Bra<double, NW>& b, double* scale) {
+  constexpr int X0 = 2 * LE + 1, X2 = 2 * LN + 1;
+  double H[6] = {0, 0, 0, 0, 0, 0};   // 2 sum_k xi_k c_k c_k^T: 00 01 02 11 12 22
+  for (int k = 0; k < nk; k++) {
+    const double x0 = 2.0 * xi[k] * c[k][0], x1 = 2.0 * xi[k] * c[k][1];
+    H[0] = fma(x0, c[k][0], H[0]);
+    H[1] = fma(x0, c[k][1], H[1]);
+    H[2] = fma(x0, c[k][2], H[2]);
+    H[3] = fma(x1, c[k][1], H[3]);
+    H[4] = fma(x1, c[k][2], H[4]);
+    H[5] = fma(2.0 * xi[k] * c[k][2], c[k][2], H[5]);
+  }
+  double ex = 0.0;
+  for (int d = 0; d < 3; d++) {
+    const double X[3] = {r0[kRX + d], r1[kRX + d], r2[kRX + d]};
+    const int t0 = (int)r0[kRT + d], t1 = (int)r1[kRT + d], t2 = (int)r2[kRT + d];
+    double g0 = 0.0, g1 = 0.0, g2 = 0.0;   // -gradient
+    for (int k = 0; k < nk; k++) {
+      const double u = c[k][0] * X[0] + c[k][1] * X[1] + c[k][2] * X[2], xu = xi[k] * u;
+      ex = fma(xu, u, ex);
+      g0 = fma(-2.0 * xu, c[k][0], g0);
+      g1 = fma(-2.0 * xu, c[k][1], g1);
+      g2 = fma(-2.0 * xu, c[k][2], g2);
+    }
+    const int w2 = t2 + 1, w1 = (t1 + 1) * w2;
+    double V[X0 * X0 * X2];
+    for (int n0 = 0; n0 <= t0; n0++)
+      for (int n1 = 0; n1 <= t1; n1++)
+        for (int n2 = 0; n2 <= t2; n2++) {
+          const int o = n0 * w1 + n1 * w2 + n2;
+          double v = 1.0;
+          if (n0 > 0) {
+            v = g0 * V[o - w1];
+            if (n0 > 1) v = fma(-H[0] * (double)(n0 - 1), V[o - 2 * w1], v);
+            if (n1 > 0) v = fma(-H[1] * (double)n1, V[o - w1 - w2], v);
+            if (n2 > 0) v = fma(-H[2] * (double)n2, V[o - w1 - 1], v);
+          } else if (n1 > 0) {
+            v = g1 * V[o - w2];
+            if (n1 > 1) v = fma(-H[3] * (double)(n1 - 1), V[o - 2 * w2], v);
+            if (n2 > 0) v = fma(-H[4] * (double)n2, V[o - w2 - 1], v);
+          } else if (n2 > 0) {
+            v = g2 * V[o - 1];
+            if (n2 > 1) v = fma(-H[5] * (double)(n2 - 1), V[o - 2], v);
+          }
+          V[o] = v;
+        }
+    for (int n0 = 0; n0 <= t0; n0++)
+      for (int n1 = 0; n1 <= t1; n1++) fold_line(V + n0 * w1 + n1 * w2, 1, t2, r2 + kRE + 5 * d);
+    for (int n0 = 0; n0 <= t0; n0++)
+      for (int n2 = 0; n2 <= t2; n2++) fold_line(V + n0 * w1 + n2, w2, t1, r1 + kRE + 5 * d);
+    for (int n1 = 0; n1 < w1; n1++) fold_line(V + n1, w1, t0, r0 + kRE + 5 * d);
+    const int n = t0 + t1 + t2;
+    for (int k = 0; k <= n; k++) b.W[d][k] = 0.0;
+    const double* v = V;
+    double p0 = 1.0;
+    for (int x0 = 0; x0 <= t0; x0++) {
+      double p01 = p0;
+      for (int x1 = 0; x1 <= t1; x1++) {
+        double p = p01;
+        for (int x2 = 0; x2 <= t2; x2++) {
+          b.W[d][x0 + x1 + x2] = fma(p, *v++, b.W[d][x0 + x1 + x2]);
+          if (x2 < t2) p *= cof[2];
+        }
+        if (x1 < t1) p01 *= cof[1];
+      }
+      if (x0 < t0) p0 *= cof[0];
+    }
+    b.N[d] = n;
+  }
+  *scale = exp(-ex);
 }
 
 // G4_MD_xgVepg's composite (XC1_G4_MD.f:1559-1978): e1 (r1), e2 (r2), proton
@@ -178,9 +291,12 @@ G3_HD void build_bra_vep(const double* r1, const double* r2, const double* rp,
   const R c[3][3] = {{R(1), R(0), R(-1)},
                      {C1 / (C1 + P4), R(-1), P4 / (C1 + P4)},
                      {R(0), R(0), R(0)}};
-  fold_bra<R, LE, LN, NW>(r1, r2, rp, 2, xi, c, cof, b);
+  R scale = R(1);
+  if constexpr (sizeof(R) == sizeof(float)) fold_bra<R, LE, LN, NW>(r1, r2, rp, 2, xi, c, cof, b);
+  else fold_bra<LE, LN, NW>(r1, r2, rp, 2, xi, c, cof, b, &scale);
   b.Z = Tx4;
   b.pref = C0 * CB0;
+  if constexpr (sizeof(R) != sizeof(float)) b.pref *= scale;
 }
 
 // G4_MD_xgVeeg's composite (XC1_G4_MD.f:796-1125): e1 (r1), e3 (r3), proton
@@ -206,9 +322,12 @@ G3_HD void build_bra_vee(const double* r1, const double* r3, const double* rp,
   const R c[3][3] = {{R(1), R(0), R(-1)},
                      {R(0), R(1), R(-1)},
                      {P1 / (P1 + C1), -P3 / (P3 + C3), C1 / (P1 + C1) - C3 / (P3 + C3)}};
-  fold_bra<R, LE, LN, NW>(r1, r3, rp, 3, xi, c, cof, b);
+  R scale = R(1);
+  if constexpr (sizeof(R) == sizeof(float)) fold_bra<R, LE, LN, NW>(r1, r3, rp, 3, xi, c, cof, b);
+  else fold_bra<LE, LN, NW>(r1, r3, rp, 3, xi, c, cof, b, &scale);
   b.Z = W1;
   b.pref = C0 * CB0;
+  if constexpr (sizeof(R) != sizeof(float)) b.pref *= scale;
 }
 
 // One (bra, ket) Coulomb integral, pref C4 sum_tuv W_x W_y W_z R_tuv, with
@@ -262,6 +381,283 @@ G3_HD double fb_eval(const Bra<R, NW>& b, R pk, const R* Xk, const R (*Ek)[NK + 
     return bm;
   });
   return (double)(b.pref * C4) * s;
+}
+
+// ---- FP64 evaluation -----------------------------------------------------------
+// The same integral with the fewest FP64 instructions (2 per SM and clock on
+// this GPU; integer and memory instructions beside them are free): one rsqrt
+// serves alpha and the prefactor, bra and ket are normalised so that the
+// common low orders multiply by nothing, (-alpha)^m is part of the Hermite
+// powers, and the Boys recursion has one loop for both ranges of T.  About
+// 120 instructions an evaluation where fb_eval<double> takes 230.
+
+#if defined(__CUDACC__)
+#define NX_LOOP _Pragma("unroll 1")
+#else
+#define NX_LOOP
+#endif
+
+G3_HD double rsqrt64(double x) {
+#if defined(__CUDA_ARCH__)
+  return rsqrt(x);
+#else
+  return 1.0 / sqrt(x);
+#endif
+}
+
+G3_HD long long bits64(double x) {
+#if defined(__CUDA_ARCH__)
+  return __double_as_longlong(x);
+#else
+  long long b;
+  memcpy(&b, &x, sizeof(b));
+  return b;
+#endif
+}
+
+// |x| < 1e-100 -> 0 (underflow.f:2-11), compared as integers (the bits of 1e-100)
+G3_HD double underflow_bits(double x) {
+  return (bits64(x) & 0x7fffffffffffffffLL) < 0x2b2bff2ee48e0530LL ? 0.0 : x;
+}
+
+// Gamma(L + 1/2) / 2, L = 0..16: F_L(T) ~ Gamma(L + 1/2) / (2 T^(L + 1/2))
+#define NX_ASYM_VALUES \
+    0.886226925452758, 0.443113462726379, 0.6646701940895685, 1.6616754852239213, \
+    5.815864198283724, 26.17138889227676, 143.94263890752217, 935.6271528988942, \
+    7017.2036467417065, 59646.230997304505, 566639.1944743928, 5949711.541981124, \
+    68421682.73278293, 855271034.1597866, 11546158961.15712, 167419304936.77823, \
+    2594999226520.0625
+#if defined(__CUDACC__)
+static __device__ const double kAsymDev[17] = {NX_ASYM_VALUES};
+#endif
+static const double kAsymHost[17] = {NX_ASYM_VALUES};
+#undef NX_ASYM_VALUES
+G3_HD double asym(int L) {
+#if defined(__CUDA_ARCH__)
+  return __ldg(&kAsymDev[L]);
+#else
+  return kAsymHost[L];
+#endif
+}
+
+// t! / ((2i-t)! (t-i)! 2^(t-i)), t, i <= 12 (zero unless i <= t <= 2i)
+#define NX_HERMX_VALUES \
+    1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 1.0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 0, 3.0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 0, 3.0, 6.0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 0, 0, 15.0, 10.0, 1.0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 0, 0, 15.0, 45.0, 15.0, 1.0, 0, 0, 0, 0, 0, 0, \
+    0, 0, 0, 0, 105.0, 105.0, 21.0, 1.0, 0, 0, 0, 0, 0, \
+    0, 0, 0, 0, 105.0, 420.0, 210.0, 28.0, 1.0, 0, 0, 0, 0, \
+    0, 0, 0, 0, 0, 945.0, 1260.0, 378.0, 36.0, 1.0, 0, 0, 0, \
+    0, 0, 0, 0, 0, 945.0, 4725.0, 3150.0, 630.0, 45.0, 1.0, 0, 0, \
+    0, 0, 0, 0, 0, 0, 10395.0, 17325.0, 6930.0, 990.0, 55.0, 1.0, 0, \
+    0, 0, 0, 0, 0, 0, 10395.0, 62370.0, 51975.0, 13860.0, 1485.0, 66.0, 1.0
+#if defined(__CUDACC__)
+static __device__ const double kHermXDev[13 * 13] = {NX_HERMX_VALUES};
+#endif
+static const double kHermXHost[13 * 13] = {NX_HERMX_VALUES};
+#undef NX_HERMX_VALUES
+G3_HD double hermx(int t, int i) {
+#if defined(__CUDA_ARCH__)
+  return __ldg(&kHermXDev[t * 13 + i]);
+#else
+  return kHermXHost[t * 13 + i];
+#endif
+}
+
+// The factors of F_i(alpha R^2) in sum_t W[t] d^t/dR^t F_0(alpha R^2), i <= n:
+//   A[i] = sum_t W[t] t! / ((2i-t)! (t-i)!) (-2 alpha R)^(2i-t) (-alpha)^(t-i)
+// with y = -2 alpha R and z = -2 alpha.  Orders up to 4 straight (s, p and
+// most d pairs), beyond by Horner in y.
+G3_HD void hermite_scaled(int n, const double* W, double y, double z, double* A) {
+  A[0] = W[0];
+  if (n == 0) return;
+  if (n == 1) {
+    A[1] = W[1] * y;
+    return;
+  }
+  const double a1 = fma(W[1], y, W[2] * z);
+  if (n == 2) {
+    A[1] = a1;
+    A[2] = W[2] * y * y;
+    return;
+  }
+  if (n == 3) {
+    const double w3 = W[3], y2 = y * y;
+    A[2] = fma(W[2], y, 3.0 * (w3 * z)) * y;
+    A[1] = a1;
+    A[3] = w3 * y2 * y;
+    return;
+  }
+  if (n == 4) {
+    const double w3 = W[3], w4 = W[4], y2 = y * y, w4z = w4 * z;
+    A[2] = fma(W[2], y2, 3.0 * (z * fma(w3, y, w4z)));
+    A[1] = a1;
+    A[3] = y2 * fma(w3, y, 6.0 * w4z);
+    A[4] = w4 * y2 * y2;
+    return;
+  }
+  double zp[7];
+  zp[0] = 1.0;
+  for (int k = 1; k <= n / 2; k++) zp[k] = zp[k - 1] * z;
+  double yp = 1.0;   // y^(2i - min(2i, n))
+  for (int i = 1; i <= n; i++) {
+    const int hi = 2 * i < n ? 2 * i : n;
+    double a = W[i];
+    for (int t = i + 1; t <= hi; t++) a = fma(a, y, W[t] * (hermx(t, i) * zp[t - i]));
+    if (2 * i > n) {
+      yp *= (2 * i == n + 1) ? y : y * y;
+      a *= yp;
+    }
+    A[i] = a;
+  }
+}
+
+// sum_m F_m(T) B[m], m <= L <= 16, with boys()'s Boys function: F_L from the
+// Taylor expansion (T <= 20) or the asymptotic form, and one downward
+// recursion F_m = (2T F_(m+1) + e) / (2m + 1) for both, e = exp(-T) or 0 (with
+// e = 0 it is the asymptotic form's F_(m+1) = F_m (m + 1/2) / T).
+G3_HD double boys_dot(int L, double T, const double* B) {
+  double f, e = 0.0;
+  if (bits64(T) <= 0x4034000000000000LL) {   // T <= 20 (T >= 0; NaN goes below)
+    const double kMagic = 6755399441055744.0;   // 1.5 * 2^52: its sum rounds 16 T to an integer
+    const double t = fma(T, 16.0, kMagic);
+    int g = (int)bits64(t);
+    g = g < 0 ? 0 : (g > kBoysRows - 1 ? kBoysRows - 1 : g);
+    const double d = fma(t - kMagic, 0.0625, -T);
+    const int row = g * kBoysCols;
+    const double d2 = d * 0.5, d3 = d * (1.0 / 3.0), d4 = d * 0.25, d5 = d * 0.2,
+                 d6 = d * (1.0 / 6.0);
+    f = boys_tab(row + L + 6);
+    f = fma(f, d6, boys_tab(row + L + 5));
+    f = fma(f, d5, boys_tab(row + L + 4));
+    f = fma(f, d4, boys_tab(row + L + 3));
+    f = fma(f, d3, boys_tab(row + L + 2));
+    f = fma(f, d2, boys_tab(row + L + 1));
+    f = fma(f, d, boys_tab(row + L));
+    if (L == 0) return f * B[0];
+    e = 1.0 + d6;   // exp(d), the same seven terms
+    e = fma(e, d5, 1.0);
+    e = fma(e, d4, 1.0);
+    e = fma(e, d3, 1.0);
+    e = fma(e, d2, 1.0);
+    e = fma(e, d, 1.0);
+    e *= boys_tab(row + kBoysCols - 1);
+  } else {
+    const double rs = rsqrt64(T), rT = rs * rs;
+    if (!(T < 1.0e15)) {   // T^-L would leave the range: upwards (and NaN)
+      double s = B[L];
+      for (int m = L; m >= 1; m--) s = fma(s, rT * ((double)m - 0.5), B[m - 1]);
+      return (0.886226925452758 * rs) * s;
+    }
+    f = asym(L) * rs;
+    double p = rT;
+    for (int k = L; k > 0; k >>= 1) {
+      if (k & 1) f *= p;
+      if (k > 1) p *= p;
+    }
+  }
+  double s = f * B[L];
+  const double t2 = T + T;
+  NX_LOOP
+  for (int m = L - 1; m >= 0; m--) {
+    f = fma(f, t2, e) * boys_rinv(m);
+    s = fma(f, B[m], s);
+  }
+  return s;
+}
+
+// B <- B (*) A, orders L and n (B has room for L + n + 1)
+G3_HD void convolve(double* B, int L, const double* A, int n) {
+  NX_LOOP
+  for (int m = L + n; m >= 0; m--) {
+    const int lo = m > L ? m - L : 0, hi = m < n ? m : n;
+    double b = A[lo] * B[m - lo];
+    for (int i = lo + 1; i <= hi; i++) b = fma(A[i], B[m - i], b);
+    B[m] = b;
+  }
+}
+
+// A bra of build_bra_* made ready: the ket-independent part of the Coulomb
+// prefactor into pref, and orderless directions' W into it as well.
+template <int NW>
+G3_HD void finish_bra(Bra<double, NW>& b) {
+  b.pref *= 34.98683665524963 / b.Z;   // 2 pi^(5/2) of the truncated pi
+  for (int d = 0; d < 3; d++)
+    if (b.N[d] == 0) {
+      b.pref *= b.W[d][0];
+      b.W[d][0] = 1.0;
+    }
+}
+
+// The free electron's pair density, from its record: Hermite coefficients
+// with (-1)^t over the top one, whose product is in f (with 1/p).
+template <int NK>
+struct Ket {
+  double p, f, X[3], e[3][NK > 0 ? NK : 1];
+  int t[3];
+};
+template <int NK>
+G3_HD void load_ket(const double* rk, Ket<NK>& k) {
+  k.p = rk[kRP];
+  double f = 1.0 / k.p;
+  for (int d = 0; d < 3; d++) {
+    const int n = (int)rk[kRT + d];
+    const double* E = rk + kRE + 5 * d;
+    k.X[d] = rk[kRX + d];
+    k.t[d] = n;
+    const double top = E[n];   // K / (2p)^n: zero only where K underflowed
+    const double r = top != 0.0 ? 1.0 / top : 0.0;
+    f *= (n & 1) ? -top : top;
+    if (NK > 0)
+      for (int q = 0; q < n; q++) k.e[d][q] = ((n - q) & 1) ? -(E[q] * r) : E[q] * r;
+  }
+  k.f = f;
+}
+
+// One (finished bra, ket) integral.
+template <int NW, int NK>
+G3_HD double fb_value(const Bra<double, NW>& b, const Ket<NK>& k) {
+  constexpr int NT = NW + NK;
+  const double rs = rsqrt64(b.Z + k.p), z = b.Z * k.p * (rs * rs);   // z: alpha
+  double R[3], R2 = 0.0;
+  for (int d = 0; d < 3; d++) {
+    R[d] = b.C[d] - k.X[d];
+    R2 = fma(R[d], R[d], R2);
+  }
+  const double T = z * R2, m2 = -(z + z);
+  double B[3 * NT + 1];
+  B[0] = 1.0;
+  int L = 0;
+  NX_LOOP
+  for (int d = 0; d < 3; d++) {
+    const int nb = b.N[d], tk = NK > 0 ? k.t[d] : 0, n = nb + tk;
+    if (n == 0) continue;   // W = 1 after the normalisations
+    double Wc[NT + 1];
+    const double* W = b.W[d];
+    if (tk > 0) {   // Wc[m] = W[m - tk] + sum_q e[q] W[m - q]
+      for (int m = 0; m <= n; m++) {
+        double w = m >= tk ? b.W[d][m - tk] : 0.0;
+        for (int q = 0; q < tk; q++)
+          if (m >= q && m - q <= nb) w = fma(k.e[d][q], b.W[d][m - q], w);
+        Wc[m] = w;
+      }
+      W = Wc;
+    }
+    const double y = m2 * R[d];
+    if (L == 0) {
+      hermite_scaled(n, W, y, m2, B);
+    } else {
+      double A[NT + 1];
+      hermite_scaled(n, W, y, m2, A);
+      convolve(B, L, A, n);
+    }
+    L += n;
+  }
+  return (b.pref * k.f) * rs * boys_dot(L, T, B);
 }
 
 }  // namespace g3

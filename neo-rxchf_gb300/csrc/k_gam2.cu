@@ -211,14 +211,8 @@ gam2_pair_kernel(DevSystem S, const double* __restrict__ grad, int Pp0, long lon
   const bool on = pos < v.nket;
   const int kid = on ? v.kperm[pos] : 0;
   const double* rk = v.erec + (size_t)kRLen * kid;
-  double Xk[3], Ek[3][NK + 1];
-  int tk[3];
-  for (int d = 0; d < 3; d++) {
-    Xk[d] = rk[kRX + d];
-    tk[d] = (int)rk[kRT + d];
-    for (int t = 0; t <= NK; t++) Ek[d][t] = (t & 1) ? -rk[kRE + 5 * d + t] : rk[kRE + 5 * d + t];
-  }
-  const double pk = rk[kRP];
+  g3::Ket<NK> ket;
+  g3::load_ket<NK>(rk, ket);
   Bra<double, NW>* bras = s_bra[wid];
   double acc = 0.0;
   for (int c0 = b0; c0 < b1; c0 += 32) {
@@ -232,14 +226,15 @@ gam2_pair_kernel(DevSystem S, const double* __restrict__ grad, int Pp0, long lon
       double g, w;
       pair_term(S, q0 + q / nb, g, w);
       Bra<double, NW>& b = bras[lane];
-      if (kind == 0) build_bra_pair<double, 2 * LE, 2 * LN, NW>(rb, rp, g, b);
-      else build_bra_pair<double, 2 * LN, 2 * LE, NW>(rp, rb, g, b);
+      if (kind == 0) build_bra_pair<2 * LE, 2 * LN, NW>(rb, rp, g, b);
+      else build_bra_pair<2 * LN, 2 * LE, NW>(rp, rb, g, b);
+      g3::finish_bra<NW>(b);
       b.wgt = (kind == 0 ? w : -w) * rb[kRC] * rp[kRC];
     }
     __syncwarp();
     if (on)
       for (int i = 0; i < nv; i++)
-        acc = fma(bras[i].wgt, g3::fb_eval<double, NW, NK>(bras[i], pk, Xk, Ek, tk), acc);
+        acc = fma(bras[i].wgt, g3::fb_value<NW, NK>(bras[i], ket), acc);
   }
   if (on) Y[((long long)split * nunit + u) * v.nket + kid] = acc * rk[kRC];
 }

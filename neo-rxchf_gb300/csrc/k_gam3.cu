@@ -31,7 +31,7 @@
 //     not depend on the ket, so a CTA builds the bras of one canonical
 //     (proton pair, electron pair, electron pair) -- every primitive pair and
 //     geminal pair -- once in shared memory and sweeps all primitive-pair
-//     kets against them.  Per (bra, ket) (g3_fatbra.cuh fb_eval):
+//     kets against them.  Per (bra, ket) (g3_fatbra.cuh fb_eval, fb_value):
 //       W_d = W'_d (*) (-1)^t E_d                 (1-D convolutions)
 //       S   = sum_{t,u,v} W_x[t] W_y[u] W_z[v] R_tuv(alpha, R)
 //           = sum_m (-alpha)^m F_m(T) sum_{i+j+k=m} A_x[i] A_y[j] A_z[k],
@@ -39,6 +39,13 @@
 //     the Hermite-Coulomb sum in factorised form, O(L^2) work instead of
 //     the O(L^4) R_tuv table; the seeds (-alpha)^m F_m(T) and their final
 //     sum are FP64 in both precisions.
+//
+// FP64 instructions bound the FP64 build (2 per SM and clock): fb_value takes
+// about half of fb_eval's, G4Vep runs over unordered (e1, e2) pairs, the bras
+// fold one particle at a time, and warps share (32 kets, a quarter of the
+// bras) units so that none idles in a last round of few kets.  Measured (one
+// GB300, neoxc_gam3_ic1): nebf = 6 s/p of 3 primitives, npbf = 4 s/p/d,
+// NG = 3: 516 -> 279 ms; FP32 tables at nebf = 4, npbf = 2: 6.5 -> 3.8 ms.
 //
 // The prefactors, exponents and centres follow G4_MD_xgVepg / G4_MD_xgVeeg
 // (truncated pi, the reference's underflow on every G4Vep value); only the
@@ -60,6 +67,7 @@
 // grid drains through a device counter (gam3_fb_persistent); the per-block
 // arithmetic is that of gam3_fb_kernel, so each system's R4 is bit-identical
 // to its separate build.
+#include <algorithm>
 #include <type_traits>
 #include <vector>
 
@@ -117,6 +125,9 @@ __global__ void g3_records_kernel(DevSystem S, double* __restrict__ erec,
 }
 
 constexpr int kFbThreads = 128;   // threads (and bras per chunk) of a CTA
+constexpr int kFbShares = 4;      // shares of a chunk's bras that warps take
+
+__host__ __device__ __forceinline__ int nPe_of(int ne) { return ne * (ne + 1) / 2; }
 
 // One CTA's work: block blk (Pp, Pa, Pb) and ket tile `tile` of one pass.
 // MODE 0: G4Vep, (Pp, P1, P2), kets e3 -> R4[Pp][P1][P2][P3]  = -sum
@@ -132,6 +143,11 @@ __device__ __forceinline__ void fb_block(const DevSystem& S, const double* __res
   using R = typename std::conditional<F32, float, double>::type;
   constexpr int NW = 4 * LE + 2 * LN;   // bra Hermite order per direction
   constexpr int NK = 2 * LE;            // ket Hermite order per direction
+  // G4Vep summed over (k, l) does not change when e1 and e2 are exchanged, so
+  // the FP64 pass takes P1 >= P2 only.  (The FP32 bras of the two orders
+  // round differently; that pass keeps both.)
+  constexpr bool kHalf = !F32 && MODE == 0;
+  if (kHalf && blk / nPe_of(S.nebf) % nPe_of(S.nebf) < blk % nPe_of(S.nebf)) return;
   __syncthreads();   // the previous block's reads of the shared tables are done
   Bra<R, NW>* bras = reinterpret_cast<Bra<R, NW>*>(smraw);
   double* acc_s = reinterpret_cast<double*>(smraw + sizeof(Bra<R, NW>) * kFbThreads);
@@ -158,7 +174,10 @@ __device__ __forceinline__ void fb_block(const DevSystem& S, const double* __res
     for (int k = 0; k < ng; k++)
       for (int l = 0; l < ng; l++) wsum += fabs(S.bgem[k] * S.bgem[l]);
 
-  for (int k = threadIdx.x; k < nkt; k += blockDim.x) acc_s[k] = 0.0;
+  // Lane sums of ket kk, one row per bra share: acc_s[share * nkt + kk]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ngrp = (nkt + 31) / 32;
+  for (int k = threadIdx.x; k < kFbShares * nkt; k += blockDim.x) acc_s[k] = 0.0;
   for (int c0 = 0; c0 < nbra; c0 += kFbThreads) {
     const int nvalid = nbra - c0 < kFbThreads ? nbra - c0 : kFbThreads;
     __syncthreads();
@@ -175,6 +194,7 @@ __device__ __forceinline__ void fb_block(const DevSystem& S, const double* __res
         build_bra_vep<R, LE, LN, NW>(ra, rb, rp, (R)S.ggem[k], (R)S.ggem[l], b);
       else
         build_bra_vee<R, LE, LN, NW>(ra, rb, rp, (R)S.ggem[k], (R)S.ggem[l], b);
+      if constexpr (!F32) finish_bra<NW>(b);
       b.wgt = (MODE == 0 ? -1.0 : 2.0) * (S.bgem[k] * S.bgem[l]) * ra[kRC] * rb[kRC] *
               rp[kRC];
       // Vep: S1 S2 Qp (x Q3 of the ket); Vee: Q1 S3 Sp (x Q2 of the ket)
@@ -183,42 +203,64 @@ __device__ __forceinline__ void fb_block(const DevSystem& S, const double* __res
       bras[threadIdx.x] = b;
     }
     __syncthreads();
-    for (int kk = threadIdx.x; kk < nkt; kk += blockDim.x) {
+    // Warps take (32 kets, share of the bras): with all the kets on the CTA's
+    // threads, a last round of few kets left most of its warps idle.
+    const int nsh = nvalid >= 16 ? kFbShares : (nvalid >= 8 ? 2 : 1);
+    for (int unit = warp; unit < ngrp * nsh; unit += kFbThreads / 32) {
+      const int grp = unit / nsh, sh = unit - grp * nsh;
+      const int i0 = nvalid * sh / nsh, i1 = nvalid * (sh + 1) / nsh;
+      const int kk = grp * 32 + lane;
+      if (kk >= nkt) continue;
       const int kid = kperm[k0 + kk];
       const double* rk = erec + (size_t)kRLen * kid;
-      const R pk = (R)rk[kRP];
-      R Xk[3], Ek[3][NK + 1];
-      int tk[3];
-      for (int d = 0; d < 3; d++) {
-        Xk[d] = (R)rk[kRX + d];
-        tk[d] = (int)rk[kRT + d];
-        for (int t = 0; t <= NK; t++)
-          Ek[d][t] = (t & 1) ? -(R)rk[kRE + 5 * d + t] : (R)rk[kRE + 5 * d + t];
-      }
       const double qk = rk[kRQ];
       const double rkc = rk[kRC];
       double part = 0.0;
-      for (int bi = 0; bi < nvalid; bi++) {
-        const Bra<R, NW>& b = bras[bi];
-        if (screen > 0.0 && b.est * qk < screen) continue;
-        double v = fb_eval<R, NW, NK>(b, pk, Xk, Ek, tk);
-        if (MODE == 0) v = md::underflow(v);   // zz = underflow(G4_MD_xgVepg)
-        part += b.wgt * v;
+      if constexpr (F32) {
+        const R pk = (R)rk[kRP];
+        R Xk[3], Ek[3][NK + 1];
+        int tk[3];
+        for (int d = 0; d < 3; d++) {
+          Xk[d] = (R)rk[kRX + d];
+          tk[d] = (int)rk[kRT + d];
+          for (int t = 0; t <= NK; t++)
+            Ek[d][t] = (t & 1) ? -(R)rk[kRE + 5 * d + t] : (R)rk[kRE + 5 * d + t];
+        }
+        for (int bi = i0; bi < i1; bi++) {
+          const Bra<R, NW>& b = bras[bi];
+          if (screen > 0.0 && b.est * qk < screen) continue;
+          double v = fb_eval<R, NW, NK>(b, pk, Xk, Ek, tk);
+          if (MODE == 0) v = underflow_bits(v);   // zz = underflow(G4_MD_xgVepg)
+          part += b.wgt * v;
+        }
+      } else {
+        Ket<NK> ket;
+        load_ket<NK>(rk, ket);
+        for (int bi = i0; bi < i1; bi++) {
+          const Bra<R, NW>& b = bras[bi];
+          if (screen > 0.0 && b.est * qk < screen) continue;
+          double v = fb_value<NW, NK>(b, ket);
+          if (MODE == 0) v = underflow_bits(v);
+          part = fma(b.wgt, v, part);
+        }
       }
-      acc_s[kid - k0] += part * rkc;
+      acc_s[sh * nkt + kid - k0] += part * rkc;
     }
   }
   __syncthreads();
   const long long nP = nPe;
   for (int P = P0 + threadIdx.x; P < P1t; P += blockDim.x) {
     double s = 0.0;
-    for (int k = kofs[P]; k < kofs[P + 1]; k++) s += acc_s[k - k0];
-    if (MODE == 0)
+    for (int sh = 0; sh < kFbShares; sh++)
+      for (int k = kofs[P]; k < kofs[P + 1]; k++) s += acc_s[sh * nkt + k - k0];
+    if (MODE == 0) {
       r4[((Pp * nP + Pa) * nP + Pb) * nP + P] = s;
-    else if (store1)
+      if (kHalf && Pa != Pb) r4[((Pp * nP + Pb) * nP + Pa) * nP + P] = s;
+    } else if (store1) {
       r4[((Pp * nP + Pa) * nP + P) * nP + Pb] = s;
-    else
+    } else {
       r4[((Pp * nP + Pa) * nP + P) * nP + Pb] += s;
+    }
   }
 }
 
@@ -312,13 +354,19 @@ __global__ void gam3_expand_kernel(int ne, int np, const double* __restrict__ au
   }
 }
 
+// kets: the most kets of a tile
+template <class R, int NW>
+size_t fb_smem(int kets) {
+  return sizeof(Bra<R, NW>) * kFbThreads + sizeof(double) * (size_t)kFbShares * kets;
+}
+
 template <bool F32, int LE, int LN>
-cudaError_t persistent_t(const G3BatchSys* d_sys, const long long* d_prefix, int ngroups,
+cudaError_t persistent_t(int kets, const G3BatchSys* d_sys, const long long* d_prefix, int ngroups,
                          int chunk, long long limit, double screen,
                          unsigned long long* d_counter, int ctas_per_sm, cudaStream_t s) {
   using R = typename std::conditional<F32, float, double>::type;
   constexpr int NW = 4 * LE + 2 * LN;
-  const size_t smem = sizeof(Bra<R, NW>) * kFbThreads + sizeof(double) * kG3MaxTileKets;
+  const size_t smem = fb_smem<R, NW>(kets);
   cudaError_t e = cudaFuncSetAttribute(gam3_fb_persistent<F32, LE, LN>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -336,12 +384,12 @@ cudaError_t persistent_t(const G3BatchSys* d_sys, const long long* d_prefix, int
 }
 
 template <bool F32>
-cudaError_t persistent_dispatch(int le, int lp, const G3BatchSys* d_sys,
+cudaError_t persistent_dispatch(int kets, int le, int lp, const G3BatchSys* d_sys,
                                 const long long* d_prefix, int ngroups, int chunk,
                                 long long limit, double screen, unsigned long long* d_counter,
                                 int ctas_per_sm, cudaStream_t s) {
   const int LN = lp == 0 ? 0 : 2;
-#define PD(a, b) persistent_t<F32, a, b>(d_sys, d_prefix, ngroups, chunk, limit, screen, \
+#define PD(a, b) persistent_t<F32, a, b>(kets, d_sys, d_prefix, ngroups, chunk, limit, screen, \
                                          d_counter, ctas_per_sm, s)
   switch (le * 3 + LN) {
     case 0: return PD(0, 0);
@@ -360,7 +408,7 @@ cudaError_t fb_t(const DevSystem& sys, const double* erec, const double* prec,
                  double screen, double* r4, cudaStream_t s) {
   using R = typename std::conditional<F32, float, double>::type;
   constexpr int NW = 4 * LE + 2 * LN;
-  const size_t smem = sizeof(Bra<R, NW>) * kFbThreads + sizeof(double) * kG3MaxTileKets;
+  const size_t smem = fb_smem<R, NW>(std::min(sys.g3_nket, kG3MaxTileKets));
   const int nPe = sys.nebf * (sys.nebf + 1) / 2;
   const int nPp = sys.npbf * (sys.npbf + 1) / 2;
   const long long nblk = (long long)nPp * nPe * nPe;
@@ -418,10 +466,12 @@ cudaError_t launch_gam3_batch_pairs(const G3BatchSys* h_sys, int nsys, int fp32,
   if (nsys < 1 || chunk < 1) return cudaErrorInvalidValue;
   const int le = h_sys[0].S.lmax_e, lp = h_sys[0].S.lmax_p;
   std::vector<long long> prefix(2 * (size_t)nsys + 1, 0);
+  int kets = 0;
   for (int k = 0; k < nsys; k++) {
     const DevSystem& S = h_sys[k].S;
     if (S.lmax_e != le || (S.lmax_p == 0) != (lp == 0) || S.g3_ntile < 1 || !S.g3i || !S.g3rec)
       return cudaErrorInvalidValue;   // one angular class per launch
+    kets = std::max(kets, std::min(S.g3_nket, kG3MaxTileKets));
     const long long nPe = (long long)S.nebf * (S.nebf + 1) / 2;
     const long long nPp = (long long)S.npbf * (S.npbf + 1) / 2;
     const long long items = nPp * nPe * nPe * S.g3_ntile;
@@ -446,9 +496,9 @@ cudaError_t launch_gam3_batch_pairs(const G3BatchSys* h_sys, int nsys, int fp32,
   e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return e;
   const long long lim = limit < 0 ? prefix[2 * nsys] : limit;
-  return fp32 ? persistent_dispatch<true>(le, lp, d_sys, d_prefix, 2 * nsys, chunk, lim, screen,
+  return fp32 ? persistent_dispatch<true>(kets, le, lp, d_sys, d_prefix, 2 * nsys, chunk, lim, screen,
                                           d_counter, ctas_per_sm, s)
-              : persistent_dispatch<false>(le, lp, d_sys, d_prefix, 2 * nsys, chunk, lim, screen,
+              : persistent_dispatch<false>(kets, le, lp, d_sys, d_prefix, 2 * nsys, chunk, lim, screen,
                                            d_counter, ctas_per_sm, s);
 }
 

@@ -79,17 +79,14 @@ void hc_gam2(const HP* hA, const HP* hB, int ng, const double* gm, int nat, cons
   static thread_local G3 st;
   const double gm6[6] = {0.0, 0.0, gm[0], 0.0, 0.0, 0.0};
   g3::Bra<double, 8> b;
-  double Ek[3][5], X[3];
-  int tk[3];
-  for (int d = 0; d < 3; d++) {
-    X[d] = r[0][g3::kRX + d];
-    tk[d] = (int)r[0][g3::kRT + d];
-    for (int t = 0; t < 5; t++) Ek[d][t] = (t & 1) ? -r[0][g3::kRE + 5 * d + t] : r[0][g3::kRE + 5 * d + t];
-  }
-  g2::build_bra_pair<double, 4, 4, 8>(r[1], r[2], gm[0], b);
-  pair[0] = g3::fb_eval<double, 8, 4>(b, r[0][g3::kRP], X, Ek, tk);
-  g2::build_bra_pair<double, 4, 4, 8>(r[2], r[1], gm[0], b);
-  pair[1] = g3::fb_eval<double, 8, 4>(b, r[0][g3::kRP], X, Ek, tk);
+  g3::Ket<4> ket;
+  g3::load_ket<4>(r[0], ket);
+  g2::build_bra_pair<4, 4, 8>(r[1], r[2], gm[0], b);
+  g3::finish_bra<8>(b);
+  pair[0] = g3::fb_value<8, 4>(b, ket);
+  g2::build_bra_pair<4, 4, 8>(r[2], r[1], gm[0], b);
+  g3::finish_bra<8>(b);
+  pair[1] = g3::fb_value<8, 4>(b, ket);
   md::g3_setup(st, A, B, gm6, 0);
   pair[2] = md::g3_vee(st);
   Prim A3[3], B3[3];
@@ -99,5 +96,13 @@ void hc_gam2(const HP* hA, const HP* hB, int ng, const double* gm, int nat, cons
   pair[3] = md::g3_vee(st);
   ov[0] = g2::two_body_overlap(r[0], r[2], gm[0]);
   ov[1] = md::g2_xggs(A[0], A[2], B[0], B[2], gm[0], 0.0);
+}
+
+double hc_boys_dot(int L, double T, const double* B) { return g3::boys_dot(L, T, B); }
+double hc_boys_ref(int L, double T, const double* B) {
+  double F[32], s = 0.0;
+  boys(L, T, F);
+  for (int m = 0; m <= L; m++) s += F[m] * B[m];
+  return s;
 }
 }

@@ -57,6 +57,25 @@ def test_pair_density_integrals_match_element_integrals(host, le, ln):
             assert abs(x - y) <= 1e-10 * abs(y) + 1e-14 * max(abs(pair).max(), abs(ov).max())
 
 
+@pytest.mark.parametrize("L", [0, 1, 2, 7, 12, 16])
+def test_boys_dot_is_the_boys_function(host, L):
+    """One recursion for both ranges of T: the table's grid points and their
+    midpoints, the branch at T = 20, tiny, large and enormous T (positive
+    weights, so the sum has the relative accuracy of its terms)."""
+    host.hc_boys_dot.restype = host.hc_boys_ref.restype = C.c_double
+    rng = np.random.Generator(np.random.PCG64(L))
+    T = [0.0, 1e-300, 1e-12, 1 / 32, 1 / 16, 19.96875, np.nextafter(20, 0), 20.0, np.nextafter(20, 21), 35.0, 1e4,
+         1e14, 1e16, 1e60] + list(rng.uniform(0, 40, 200))
+    for t in T:
+        B = rng.uniform(0.1, 1.0, L + 1)
+        if t > 1e14:
+            B[:] = 0.0
+            B[0] = 1.0
+        x, y = (f(L, C.c_double(t), B.ctypes.data_as(C.c_void_p)) for f in (host.hc_boys_dot, host.hc_boys_ref))
+        assert abs(x - y) <= 2e-14 * abs(y), (t, x, y)
+    assert np.isnan(host.hc_boys_dot(L, C.c_double(float("nan")), B.ctypes.data_as(C.c_void_p)))
+
+
 def _system(**kw):
     from neoxc import basis
     return basis.synthetic(**kw)
