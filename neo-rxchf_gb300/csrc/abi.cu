@@ -141,7 +141,7 @@ int need(bool ok, const char* what) {
 // ---- basis staging for the MD builders ------------------------------------
 struct SysUpload {
   DevSystem d{};
-  DBuf eprim, pprim, kps, kpe, zan, cat, bgem, ggem, g3i, g3rec;
+  DBuf eprim, pprim, kps, kpe, zan, cat, bgem, ggem, g3i, g3rec, g3grad;
 };
 
 int stage_system(SysUpload& u, cudaStream_t s, int64_t nebf, int64_t npebf,
@@ -289,7 +289,9 @@ int stage_system(SysUpload& u, cudaStream_t s, int64_t nebf, int64_t npebf,
     u.d.g3i = u.g3i.as<int>();
     RC(dalloc(u.g3rec, sizeof(double) * g3_record_doubles(nket, (int)npbf), s));
     u.d.g3rec = u.g3rec.as<double>();
-    CU(launch_g3_records(u.d, const_cast<double*>(u.d.g3rec), s));
+    RC(dalloc(u.g3grad, sizeof(double) * g3_gradient_doubles(nket, (int)npbf), s));
+    u.d.g3grad = u.g3grad.as<double>();
+    CU(launch_g3_records(u.d, u.g3rec.as<double>(), u.g3grad.as<double>(), s));
   }
   return NEOXC_OK;
 }
@@ -299,6 +301,15 @@ int build_gam2(const DevSystem& d, int rx, double* x1, double* x2, cudaStream_t 
   DBuf scr;
   RC(dalloc(scr, sizeof(double) * gam2_scratch_doubles(d, rx, d.npbf * (d.npbf + 1) / 2), s));
   CU(launch_gam2_build(d, rx, scr.as<double>(), x1, x2, s));
+  return NEOXC_OK;
+}
+
+// The separable gam_3 factors (launch_gam3_aux), with the scratch they take.
+int build_gam3_aux(const DevSystem& d, double* aux, cudaStream_t s, const double* gee_in = nullptr,
+                   const double* hc_in = nullptr, const double* w3_in = nullptr) {
+  DBuf scr;
+  RC(dalloc(scr, sizeof(double) * gam2_scratch_doubles(d, 1, d.npbf * (d.npbf + 1) / 2), s));
+  CU(launch_gam3_aux(d, aux, scr.as<double>(), s, gee_in, hc_in, w3_in));
   return NEOXC_OK;
 }
 
@@ -534,7 +545,7 @@ int neoxc_gam3_ic1_opts(int64_t options, int64_t Nchunks, int64_t nebf, int64_t 
     CU(cudaEventCreate(&ev[1]));
     CU(cudaEventRecord(ev[0], s));
   }
-  CU(launch_gam3_aux(u.d, aux.as<double>(), s));
+  RC(build_gam3_aux(u.d, aux.as<double>(), s));
   CU(launch_gam3_raw(u.d, aux.as<double>(), d.as<double>(), s,
                      (options & NEOXC_SCF_MIXED) ? 1 : 0,
                      (options & NEOXC_SCF_SCREEN) ? kScreenThreshold : 0.0));
@@ -654,7 +665,7 @@ int neoxc_gam3_ic1_batch(const neoxc_xchf_job* jobs, int64_t njobs, int64_t opti
   CU(cudaEventCreate(&ev[1]));
   RC(finish(s));
   CU(cudaEventRecord(ev[0], s));
-  for (int64_t k = 0; k < njobs; k++) CU(launch_gam3_aux(up[k].d, aux[k].as<double>(), s));
+  for (int64_t k = 0; k < njobs; k++) RC(build_gam3_aux(up[k].d, aux[k].as<double>(), s));
   // one persistent launch per angular class
   std::map<int, std::vector<int64_t>> classes;
   for (int64_t k = 0; k < njobs; k++) classes[g3_tune_key(up[k].d, fp32)].push_back(k);
@@ -1187,7 +1198,7 @@ static int gam3_dscf_dev(const SysUpload& u, cudaStream_t s, const double* dde,
   RC(dalloc(slice, sizeof(double) * n6, s));
   RC(dalloc(part, sizeof(double) * eg3_partial_doubles(ne, np), s));
   RC(dalloc(aux, sizeof(double) * gam3_aux_doubles(ne, np), s));
-  CU(launch_gam3_aux(u.d, aux.as<double>(), s));
+  RC(build_gam3_aux(u.d, aux.as<double>(), s));
   CU(launch_gam3_pairs(u.d, aux.as<double>(), s, 0, 0.0));
   CU(launch_eg3_weights(ne, dde, part.as<double>(), s));
   for (int64_t pp = 0; pp < (int64_t)np * np; pp++) {
@@ -1422,7 +1433,7 @@ static int onebody_impl(int64_t nebf, int64_t npebf, int64_t npbf, int64_t nat,
   if (want_g1) {
     RC(dalloc(g1, sizeof(double) * n1, s));
     RC(dalloc(g1s, sizeof(double) * n1, s));
-    CU(launch_gam1(u.d, g1.as<double>(), g1s.as<double>(), s, 0, gam1_pairs_only));
+    CU(launch_gam1(u.d, g1.as<double>(), g1s.as<double>(), s, gam1_pairs_only));
     RC(back(GAM_1, g1, n1));
     RC(back(GAM_1s, g1s, n1));
   }
@@ -1740,7 +1751,7 @@ static int xchf_scf_on(cudaStream_t s, int64_t nelec, int64_t nucst, int64_t neb
   CU(launch_scf_onebody(u.d, Se.as<double>(), Sp.as<double>(), Hce.as<double>(),
                         Hcp.as<double>(), s));
   CU(launch_gam_ep(u.d, Gep.as<double>(), s));
-  CU(launch_gam1(u.d, G1.as<double>(), G1s.as<double>(), s, 0));
+  CU(launch_gam1(u.d, G1.as<double>(), G1s.as<double>(), s));
   CU(launch_gam_ee(u.d, Gee.as<double>(), s));
   if (nelec > 1) {
     RC(build_gam2(u.d, 0, G2.as<double>(), G2s.as<double>(), s));
@@ -1748,8 +1759,10 @@ static int xchf_scf_on(cudaStream_t s, int64_t nelec, int64_t nucst, int64_t neb
   if (nelec > 2) {
     DBuf aux;
     RC(dalloc(aux, sizeof(double) * gam3_aux_doubles(ne, np), s));
-    // GAM_ee and the core Hamiltonian (Hce, pack_2D order) are already built
-    CU(launch_gam3_aux(u.d, aux.as<double>(), s, Gee.as<double>(), Hce.as<double>()));
+    // GAM_ee, the core Hamiltonian (Hce, pack_2D order) and W3 (= GM2sICR) are
+    // already built
+    RC(build_gam3_aux(u.d, aux.as<double>(), s, Gee.as<double>(), Hce.as<double>(),
+                      G2s.as<double>()));
     CU(launch_gam3_raw(u.d, aux.as<double>(), G3.as<double>(), s, mixed,
                        (options & NEOXC_SCF_SCREEN) ? kScreenThreshold : 0.0));
     CU(launch_gam3_symmetrize(ne, np, G3.as<double>(), s));
@@ -2773,7 +2786,7 @@ int xcuhf_scf_on(cudaStream_t s, int64_t nelec, int64_t NAE, int64_t NBE, int64_
   CU(launch_scf_onebody(u.d, Se.as<double>(), Sp.as<double>(), Hce.as<double>(),
                         Hcp.as<double>(), s));
   CU(launch_gam_ep(u.d, Gep.as<double>(), s));
-  CU(launch_gam1(u.d, G1.as<double>(), G1s.as<double>(), s, 0));
+  CU(launch_gam1(u.d, G1.as<double>(), G1s.as<double>(), s));
   CU(launch_gam_ee(u.d, Gee.as<double>(), s));
   if (nelec > 1) {
     RC(build_gam2(u.d, 0, G2.as<double>(), G2s.as<double>(), s));
@@ -2781,7 +2794,8 @@ int xcuhf_scf_on(cudaStream_t s, int64_t nelec, int64_t NAE, int64_t NBE, int64_
   if (nelec > 2) {
     DBuf aux;
     RC(dalloc(aux, sizeof(double) * gam3_aux_doubles(ne, np), s));
-    CU(launch_gam3_aux(u.d, aux.as<double>(), s, Gee.as<double>(), Hce.as<double>()));
+    RC(build_gam3_aux(u.d, aux.as<double>(), s, Gee.as<double>(), Hce.as<double>(),
+                      G2s.as<double>()));
     CU(launch_gam3_raw(u.d, aux.as<double>(), G3.as<double>(), s, mixed,
                        (options & NEOXC_SCF_SCREEN) ? kScreenThreshold : 0.0));
     CU(launch_gam3_symmetrize(ne, np, G3.as<double>(), s));
@@ -3054,7 +3068,7 @@ int rx_scf_on(cudaStream_t s, int64_t kind, int64_t NAE, int64_t NAalpE, int64_t
   RC(dalloc(G2x, sizeof(double) * ng2, s));
   CU(launch_scf_onebody(u.d, Se.as<double>(), Sp.as<double>(), Hce.as<double>(),
                         Hcp.as<double>(), s));
-  CU(launch_gam1(u.d, G1.as<double>(), G1s.as<double>(), s, 0, 1));
+  CU(launch_gam1(u.d, G1.as<double>(), G1s.as<double>(), s, 1));
   CU(launch_gam_ee(u.d, Gee.as<double>(), s));
   RC(build_gam2(u.d, 1, G2.as<double>(), G2x.as<double>(), s));
   // SCF state

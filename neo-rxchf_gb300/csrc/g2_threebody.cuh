@@ -81,16 +81,22 @@ G3_HD double coulomb_sum(const int* n, const double (*W)[NT + 1], const double* 
   return g3::boys_dot(n[0] + n[1] + n[2], T, B);
 }
 
-// One primitive triple and geminal pair.  FULL: *x1 = the Coulomb, nuclear
+// What three_body evaluates: everything of the symmetrised gam_2 integrand
+// that couples all three particles, 1/r_12 alone, or the overlap alone.
+enum TripleMode { kAll = 0, kCoulomb12 = 1, kOverlap = 2 };
+
+// One primitive triple and geminal pair.  kAll: *x1 = the Coulomb, nuclear
 // and kinetic terms of the symmetrised gam_2 integrand that couple all three
 // particles, <gk(1p) gl(2p)| 1/r_12 - 1/r_1p - 1/r_2p + sum_C Z (1/r_pC -
-// 1/r_1C - 1/r_2C) + T_p + (T_1 + T_2)/2 as above |>, *x2 = the overlap; else
-// *x2 = the 1/r_12 term alone (the RXCHF-ne exchange tensor).
-template <int LE, int LN, bool FULL>
+// 1/r_1C - 1/r_2C) + T_p + (T_1 + T_2)/2 as above |>, *x2 = the overlap;
+// kCoulomb12: *x2 = the 1/r_12 term (the RXCHF-ne exchange tensor);
+// kOverlap: *x2 = the overlap.
+template <int LE, int LN, int MODE>
 G3_HD void three_body(const double* r1, const double* r2, const double* rp, const double* e1,
                       const double* e2, const double* ep, double gk, double gl, int nat,
                       const double* cat, const double* zan, double rpmass, double* x1,
                       double* x2) {
+  constexpr bool FULL = MODE == kAll;
   constexpr int M1 = 2 * LE, M3 = 2 * LN;         // largest Hermite orders of a pair
   constexpr int K = FULL ? 2 : 0;                 // kinetic extension of D
   constexpr int S2 = M3 + K + 1, S1 = (M1 + K + 1) * S2;   // strides of D
@@ -206,6 +212,20 @@ G3_HD void three_body(const double* r1, const double* r2, const double* rp, cons
         kin2[d] = fma(-0.5, d2, q2);
         kin3[d] = fma(0.5, q3, -0.25 * (d1 + d2));
       }
+      if constexpr (MODE == kOverlap) {
+        double x = 0.0;
+        for (int a = 0; a <= t1; a++) {
+          double y = 0.0;
+          for (int b = 0; b <= t2; b++) {
+            double z = D[a * S1 + b * S2] * E3[0];
+            for (int c = 1; c <= t3; c++) z = fma(D[a * S1 + b * S2 + c], E3[c], z);
+            y = fma(z, E2[b], y);
+          }
+          x = fma(y, E1[a], x);
+        }
+        V[d][0] = x;
+        continue;
+      }
       // V(x1,x2,x3), compact strides, one axis at a time in place
       double* v = V[d];
       const int w2 = t3 + 1, w1 = (t2 + 1) * w2;
@@ -220,6 +240,11 @@ G3_HD void three_body(const double* r1, const double* r2, const double* rp, cons
     }
   }
   const double kPi = 3.14159265358979e+00;   // the MD kernels' truncated pi
+  if constexpr (MODE == kOverlap) {
+    *x1 = 0.0;
+    *x2 = (kPi * kPi * kPi * kPi) * sqrt(kPi) * (rdet * rsd) * (V[0][0] * V[1][0] * V[2][0]);
+    return;
+  }
   double acc = 0.0;
   // the operators: 1/r_12, then (FULL) 1/r_1p, 1/r_2p and the nuclear
   // attraction of 1, 2 and p
@@ -330,6 +355,160 @@ G3_HD double two_body_overlap(const double* r1, const double* rp, double g) {
     res *= acc;
   }
   return (kPi * kPi * kPi) * (rd * rs) * exp(-ex) * res;
+}
+
+// (r | s): Coulomb integral of two pair densities (gfvee, vee.f:3-78; gam_ep).
+template <int NT>
+G3_HD double pair_coulomb(const double* r, const double* s) {
+  const double kPi = 3.14159265358979323846;
+  const double p = r[kRP], q = s[kRP], rs = rsqrt64(p + q), pq = p * q, alpha = pq * (rs * rs);
+  double W[3][NT + 1], R[3], R2 = 0.0;
+  int n[3];
+  for (int d = 0; d < 3; d++) {
+    const int t = (int)r[kRT + d], u = (int)s[kRT + d];
+    const double* E = r + kRE + 5 * d;
+    const double* F = s + kRE + 5 * d;
+    n[d] = t + u;
+    for (int k = 0; k <= n[d]; k++) W[d][k] = 0.0;
+    for (int b = 0; b <= u; b++) {
+      const double f = (b & 1) ? -F[b] : F[b];
+      for (int a = 0; a <= t; a++) W[d][a + b] = fma(E[a], f, W[d][a + b]);
+    }
+    R[d] = r[kRX + d] - s[kRX + d];
+    R2 = fma(R[d], R[d], R2);
+  }
+  return (2.0 * kPi * kPi * sqrt(kPi)) * rs / pq * coulomb_sum<NT>(n, W, R, alpha * R2, alpha);
+}
+
+// The multiplicative terms of xcalc_GAM1_MD's integrand (gam_1_OMP.f:398-836)
+// for an electron and a proton pair density coupled by exp(-g r^2):
+// *e = -Z/r_eC + Z/r_pC - 1/r_ep, *ov = the overlap.
+template <int LE, int LN>
+G3_HD void two_body(const double* r1, const double* rp, double g, int nat, const double* cat,
+                    const double* zan, double* e, double* ov) {
+  constexpr int M1 = 2 * LE, M3 = 2 * LN, NT = M1 + M3;
+  const double kPi = 3.14159265358979e+00;
+  const double P1 = r1[kRP], P3 = rp[kRP], a11 = P3 + g, a33 = P1 + g;
+  const double det = fma(P1, P3, g * (P1 + P3));
+  const double rs = rsqrt64(det), rd = rs * rs, K = P1 * P3 * g * rd;
+  double V[3][(M1 + 1) * (M3 + 1)], u[3], ex = 0.0;
+  int T1[3], T3[3], n[3];
+  NX_LOOP
+  for (int d = 0; d < 3; d++) {
+    const int t1 = (int)r1[kRT + d], t3 = (int)rp[kRT + d];
+    T1[d] = t1;
+    T3[d] = t3;
+    n[d] = t1 + t3;
+    u[d] = r1[kRX + d] - rp[kRX + d];
+    ex = fma(K * u[d], u[d], ex);
+    double gd[NT + 1];
+    gd[0] = 1.0;
+    const double h = -2.0 * K;
+    for (int k = 1; k <= n[d]; k++)
+      gd[k] = h * (k > 1 ? fma(u[d], gd[k - 1], (double)(k - 1) * gd[k - 2]) : u[d] * gd[0]);
+    const int w = t3 + 1;
+    for (int i = 0; i <= t1; i++) {
+      for (int c = 0; c <= t3; c++) V[d][i * w + c] = (c & 1) ? -gd[i + c] : gd[i + c];
+      fold_line(V[d] + i * w, 1, t3, rp + kRE + 5 * d);
+    }
+    for (int c = 0; c <= t3; c++) fold_line(V[d] + c, w, t1, r1 + kRE + 5 * d);
+  }
+  const double base = exp(-ex);
+  double acc = 0.0;
+  NX_LOOP
+  for (int op = 0; op < 3; op++) {   // 1/r_ep, 1/r_eC, 1/r_pC
+    const double v = op == 0 ? P1 + P3 : (op == 1 ? a11 : a33);
+    const double b1 = (op == 0 ? P3 * P1 : (op == 1 ? a11 * P1 : g * P1)) * rd;
+    const double b3 = op == 0 ? -b1 : (op == 1 ? g * P3 : a33 * P3) * rd;
+    const double rv = rsqrt64(v), alpha = det * rv * rv;
+    double W[3][NT + 1];
+    NX_LOOP
+    for (int d = 0; d < 3; d++) {
+      for (int k = 0; k <= n[d]; k++) W[d][k] = 0.0;
+      const double* vv = V[d];
+      double p1 = 1.0;
+      for (int i = 0; i <= T1[d]; i++) {
+        double p = p1;
+        for (int c = 0; c <= T3[d]; c++) {
+          W[d][i + c] = fma(p, *vv++, W[d][i + c]);
+          p *= b3;
+        }
+        p1 *= b1;
+      }
+    }
+    const int nc = op == 0 ? 1 : nat;
+    double sum = 0.0;
+    NX_LOOP
+    for (int c = 0; c < nc; c++) {
+      double R[3], R2 = 0.0;
+      for (int d = 0; d < 3; d++) {
+        R[d] = b1 * u[d];   // the mean of e or p lies at c_p + b1 u
+        if (op > 0) R[d] = (R[d] + rp[kRX + d]) - cat[3 * c + d];
+        R2 = fma(R[d], R[d], R2);
+      }
+      const double x = coulomb_sum<NT>(n, W, R, alpha * R2, alpha);
+      sum = op == 0 ? x : fma(zan[c], x, sum);
+    }
+    acc = op == 2 ? fma(sum, rv, acc) : fma(-sum, rv, acc);
+  }
+  *e = 2.0 * kPi * kPi * sqrt(kPi) * rd * base * acc;
+  *ov = (kPi * kPi * kPi) * (rd * rs) * base * (V[0][0] * V[1][0] * V[2][0]);
+}
+
+// pgike1 (g2.f:545-651): kinetic energy of particle 1 with geminal exponents
+// gA (bra) and gB (ket), by the formulas of md::pgike1 operation by operation
+// (the kinetic terms of a nearly dependent basis cancel to the last digits of
+// the reference's logged energies, so its rounding is kept), with the Hermite
+// vectors, the Gaussian derivatives and the exponentials shared by the ten
+// 1-D overlaps of a direction instead of rebuilt for each.
+G3_HD double pair_kinetic(const md::Prim& A1, const md::Prim& A2, const md::Prim& B1,
+                          const md::Prim& B2, double gA, double gB, double xmass) {
+  constexpr int N = 2 * md::LP + 3;   // Hermite entries with the ket raised by two
+  const double g = gA + gB, PI = 3.141592650;   // pgi_hint0_1D's pi (g2.f:200-234)
+  double S[3], T[3];
+  NX_LOOP
+  for (int d = 0; d < 3; d++) {
+    const double a1 = A1.a, a2 = A2.a, b1 = B1.a, b2 = B2.a;
+    const double X1 = A1.c[d], X2 = A2.c[d], Y1 = B1.c[d], Y2 = B2.c[d];
+    const int I1 = A1.l[d], I2 = A2.l[d], L1 = B1.l[d], L2 = B2.l[d];
+    const double p1 = a1 + b1, q1 = (a1 * b1) / (a1 + b1), Q1 = X1 - Y1;
+    const double p2 = a2 + b2, q2 = (a2 * b2) / (a2 + b2), Q2 = X2 - Y2;
+    const double Pm1 = (a1 * X1 + b1 * Y1) / (a1 + b1);
+    const double Pm2 = (a2 * X2 + b2 * Y2) / (a2 + b2);
+    const double K1 = exp(-q1 * Q1 * Q1), K2 = exp(-q2 * Q2 * Q2);
+    const double s = (p1 * p2) + (p1 * g) + (p2 * g);
+    const double q = (p1 * p2 * g) / s, pre = sqrt(PI * PI / s);
+    double E1[5][2 * md::TMX + 1], E2[3][2 * md::TMX + 1], gd[2 * N + 1];
+    md::gauss_derivs(I1 + L1 + I2 + L2 + 4, q, Pm1 - Pm2, gd);
+    NX_LOOP
+    for (int k = 0; k < 5; k++)   // ket L1 - 2 .. L1 + 2
+      if (L1 + k - 2 >= 0) md::hermite_e(I1, L1 + k - 2, K1, a1, b1, p1, q1, Q1, E1[k]);
+    NX_LOOP
+    for (int k = 0; k < 3; k++) md::hermite_e(I2, L2 + k, K2, a2, b2, p2, q2, Q2, E2[k]);
+    auto ov = [&](int k, int m) {
+      double acc = 0.0;
+      for (int t1 = 0; t1 <= I1 + L1 + k - 2; t1++)
+        for (int t2 = 0; t2 <= I2 + L2 + m; t2++)
+          acc += E1[k][t1] * E2[m][t2] * (((t2 & 1) ? -1.0 : 1.0) * pre * gd[t1 + t2]);
+      return acc;
+    };
+    const double X12 = Y1 - Y2;
+    const double o00 = ov(2, 0), o01 = ov(2, 1), o02 = ov(2, 2), o10 = ov(3, 0), o11 = ov(3, 1),
+                 o20 = ov(4, 0);
+    const double om0 = L1 >= 1 ? ov(1, 0) : 0.0, om1 = L1 >= 1 ? ov(1, 1) : 0.0;
+    const double omm = L1 >= 2 ? ov(0, 0) : 0.0;
+    const double d1 = (double)(L1 * (L1 - 1)), d2 = -2.0 * b1 * (double)((2 * L1) + 1);
+    const double d3 = 4.0 * b1 * b1, c1 = (double)L1, c2 = -2.0 * b1;
+    const double W1 = (d1 * omm) + (d2 * o00) + (d3 * o20);
+    const double z1 = L1 >= 1 ? o00 - om1 + (X12 * om0) : 0.0;
+    const double z2 = o20 - o11 + (X12 * o10);
+    const double W2 = -2.0 * gB * ((c1 * z1) + (c2 * z2));
+    const double t2 = o20 + o02 + (X12 * X12 * o00) - (2.0 * o11) - (2.0 * X12 * o01) + (2.0 * X12 * o10);
+    const double W3 = (-2.0 * gB * o00) + (4.0 * gB * gB * t2);
+    S[d] = o00;
+    T[d] = -(W1 + (2.0 * W2) + W3) * 0.50 / xmass;
+  }
+  return (T[0] * S[1] * S[2]) + (S[0] * T[1] * S[2]) + (S[0] * S[1] * T[2]);
 }
 
 // Composite bra of pair densities A (kept) and B (integrated out with the

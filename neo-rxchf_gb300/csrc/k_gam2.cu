@@ -54,16 +54,6 @@ using g3::Bra;
 
 constexpr int kWarps = 2;   // independent warps of a CTA
 
-__device__ __forceinline__ md::Prim to_md(const DevPrim& d) {
-  md::Prim p;
-  p.a = d.a;
-  for (int k = 0; k < 3; k++) {
-    p.c[k] = d.c[k];
-    p.l[k] = d.l[k];
-  }
-  return p;
-}
-
 __host__ __device__ __forceinline__ void unpair(int P, int& i, int& j) {
   int a = (int)((sqrtf(8.0f * (float)P + 1.0f) - 1.0f) * 0.5f);
   while (a * (a + 1) / 2 > P) a--;
@@ -72,42 +62,25 @@ __host__ __device__ __forceinline__ void unpair(int P, int& i, int& j) {
   j = P - a * (a + 1) / 2;
 }
 
-struct Gam2View {   // the pair tables of DevSystem (stage_system) and this build's arrays
+struct Gam2View {   // the pair tables of DevSystem (stage_system)
   const double *erec, *prec;      // pair records
   const double *egrad, *pgrad;    // gradient records
   const int *kofs, *kperm;        // primitive pairs of a contracted pair; class order
   int nket, nPe;
 };
 
-__host__ __device__ __forceinline__ Gam2View view(const DevSystem& S, const double* grad) {
+__host__ __device__ __forceinline__ Gam2View view(const DevSystem& S) {
   Gam2View v;
   v.nPe = S.nebf * (S.nebf + 1) / 2;
   v.nket = S.g3_nket;
   v.erec = S.g3rec;
   v.prec = S.g3rec + (size_t)kRLen * v.nket;
-  v.egrad = grad;
-  v.pgrad = grad + (size_t)kGLen * v.nket;
+  v.egrad = S.g3grad;
+  v.pgrad = S.g3grad + (size_t)kGLen * v.nket;
   v.kofs = S.g3i + 2 * v.nket;
   // after kofs[nPe + 1]: tile_k and tile_P [ntile + 1 each], then the permutation
   v.kperm = v.kofs + v.nPe + 1 + 2 * (S.g3_ntile_all + 1);
   return v;
-}
-
-__global__ void gam2_gradient_kernel(DevSystem S, double* __restrict__ grad) {
-  const int nket = S.g3_nket, n = nket + S.npbf * (S.npbf + 1) / 2;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    const DevPrim *a, *b;
-    if (t < nket) {
-      a = S.eprim + S.g3i[2 * t];
-      b = S.eprim + S.g3i[2 * t + 1];
-    } else {
-      int ip, jp;
-      unpair(t - nket, ip, jp);
-      a = S.pprim + ip;
-      b = S.pprim + jp;
-    }
-    fill_gradient_record(to_md(*a), to_md(*b), grad + (size_t)kGLen * t);
-  }
 }
 
 __device__ __forceinline__ double warp_add(double v) {
@@ -134,9 +107,9 @@ __device__ __forceinline__ void pair_term(const DevSystem& S, int q, double& g, 
 // the two-particle overlap; then H[Pe], the contracted core Hamiltonian.
 template <int LE>
 __global__ void __launch_bounds__(32 * kWarps)
-gam2_factor_kernel(DevSystem S, const double* __restrict__ grad, int nPp,
+gam2_factor_kernel(DevSystem S, int nPp,
                    double* __restrict__ W, double* __restrict__ H) {
-  const Gam2View v = view(S, grad);
+  const Gam2View v = view(S);
   const int lane = threadIdx.x & 31;
   const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nw = (long long)nPp * v.nPe;
@@ -191,11 +164,11 @@ gam2_factor_kernel(DevSystem S, const double* __restrict__ grad, int nPp,
 // exponents only (RXCHF-ne).  grid (nPp * nPe, ket groups, splits) of warps.
 template <int LE, int LN, bool PAIRS>
 __global__ void __launch_bounds__(32 * kWarps)
-gam2_pair_kernel(DevSystem S, const double* __restrict__ grad, int Pp0, long long nunit,
+gam2_pair_kernel(DevSystem S, int Pp0, long long nunit,
                  double* __restrict__ Y) {
   constexpr int NW = 2 * LE + 2 * LN, NK = 2 * LE;
   __shared__ Bra<double, NW> s_bra[kWarps][32];
-  const Gam2View v = view(S, grad);
+  const Gam2View v = view(S);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const long long u = (long long)blockIdx.x * kWarps + wid;
   if (u >= nunit) return;
@@ -241,12 +214,13 @@ gam2_pair_kernel(DevSystem S, const double* __restrict__ grad, int Pp0, long lon
 
 // R1 / R2[split][Pp - Pp0][Pa][ket] for the kets of pairs P <= Pa.  Lanes take
 // those kets in class order (a queue filled by ballots over the permutation).
-template <int LE, int LN, bool FULL>
+template <int LE, int LN, int MODE>
 __global__ void __launch_bounds__(32 * kWarps)
-gam2_triple_kernel(DevSystem S, const double* __restrict__ grad, int Pp0, long long nunit,
+gam2_triple_kernel(DevSystem S, int Pp0, long long nunit,
                    double* __restrict__ R1, double* __restrict__ R2) {
+  constexpr bool FULL = MODE == kAll;
   __shared__ int s_q[kWarps][64];
-  const Gam2View v = view(S, grad);
+  const Gam2View v = view(S);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   // the last pairs have the most kets: take them first
   const long long u = nunit - 1 - ((long long)blockIdx.x * kWarps + wid);
@@ -285,7 +259,7 @@ gam2_triple_kernel(DevSystem S, const double* __restrict__ grad, int Pp0, long l
         const double* r1 = v.erec + (size_t)kRLen * (ka + ua);
         const double* e1 = v.egrad + (size_t)kGLen * (ka + ua);
         double x1, x2;
-        three_body<LE, LN, FULL>(r1, r2, rp, e1, e2, ep, S.ggem[k], S.ggem[l], S.nat, S.cat,
+        three_body<LE, LN, MODE>(r1, r2, rp, e1, e2, ep, S.ggem[k], S.ggem[l], S.nat, S.cat,
                                  S.zan, rpm, &x1, &x2);
         const double w = S.bgem[k] * S.bgem[l] * r1[kRC];
         if (FULL) s1 = fma(w, x1, s1);
@@ -372,7 +346,7 @@ constexpr size_t kChunkDoubles = (size_t)1 << 25;   // scratch aim of a chunk: 2
 
 struct Plan {
   int nPe, nPp, nket, chunk, spY, spR;
-  size_t grad, fac, per;   // gradient records; W and H; doubles per proton pair of a chunk
+  size_t fac, per;   // W and H; doubles per proton pair of a chunk
 };
 
 // max_prim: primitive pairs of the largest contracted pair (bounds the splits)
@@ -389,20 +363,18 @@ Plan make_plan(int ne, int np, int nket, int max_prim, int ng, bool rx, int nPp_
   const long long nt = ng + ng * (ng + 1) / 2;
   p.spY = split((kWantWarps + units * groups - 1) / (units * groups), (2 * max_prim * nt + 31) / 32);
   p.spR = split((kWantWarps + units - 1) / units, (long long)max_prim * ng * ng);
-  p.grad = (size_t)kGLen * ((size_t)nket + p.nPp);
   p.fac = (size_t)p.nPp * p.nPe + p.nPe;
   const size_t row = (size_t)p.nPe * nket;
   p.per = row * ((size_t)p.spY + (rx ? 1 : 2) * (size_t)p.spR) + 3 * (size_t)p.nPe * p.nPe;
   size_t c = kChunkDoubles / p.per;
-  p.chunk = (int)std::max<size_t>(1, std::min<size_t>(c, (size_t)nPp_want));
+  p.chunk = (int)std::max<size_t>(1, std::min<size_t>(std::min<size_t>(c, (size_t)nPp_want), 32768));
   return p;
 }
 
 template <int LE, int LN, bool RX>
 cudaError_t build_t(const DevSystem& S, const Plan& p, double* scratch, int Pp0, int nPp, bool one,
                     double* x1, double* x2, cudaStream_t s) {
-  double* grad = scratch;
-  double* W = grad + p.grad;
+  double* W = scratch;
   double* H = W + (size_t)p.nPp * p.nPe;
   double* buf = W + p.fac;
   const size_t row = (size_t)p.nPe * p.nket;
@@ -417,9 +389,9 @@ cudaError_t build_t(const DevSystem& S, const Plan& p, double* scratch, int Pp0,
     double* R1c = Yc + (size_t)units * p.nPe;
     double* R2c = R1c + (size_t)units * p.nPe;
     const unsigned nb = (unsigned)((units + kWarps - 1) / kWarps);
-    gam2_triple_kernel<LE, LN, !RX><<<dim3(nb, p.spR), 32 * kWarps, 0, s>>>(S, grad, c0, units, R1, R2);
+    gam2_triple_kernel<LE, LN, RX ? kCoulomb12 : kAll><<<dim3(nb, p.spR), 32 * kWarps, 0, s>>>(S, c0, units, R1, R2);
     gam2_pair_kernel<LE, LN, RX><<<dim3(nb, (p.nket + 31) / 32, p.spY), 32 * kWarps, 0, s>>>(
-        S, grad, c0, units, Y);
+        S, c0, units, Y);
     const unsigned cb = (unsigned)std::min<long long>((units * p.nPe + 127) / 128, 152 * 16);
     gam2_contract_kernel<<<cb, 128, 0, s>>>(S, units, p.spY, 0, Y, Yc);
     if (!RX) gam2_contract_kernel<<<cb, 128, 0, s>>>(S, units, p.spR, 1, R1, R1c);
@@ -453,31 +425,104 @@ Plan plan_of(const DevSystem& S, int rx, int nPp_want) {
   return make_plan(S.nebf, S.npbf, S.g3_nket, S.g3_max_prim, S.ngtg, rx != 0, nPp_want);
 }
 
+// W3 on the packed order from the canonical overlaps (grid y: proton pairs of a chunk)
+__global__ void overlap_expand_kernel(int ne, int np, int Pp0, const double* __restrict__ R2,
+                                      double* __restrict__ W3) {
+  const int n2 = ne * ne, nPe = ne * (ne + 1) / 2;
+  const long long n4 = (long long)n2 * n2;
+  int ip, jp;
+  unpair(Pp0 + blockIdx.y, ip, jp);
+  const double* r = R2 + (long long)blockIdx.y * nPe * nPe;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n4;
+       t += (long long)gridDim.x * blockDim.x) {
+    const int e1 = (int)(t / n2), e2 = (int)(t - (long long)e1 * n2);
+    const int P1 = g3::pair_index(e1 / ne, e1 % ne), P2 = g3::pair_index(e2 / ne, e2 % ne);
+    const double v = P1 > P2 ? r[(long long)P1 * nPe + P2] : r[(long long)P2 * nPe + P1];
+    W3[((long long)ip * np + jp) * n4 + t] = v;
+    W3[((long long)jp * np + ip) * n4 + t] = v;
+  }
+}
+
+// W1 = W / 2 on [ip][jp][i][j] and the core Hamiltonian on [i][j]
+__global__ void factor_expand_kernel(int ne, int np, const double* __restrict__ W,
+                                     const double* __restrict__ H, double* __restrict__ W1,
+                                     double* __restrict__ hc) {
+  const int n2 = ne * ne, nPe = ne * (ne + 1) / 2;
+  const long long total = (long long)np * np * n2;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
+       t += (long long)gridDim.x * blockDim.x) {
+    const int e = (int)(t % n2), pp = (int)(t / n2);
+    const int P = g3::pair_index(e / ne, e % ne);
+    W1[t] = 0.5 * W[(long long)g3::pair_index(pp / np, pp % np) * nPe + P];
+    if (hc && pp == 0) hc[e] = H[P];
+  }
+}
+
+template <int LE, int LN>
+void overlap_t(const DevSystem& S, const Plan& p, int c0, long long units, double* R2, cudaStream_t s) {
+  gam2_triple_kernel<LE, LN, kOverlap><<<dim3((unsigned)((units + kWarps - 1) / kWarps), p.spR),
+                                         32 * kWarps, 0, s>>>(S, c0, units, R2, R2);
+}
+
 }  // namespace
+
+cudaError_t launch_gam3_factors(const DevSystem& S, double* scratch, const double* w3_in,
+                                double* W1, double* W3, double* hc, cudaStream_t s) {
+  const int ne = S.nebf, np = S.npbf;
+  const long long n4 = (long long)ne * ne * ne * ne;
+  cudaError_t e = launch_gam2_prepare(S, scratch, s);
+  if (e != cudaSuccess) return e;
+  const Plan p = plan_of(S, 1, np * (np + 1) / 2);
+  double* W = scratch;
+  const long long n1 = (long long)np * np * ne * ne;
+  factor_expand_kernel<<<(unsigned)std::min<long long>((n1 + 255) / 256, 152 * 16), 256, 0, s>>>(
+      ne, np, W, W + (size_t)p.nPp * p.nPe, W1, hc);
+  if (w3_in)
+    return cudaMemcpyAsync(W3, w3_in, sizeof(double) * n4 * np * np, cudaMemcpyDeviceToDevice, s);
+  double* buf = W + p.fac;
+  for (int c0 = 0; c0 < p.nPp; c0 += p.chunk) {
+    const int nc = std::min(p.chunk, p.nPp - c0);
+    const long long units = (long long)nc * p.nPe;
+    double* R2 = buf;
+    double* R2c = R2 + (size_t)p.nPe * p.nket * p.spR * nc;
+    switch (S.lmax_e * 3 + (S.lmax_p == 0 ? 0 : 2)) {
+      case 0: overlap_t<0, 0>(S, p, c0, units, R2, s); break;
+      case 2: overlap_t<0, 2>(S, p, c0, units, R2, s); break;
+      case 3: overlap_t<1, 0>(S, p, c0, units, R2, s); break;
+      case 5: overlap_t<1, 2>(S, p, c0, units, R2, s); break;
+      case 6: overlap_t<2, 0>(S, p, c0, units, R2, s); break;
+      case 8: overlap_t<2, 2>(S, p, c0, units, R2, s); break;
+      default: return cudaErrorInvalidValue;
+    }
+    const unsigned cb = (unsigned)std::min<long long>((units * p.nPe + 127) / 128, 152 * 16);
+    gam2_contract_kernel<<<cb, 128, 0, s>>>(S, units, p.spR, 1, R2, R2c);
+    overlap_expand_kernel<<<dim3((unsigned)std::min<long long>((n4 + 255) / 256, 1024), nc), 256, 0, s>>>(
+        ne, np, c0, R2c, W3);
+  }
+  return cudaGetLastError();
+}
 
 size_t gam2_scratch_doubles(const DevSystem& S, int rx, int nPp_want) {
   const Plan p = plan_of(S, rx, nPp_want);
-  return p.grad + p.fac + p.per * (size_t)p.chunk;
+  return p.fac + p.per * (size_t)p.chunk;
 }
 
 size_t gam2_scratch_bound(int ne, int np, int nket, int max_prim, int ng) {
   const Plan p = make_plan(ne, np, nket, max_prim, ng, false, np * (np + 1) / 2);
-  return p.grad + p.fac + p.per * (size_t)p.chunk;
+  return p.fac + p.per * (size_t)p.chunk;
 }
 
 cudaError_t launch_gam2_prepare(const DevSystem& S, double* scratch, cudaStream_t s) {
-  if (S.nebf < 1 || S.npbf < 1 || !S.g3i || !S.g3rec) return cudaErrorInvalidValue;
+  if (S.nebf < 1 || S.npbf < 1 || !S.g3i || !S.g3rec || !S.g3grad) return cudaErrorInvalidValue;
   const int nPe = S.nebf * (S.nebf + 1) / 2, nPp = S.npbf * (S.npbf + 1) / 2;
-  const int n = S.g3_nket + nPp;
-  gam2_gradient_kernel<<<std::min((n + 63) / 64, 152 * 8), 64, 0, s>>>(S, scratch);
-  double* W = scratch + (size_t)kGLen * n;
+  double* W = scratch;
   double* H = W + (size_t)nPp * nPe;
   const long long warps = (long long)nPp * nPe + nPe;
   const unsigned nb = (unsigned)((warps + kWarps - 1) / kWarps);
   switch (S.lmax_e) {
-    case 0: gam2_factor_kernel<0><<<nb, 32 * kWarps, 0, s>>>(S, scratch, nPp, W, H); break;
-    case 1: gam2_factor_kernel<1><<<nb, 32 * kWarps, 0, s>>>(S, scratch, nPp, W, H); break;
-    default: gam2_factor_kernel<2><<<nb, 32 * kWarps, 0, s>>>(S, scratch, nPp, W, H); break;
+    case 0: gam2_factor_kernel<0><<<nb, 32 * kWarps, 0, s>>>(S, nPp, W, H); break;
+    case 1: gam2_factor_kernel<1><<<nb, 32 * kWarps, 0, s>>>(S, nPp, W, H); break;
+    default: gam2_factor_kernel<2><<<nb, 32 * kWarps, 0, s>>>(S, nPp, W, H); break;
   }
   return cudaGetLastError();
 }

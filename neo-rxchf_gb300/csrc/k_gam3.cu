@@ -45,7 +45,8 @@
 // fold one particle at a time, and warps share (32 kets, a quarter of the
 // bras) units so that none idles in a last round of few kets.  Measured (one
 // GB300, neoxc_gam3_ic1): nebf = 6 s/p of 3 primitives, npbf = 4 s/p/d,
-// NG = 3: 516 -> 279 ms; FP32 tables at nebf = 4, npbf = 2: 6.5 -> 3.8 ms.
+// NG = 3: 516 -> 279 ms, 253 ms with the overlap-only W3 of k_gam2.cu; FP32
+// tables at nebf = 4, npbf = 2: 6.5 -> 3.8 -> 2.1 ms.
 //
 // The prefactors, exponents and centres follow G4_MD_xgVepg / G4_MD_xgVeeg
 // (truncated pi, the reference's underflow on every G4Vep value); only the
@@ -71,7 +72,7 @@
 #include <type_traits>
 #include <vector>
 
-#include "g3_fatbra.cuh"
+#include "g2_threebody.cuh"
 #include "neoxc_internal.h"
 
 namespace neoxc {
@@ -98,29 +99,25 @@ __device__ __forceinline__ void unpair(int P, int& i, int& j) {
 }
 
 // Records of every canonical electronic primitive pair (ket order) and every
-// canonical nuclear pair.
-__global__ void g3_records_kernel(DevSystem S, double* __restrict__ erec,
-                                  double* __restrict__ prec) {
-  const int nket = S.g3_nket;
-  const int nPp = S.npbf * (S.npbf + 1) / 2;
-  const int* ket_ab = S.g3i;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nket + nPp;
-       t += gridDim.x * blockDim.x) {
+// canonical nuclear pair, and their gradient records; a thread per pair and
+// kind (the two are independent chains).
+__global__ void g3_records_kernel(DevSystem S, double* __restrict__ rec, double* __restrict__ grad) {
+  const int nket = S.g3_nket, n = nket + S.npbf * (S.npbf + 1) / 2;
+  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < 2 * n; u += gridDim.x * blockDim.x) {
+    const int t = u < n ? u : u - n;
     const DevPrim* pa;
     const DevPrim* pb;
-    double* out;
     if (t < nket) {
-      pa = S.eprim + ket_ab[2 * t];
-      pb = S.eprim + ket_ab[2 * t + 1];
-      out = erec + (size_t)kRLen * t;
+      pa = S.eprim + S.g3i[2 * t];
+      pb = S.eprim + S.g3i[2 * t + 1];
     } else {
       int ip, jp;
       unpair(t - nket, ip, jp);
       pa = S.pprim + ip;
       pb = S.pprim + jp;
-      out = prec + (size_t)kRLen * (t - nket);
     }
-    fill_pair_record(to_md(*pa), to_md(*pb), pa->coef, pb->coef, out);
+    if (u < n) fill_pair_record(to_md(*pa), to_md(*pb), pa->coef, pb->coef, rec + (size_t)kRLen * t);
+    else g2::fill_gradient_record(to_md(*pa), to_md(*pb), grad + (size_t)g2::kGLen * t);
   }
 }
 
@@ -514,11 +511,13 @@ size_t g3_record_doubles(int nket, int np) {
   return (size_t)kRLen * ((size_t)nket + (size_t)np * (np + 1) / 2);
 }
 
-cudaError_t launch_g3_records(const DevSystem& sys, double* rec, cudaStream_t s) {
-  const int n = sys.g3_nket + sys.npbf * (sys.npbf + 1) / 2;
-  int blocks = (n + 127) / 128;
-  if (blocks > 152 * 8) blocks = 152 * 8;
-  g3_records_kernel<<<blocks, 128, 0, s>>>(sys, rec, rec + (size_t)kRLen * sys.g3_nket);
+size_t g3_gradient_doubles(int nket, int np) {
+  return (size_t)g2::kGLen * ((size_t)nket + (size_t)np * (np + 1) / 2);
+}
+
+cudaError_t launch_g3_records(const DevSystem& sys, double* rec, double* grad, cudaStream_t s) {
+  const int n = 2 * (sys.g3_nket + sys.npbf * (sys.npbf + 1) / 2);
+  g3_records_kernel<<<std::min((n + 63) / 64, 152 * 16), 64, 0, s>>>(sys, rec, grad);
   return cudaGetLastError();
 }
 

@@ -1,6 +1,6 @@
 // k_scf.cu -- device side of the XCHF RHF SCF (xchf1_independent/xcscf.f,
-// xchf1_fock.f) for sm_103a: the one- and two-particle integrals besides
-// gam_2/3/4, the Fock/energy assembly, ROOTHAN with a block-parallel Jacobi
+// xchf1_fock.f) for sm_103a (its integral tables: k_pair.cu, k_gam2.cu,
+// k_gam3.cu): the one-body Fock/energy assembly, ROOTHAN with a block-parallel Jacobi
 // eigensolver, and the density-change check.  Every kernel takes device
 // pointers; energies and convergence scalars live in a device array so an
 // SCF iteration needs no host round trip except the final 3-scalar read.
@@ -13,204 +13,10 @@
 // reference's Fortran arrays; the core matrices keep pack_2D order
 // ([i][j] = GAM_ecore(pack_2D(n,j,i))) and GAM_ep / GAM_1 / GAM_1s keep
 // pack_4D(nebf,nebf,npbf, je,ie,jp,ip) order, i.e. C-order [ip][jp][ie][je].
-#include <type_traits>
-
-#include "md_math.cuh"
-#include "md_math32.cuh"
 #include "neoxc_internal.h"
 
 namespace neoxc {
 namespace {
-
-using md::Prim;
-
-__device__ __forceinline__ Prim to_prim(const DevPrim& p) {
-  Prim r;
-  r.a = p.a;
-  for (int d = 0; d < 3; d++) {
-    r.c[d] = p.c[d];
-    r.l[d] = p.l[d];
-  }
-  return r;
-}
-
-__device__ __forceinline__ double gfovlap(const Prim& A, const Prim& B) {
-  double s = 1.0;
-  for (int d = 0; d < 3; d++) s *= md::ovl1d(A.l[d], A.a, A.c[d], B.l[d], B.a, B.c[d]);
-  return s;
-}
-
-// gam_epcore.f:200-270 xcalc_GAM_epcore
-__device__ __noinline__ double xcalc_epcore(const Prim& A, const Prim& B,
-                                            const DevSystem& S, double xmass,
-                                            double coul_sign) {
-  const double ke = md::gfke(A, B, xmass);
-  double v = 0.0;
-  for (int k = 0; k < S.nat; k++) {
-    const double C[3] = {S.cat[3 * k], S.cat[3 * k + 1], S.cat[3 * k + 2]};
-    v = v + coul_sign * S.zan[k] * md::gfvec(A, B, C);
-  }
-  return ke + v;
-}
-
-// ---- overlaps and core Hamiltonians (pure_ovlap.f, gam_epcore.f) ----------
-// t < ne^2: electronic pair (i,j); then np^2 nuclear pairs.  Sums over the
-// primitive pairs in the reference's order (bra primitive outer).
-__global__ void onebody_kernel(DevSystem S, double* __restrict__ Se,
-                               double* __restrict__ Sp, double* __restrict__ Hce,
-                               double* __restrict__ Hcp) {
-  const int ne = S.nebf, np = S.npbf;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < ne * ne) {
-    const int i = t / ne, j = t - i * ne;
-    double so = 0.0, h = 0.0;
-    for (int a = S.kpestr[i]; a <= S.kpeend[i]; a++)
-      for (int b = S.kpestr[j]; b <= S.kpeend[j]; b++) {
-        const Prim A = to_prim(S.eprim[a]), B = to_prim(S.eprim[b]);
-        const double c = S.eprim[a].coef, d = S.eprim[b].coef;
-        so = so + gfovlap(A, B) * c * d;
-        h = h + xcalc_epcore(A, B, S, 1.0, -1.0) * c * d;
-      }
-    Se[i * ne + j] = so;   // pack_2D(ne, j, i) order; symmetric
-    Hce[i * ne + j] = h;
-  } else if (t < ne * ne + np * np) {
-    const int k = t - ne * ne, p = k / np, q = k - p * np;
-    const Prim A = to_prim(S.pprim[p]), B = to_prim(S.pprim[q]);
-    const double c = S.pprim[p].coef, d = S.pprim[q].coef;
-    Sp[p * np + q] = gfovlap(A, B) * c * d;
-    Hcp[p * np + q] = xcalc_epcore(A, B, S, S.pmass, 1.0) * c * d;
-  }
-}
-
-// ---- GAM_ep (gam_ep.f:2-219): -(e p | e' p'), C-order [ip][jp][ie][je] ----
-__global__ void gam_ep_kernel(DevSystem S, double* __restrict__ Gep) {
-  const int ne = S.nebf, np = S.npbf;
-  const int total = np * np * ne * ne;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= total) return;
-  int r = t;
-  const int je = r % ne; r /= ne;
-  const int ie = r % ne; r /= ne;
-  const int jp = r % np; r /= np;
-  const int ip = r;
-  const Prim P1 = to_prim(S.pprim[ip]), P2 = to_prim(S.pprim[jp]);
-  const double cp = S.pprim[ip].coef, cq = S.pprim[jp].coef;
-  double acc = 0.0;
-  for (int a = S.kpestr[ie]; a <= S.kpeend[ie]; a++)
-    for (int b = S.kpestr[je]; b <= S.kpeend[je]; b++) {
-      const double v = -md::gfvee(to_prim(S.eprim[a]), P1, to_prim(S.eprim[b]), P2);
-      acc = acc + v * cp * cq * S.eprim[a].coef * S.eprim[b].coef;
-    }
-  Gep[t] = acc;
-}
-
-// ---- gam_1 (gam_1_OMP.f:398-836 xcalc_GAM1_MD) -----------------------------
-// A = (e, p), B = (e', p'); one geminal work item of the reference's
-// result (gi < ng: the single-geminal terms of k = gi; else the pair
-// (k, l)): ansE = TE + TP - VCE + VCP - VMX and ansS = 2 OGX + OGG are
-// linear in these items, so the lanes of a warp share them.  P is md::Prim
-// (FP64) or md32::Prim (FP32 integrals, mixed path); the integral calls
-// resolve by argument-dependent lookup and every geminal/atom sum is FP64.
-template <class P>
-__device__ __noinline__ void xcalc_gam1_item(const P* A, const P* B, const DevSystem& S,
-                                             int gi, double* ansE, double* ansS) {
-  using R = typename std::remove_cv<decltype(P::a)>::type;
-  const R zero = R(0.0), one = R(1.0), pmass = (R)S.pmass;
-  const int ng = S.ngtg;
-  if (gi < ng) {
-    const R GV = (R)S.ggem[gi];
-    const double BV = S.bgem[gi];
-    const double tegx = BV * (double)pgike1(A[0], A[1], B[0], B[1], GV, zero, one);
-    const double tpgx = BV * (double)pgike1(A[1], A[0], B[1], B[0], GV, zero, pmass);
-    double ve = 0.0, vp = 0.0;
-    for (int c = 0; c < S.nat; c++) {
-      const R C[3] = {(R)S.cat[3 * c], (R)S.cat[3 * c + 1], (R)S.cat[3 * c + 2]};
-      ve = (double)g2_xggvec(A[0], A[1], B[0], B[1], GV, zero, C) * S.zan[c] + ve;
-      vp = (double)g2_xggvec(A[1], A[0], B[1], B[0], GV, zero, C) * S.zan[c] + vp;
-    }
-    const double vm = (double)g2_xggvee(A[0], A[1], B[0], B[1], GV, zero);
-    const double texg = BV * (double)pgike1(A[0], A[1], B[0], B[1], zero, GV, one);
-    const double tpxg = BV * (double)pgike1(A[1], A[0], B[1], B[0], zero, GV, pmass);
-    // TE + TP - 2 VCEGX + 2 VCPGX - 2 VMGX (this k's share)
-    *ansE = (tegx + texg) + (tpgx + tpxg) - 2.0 * (BV * ve) + 2.0 * (BV * vp) -
-            2.0 * (BV * vm);
-    *ansS = 2.0 * (BV * (double)g2_xggs(A[0], A[1], B[0], B[1], GV, zero));
-    return;
-  }
-  const int k = (gi - ng) / ng, l = (gi - ng) - k * ng;
-  const R GV = (R)S.ggem[k], GW = (R)S.ggem[l];
-  const double BB = S.bgem[k] * S.bgem[l];
-  const double tegg = BB * (double)pgike1(A[0], A[1], B[0], B[1], GV, GW, one);
-  const double tpgg = BB * (double)pgike1(A[1], A[0], B[1], B[0], GV, GW, pmass);
-  double vee = 0.0, vpp = 0.0;
-  for (int c = 0; c < S.nat; c++) {
-    const R C[3] = {(R)S.cat[3 * c], (R)S.cat[3 * c + 1], (R)S.cat[3 * c + 2]};
-    vee = (double)g2_xggvec(A[0], A[1], B[0], B[1], GV, GW, C) * S.zan[c] + vee;
-    vpp = (double)g2_xggvec(A[1], A[0], B[1], B[0], GV, GW, C) * S.zan[c] + vpp;
-  }
-  const double vmm = (double)g2_xggvee(A[0], A[1], B[0], B[1], GV, GW);
-  *ansE = tegg + tpgg - BB * vee + BB * vpp - BB * vmm;
-  *ansS = BB * (double)g2_xggs(A[0], A[1], B[0], B[1], GV, GW);
-}
-
-__device__ __forceinline__ md32::Prim to_prim32(const DevPrim& p) {
-  md32::Prim r;
-  r.a = (float)p.a;
-  for (int d = 0; d < 3; d++) {
-    r.c[d] = (float)p.c[d];
-    r.l[d] = p.l[d];
-  }
-  return r;
-}
-
-// One warp per contracted (ip, jp, ie, je); lanes take primitive pairs and
-// the warp sums them in a fixed shuffle order (deterministic).
-template <bool F32>
-__global__ void gam1_kernel(DevSystem S, double* __restrict__ G1,
-                            double* __restrict__ G1s, int pairs_only) {
-  const int ne = S.nebf, np = S.npbf;
-  const int total = np * np * ne * ne;
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
-  const int lane = threadIdx.x & 31;
-  if (w >= total) return;
-  int r = w;
-  const int je = r % ne; r /= ne;
-  const int ie = r % ne; r /= ne;
-  const int jp = r % np; r /= np;
-  const int ip = r;
-  const int na = S.kpeend[ie] - S.kpestr[ie] + 1;
-  const int nb = S.kpeend[je] - S.kpestr[je] + 1;
-  const int nq = na * nb, ng = S.ngtg;
-  const int g0 = pairs_only ? ng : 0, nit = pairs_only ? ng * ng : ng + ng * ng;
-  double e = 0.0, sv = 0.0;
-  // lanes take (geminal item, primitive pair), the pair fastest
-  for (int q2 = lane; q2 < nq * nit; q2 += 32) {
-    const int gq = q2 / nq, k = q2 - gq * nq, gi = g0 + gq;
-    const int a = S.kpestr[ie] + k / nb, b = S.kpestr[je] + k % nb;
-    double aE, aS;
-    if constexpr (F32) {
-      md32::Prim A[2] = {to_prim32(S.eprim[a]), to_prim32(S.pprim[ip])};
-      md32::Prim B[2] = {to_prim32(S.eprim[b]), to_prim32(S.pprim[jp])};
-      xcalc_gam1_item(A, B, S, gi, &aE, &aS);
-    } else {
-      Prim A[2] = {to_prim(S.eprim[a]), to_prim(S.pprim[ip])};
-      Prim B[2] = {to_prim(S.eprim[b]), to_prim(S.pprim[jp])};
-      xcalc_gam1_item(A, B, S, gi, &aE, &aS);
-    }
-    const double cip = S.pprim[ip].coef, cjp = S.pprim[jp].coef;
-    const double cie = S.eprim[a].coef, cje = S.eprim[b].coef;
-    e = e + aE * cip * cjp * cie * cje;
-    sv = sv + aS * cip * cjp * cie * cje;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    e += __shfl_down_sync(0xffffffffu, e, o);
-    sv += __shfl_down_sync(0xffffffffu, sv, o);
-  }
-  if (lane == 0) {
-    G1[w] = e;
-    G1s[w] = sv;
-  }
-}
 
 // ---- one-body part of xchf1_fock (E_from_GAM_ecore/pcore/ep/ee/1, S_from_GAM_1s)
 // t < ne^2 : electronic (i,j);  ne^2 <= t < ne^2+np^2 : nuclear (p,q).
@@ -1064,28 +870,6 @@ __global__ void soscf_kernel(int n, int na, const double* __restrict__ F,
 }
 
 }  // namespace
-
-cudaError_t launch_scf_onebody(const DevSystem& S, double* Se, double* Sp,
-                               double* Hce, double* Hcp, cudaStream_t s) {
-  const int n = S.nebf * S.nebf + S.npbf * S.npbf;
-  onebody_kernel<<<(n + 127) / 128, 128, 0, s>>>(S, Se, Sp, Hce, Hcp);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_gam_ep(const DevSystem& S, double* Gep, cudaStream_t s) {
-  const int n = S.npbf * S.npbf * S.nebf * S.nebf;
-  gam_ep_kernel<<<(n + 127) / 128, 128, 0, s>>>(S, Gep);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_gam1(const DevSystem& S, double* G1, double* G1s,
-                        cudaStream_t s, int fp32, int pairs_only) {
-  const long long warps = (long long)S.npbf * S.npbf * S.nebf * S.nebf;
-  const long long blocks = (warps * 32 + 127) / 128;
-  if (fp32) gam1_kernel<true><<<(unsigned)blocks, 128, 0, s>>>(S, G1, G1s, pairs_only);
-  else gam1_kernel<false><<<(unsigned)blocks, 128, 0, s>>>(S, G1, G1s, pairs_only);
-  return cudaGetLastError();
-}
 
 size_t scf_fock1_part_doubles(int ne, int np) {
   return 6 * ((size_t)ne * ne + (size_t)np * np);

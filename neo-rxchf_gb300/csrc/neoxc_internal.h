@@ -41,6 +41,8 @@ struct DevSystem {
   int g3_nket, g3_ntile, g3_ntile_all, g3_max_prim;
   const int* g3i;
   const double* g3rec;
+  // gradient records (g2_threebody.cuh) in the same order
+  const double* g3grad;
 };
 
 // Largest per-Cartesian angular momentum supported by the MD kernels.
@@ -228,9 +230,14 @@ size_t gam3_aux_doubles(int ne, int np);
 size_t gam3_r4_doubles(int ne, int np);
 // gee_in / hc_in (optional, device): GAM_ee and Hcore already built by the
 // caller (C-order [i][j][k][l] and [i][j]); copied instead of recomputed.
-cudaError_t launch_gam3_aux(const DevSystem& sys, double* aux, cudaStream_t s,
-                            const double* gee_in = nullptr,
-                            const double* hc_in = nullptr);
+// w3_in: GM2sICR, which is W3 (the overlaps of the same geminal pairs).
+// scratch: gam2_scratch_doubles(sys, 1, npbf(npbf+1)/2).
+cudaError_t launch_gam3_aux(const DevSystem& sys, double* aux, double* scratch, cudaStream_t s,
+                            const double* gee_in = nullptr, const double* hc_in = nullptr,
+                            const double* w3_in = nullptr);
+// W1, W3 and (unless null) the core Hamiltonian [i][j] (k_gam2.cu)
+cudaError_t launch_gam3_factors(const DevSystem& sys, double* scratch, const double* w3_in,
+                                double* W1, double* W3, double* hc, cudaStream_t s);
 // R4 into aux.  fp32 = 1: the four-particle integrals in FP32 with FP64
 // Boys function, seeds and sums (mixed path).  screen > 0: (bra, ket)
 // pairs whose Schwarz-type estimate is below it are skipped.
@@ -242,7 +249,8 @@ cudaError_t launch_gam3_raw_range(const DevSystem& sys, const double* aux,
                                   cudaStream_t s);
 // pair records of the gam_3 builder (sys.g3i must be set)
 size_t g3_record_doubles(int nket, int np);
-cudaError_t launch_g3_records(const DevSystem& sys, double* rec, cudaStream_t s);
+size_t g3_gradient_doubles(int nket, int np);
+cudaError_t launch_g3_records(const DevSystem& sys, double* rec, double* grad, cudaStream_t s);
 constexpr int kG3MaxTileKets = 1024;
 constexpr double kScreenThreshold = 1.0e-12;   // NEOXC_SCF_SCREEN
 // Many systems of one angular class in one persistent launch: both passes of
@@ -283,7 +291,7 @@ cudaError_t launch_gam_ep(const DevSystem& sys, double* Gep, cudaStream_t s);
 // pairs_only = 1: RXCHF_GAM1_OMP_MD (rxchf/rxchf_gam_1_OMP.f), the
 // geminal-pair terms only.
 cudaError_t launch_gam1(const DevSystem& sys, double* G1, double* G1s,
-                        cudaStream_t s, int fp32 = 0, int pairs_only = 0);
+                        cudaStream_t s, int pairs_only = 0);
 size_t scf_fock1_part_doubles(int ne, int np);
 cudaError_t launch_scf_fock1(int ne, int np, int nelec, const double* Hce,
                              const double* Hcp, const double* Gep,

@@ -105,4 +105,30 @@ double hc_boys_ref(int L, double T, const double* B) {
   for (int m = 0; m <= L; m++) s += F[m] * B[m];
   return s;
 }
+
+// got/ref pairs of one (electron, proton) pair: pair_kinetic, the
+// multiplicative terms and the overlap of two_body, pair_coulomb; mag: the
+// size of the multiplicative terms.
+void hc_gam1(const HP* hA, const HP* hB, double gk, double gl, int nat, const double* cat,
+             const double* zan, double m, double* got, double* ref, double* mag) {
+  Prim A[2], B[2];
+  for (int i = 0; i < 2; i++) { A[i] = cv(hA[i]); B[i] = cv(hB[i]); }
+  double r[2][g3::kRLen];
+  for (int i = 0; i < 2; i++) g3::fill_pair_record(A[i], B[i], 1.0, 1.0, r[i]);
+  got[0] = g2::pair_kinetic(A[0], A[1], B[0], B[1], gk, gl, m);
+  ref[0] = md::pgike1(A[0], A[1], B[0], B[1], gk, gl, m);
+  g2::two_body<2, 2>(r[0], r[1], gk + gl, nat, cat, zan, &got[1], &got[2]);
+  double ve = 0.0, vp = 0.0, me = 0.0;
+  for (int c = 0; c < nat; c++) {
+    const double x = zan[c] * md::g2_xggvec(A[0], A[1], B[0], B[1], gk, gl, cat + 3 * c);
+    const double y = zan[c] * md::g2_xggvec(A[1], A[0], B[1], B[0], gk, gl, cat + 3 * c);
+    ve += x; vp += y; me += fabs(x) + fabs(y);
+  }
+  const double vm = md::g2_xggvee(A[0], A[1], B[0], B[1], gk, gl);
+  ref[1] = vp - ve - vm;
+  *mag = me + fabs(vm);
+  ref[2] = md::g2_xggs(A[0], A[1], B[0], B[1], gk, gl);
+  got[3] = g2::pair_coulomb<8>(r[0], r[1]);
+  ref[3] = md::gfvee(A[0], A[1], B[0], B[1]);
+}
 }

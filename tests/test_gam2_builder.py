@@ -57,6 +57,36 @@ def test_pair_density_integrals_match_element_integrals(host, le, ln):
             assert abs(x - y) <= 1e-10 * abs(y) + 1e-14 * max(abs(pair).max(), abs(ov).max())
 
 
+@pytest.mark.parametrize("le,ln", [(0, 0), (1, 2), (2, 2)])
+def test_two_particle_integrals_match_element_integrals(host, le, ln):
+    """GAM_1's kinetic, multiplicative and overlap integrals and the plain
+    Coulomb integral of two pair densities (csrc/k_pair.cu)."""
+    rng = np.random.Generator(np.random.PCG64(7 + 10 * le + ln))
+    V, D = C.c_void_p, C.c_double
+
+    def prim(lmax, lo, hi, centre):
+        p = _HP()
+        p.a = float(np.exp(rng.uniform(np.log(lo), np.log(hi))))
+        for _ in range(int(rng.integers(0, lmax + 1))):
+            p.l[int(rng.integers(0, 3))] += 1
+        for d in range(3):
+            p.c[d] = float(centre[d])
+        return p
+    for _ in range(80):
+        cp = rng.uniform(-1, 1, 3)
+        A = (_HP * 2)(prim(le, 0.1, 20, rng.uniform(-1, 1, 3)), prim(ln, 4, 32, cp))
+        B = (_HP * 2)(prim(le, 0.1, 20, rng.uniform(-1, 1, 3)), prim(ln, 4, 32, cp))
+        gk, gl = rng.uniform(0.1, 10, 2)
+        cat, zan = rng.uniform(-1.5, 1.5, 6), np.array([1.0, 3.0])
+        got, ref, mag = np.zeros(4), np.zeros(4), np.zeros(1)
+        host.hc_gam1(A, B, D(gk), D(gl), 2, cat.ctypes.data_as(V), zan.ctypes.data_as(V), D(1836.0),
+                     *[x.ctypes.data_as(V) for x in (got, ref, mag)])
+        err = np.abs(got - ref)
+        assert err[0] <= 1e-11 * abs(ref[0]) + 1e-16
+        assert err[1] <= 1e-11 * mag[0]
+        assert (err[2:] <= 1e-10 * np.abs(ref[2:]) + 1e-16).all()
+
+
 @pytest.mark.parametrize("L", [0, 1, 2, 7, 12, 16])
 def test_boys_dot_is_the_boys_function(host, L):
     """One recursion for both ranges of T: the table's grid points and their
