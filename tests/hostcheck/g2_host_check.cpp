@@ -68,11 +68,15 @@ void hc_gam2(const HP* hA, const HP* hB, int ng, const double* gm, int nat, cons
       item(A, B, gm[k], gm[l], nat, cat, zan, pmass, ref);
       item(A2, B2, gm[k], gm[l], nat, cat, zan, pmass, ref);
       double x, y;
-      g2::three_body<2, 2, true>(r[0], r[1], r[2], e[0], e[1], e[2], gm[k], gm[l], nat, cat, zan,
+      g2::three_body<2, 2, g2::kAll>(r[0], r[1], r[2], e[0], e[1], e[2], gm[k], gm[l], nat, cat, zan,
                                  1.0 / pmass, &x, &y);
       got[0] += x;
       got[1] += y;
-      g2::three_body<2, 2, false>(r[0], r[1], r[2], e[0], e[1], e[2], gm[k], gm[l], nat, cat, zan,
+      double z;
+      g2::three_body<2, 2, g2::kOverlap>(r[0], r[1], r[2], e[0], e[1], e[2], gm[k], gm[l], nat, cat,
+                                         zan, 1.0 / pmass, &x, &z);
+      if (!(fabs(z - y) <= 1e-12 * fabs(y))) got[1] = NAN;   // one overlap, two ways
+      g2::three_body<2, 2, g2::kCoulomb12>(r[0], r[1], r[2], e[0], e[1], e[2], gm[k], gm[l], nat, cat, zan,
                                   1.0 / pmass, &x, &y);
       got[2] += y;
     }
