@@ -34,90 +34,18 @@
 // GAM_ee = pack_4D(je2,ie2,je1,ie1) and of one proton pair of GAM_2s =
 // index_GAM_2PK), so a table read is a linear offset.  All arithmetic is
 // FP64; table reads pass through the reference's underflow (|x|<1e-100 -> 0).
+#include <utility>
+
 #include "neoxc_internal.h"
 #include "tc_gemm.cuh"
 
 namespace neoxc {
 namespace {
 
+// |x| < 1e-100 -> 0 (underflow.f:2-11), compared as integers: an FP64 compare
+// would cost as much as the FMA that uses the element
 __device__ __forceinline__ double flush(double x) {
-  return fabs(x) < 1.0e-100 ? 0.0 : x;   // underflow.f:2-11
-}
-
-// ---- 1. G = sum_p DP(p) GAM_2s(p) ------------------------------------------
-__global__ void dp_contract_kernel(long long n4, int np,
-                                   const double* __restrict__ g2s,
-                                   const double* __restrict__ DP,
-                                   double* __restrict__ G) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < n4;
-       r += stride) {
-    double acc = 0.0;
-    for (int ip = 0; ip < np; ip++)
-      for (int jp = 0; jp < np; jp++)
-        acc = fma(DP[ip + np * jp],
-                  flush(__ldg(g2s + (long long)(ip * np + jp) * n4 + r)), acc);
-    G[r] = acc;
-  }
-}
-
-// ---- 2. one-index transforms ------------------------------------------------
-// out[row][y] = sum_k in[row][k] * M(y,k),  M(y,k) = M[y*sy + k*sk];
-// rows = n^3.  A CTA stages RB rows of `in` and M^T in shared memory.
-template <bool FLUSH>
-__global__ void xform_last_kernel(int n, long long nrow,
-                                  const double* __restrict__ in,
-                                  const double* __restrict__ M, int sy, int sk,
-                                  double* __restrict__ out) {
-  extern __shared__ double sm[];
-  double* sMt = sm;            // [k][y]
-  double* sIn = sm + n * n;    // [RB][n]
-  const int RB = blockDim.x / n;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int k = e / n, y = e - k * n;
-    sMt[e] = M[(long long)y * sy + (long long)k * sk];
-  }
-  const int rl = threadIdx.x / n, y = threadIdx.x - rl * n;
-  for (long long r0 = (long long)blockIdx.x * RB; r0 < nrow;
-       r0 += (long long)gridDim.x * RB) {
-    __syncthreads();
-    for (int e = threadIdx.x; e < RB * n; e += blockDim.x) {
-      const long long row = r0 + e / n;
-      double v = row < nrow ? in[row * n + (e % n)] : 0.0;
-      sIn[e] = FLUSH ? flush(v) : v;
-    }
-    __syncthreads();
-    const long long row = r0 + rl;
-    if (rl < RB && row < nrow) {
-      double acc = 0.0;
-      for (int k = 0; k < n; k++) acc = fma(sIn[rl * n + k], sMt[k * n + y], acc);
-      out[row * n + y] = acc;
-    }
-  }
-}
-
-// out[a][x][j] = sum_b M(x,b) * in[a][b][j],  j < m = n^2,  M(x,b) = M[x*sx + b*sb]
-__global__ void xform_second_kernel(int n, int m, const double* __restrict__ in,
-                                    const double* __restrict__ M, int sx, int sb,
-                                    double* __restrict__ out) {
-  extern __shared__ double sM[];   // [x][b]
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int x = e / n, b = e - x * n;
-    sM[e] = M[(long long)x * sx + (long long)b * sb];
-  }
-  __syncthreads();
-  const long long total = (long long)n * n * m;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < total;
-       o += stride) {
-    const long long am = o / m;
-    const int j = (int)(o - am * m);
-    const int a = (int)(am / n), x = (int)(am - (long long)a * n);
-    const double* src = in + (long long)a * n * m + j;
-    double acc = 0.0;
-    for (int b = 0; b < n; b++) acc = fma(sM[x * n + b], src[(long long)b * m], acc);
-    out[o] = acc;
-  }
+  return (__double_as_longlong(x) & 0x7fffffffffffffffLL) < 0x2b2bff2ee48e0530LL ? 0.0 : x;
 }
 
 // ---- 3. partial and double traces ------------------------------------------
@@ -290,23 +218,6 @@ __device__ __forceinline__ double block_sum(double v, double* sw) {
   return t;   // valid in thread 0
 }
 
-// grid (nchunk, np*np): part[p*nchunk + chunk]
-__global__ void fockp_dot_kernel(long long n4, int nchunk,
-                                 const double* __restrict__ g2s,
-                                 const double* __restrict__ W,
-                                 double* __restrict__ part) {
-  __shared__ double sw[32];
-  const int p = blockIdx.y;
-  const long long base = (long long)blockIdx.x * kDotChunk;
-  const long long end = base + kDotChunk < n4 ? base + kDotChunk : n4;
-  const double* g = g2s + (long long)p * n4;
-  double acc = 0.0;
-  for (long long r = base + threadIdx.x; r < end; r += blockDim.x)
-    acc = fma(flush(__ldg(g + r)), W[r], acc);
-  const double t = block_sum(acc, sw);
-  if (threadIdx.x == 0) part[(long long)p * nchunk + blockIdx.x] = t;
-}
-
 // One CTA: fockp(ip,jp) (+)= sum_chunk part; E = sum_p DP(p) * (new part).
 __global__ void fockp_reduce_kernel(int np, int nchunk,
                                     const double* __restrict__ part,
@@ -438,55 +349,290 @@ fockp_dot_mixed_kernel(long long n4, int nchunk, int np2,
   }
 }
 
-// ---- 6. focke ---------------------------------------------------------------
-// CTA per (a,c): part[(a*n+c)][x*n+b] = sum_y Ws(a,x,c,y) H_G(a,b,c,y)
-//                                      + Vs(a,x,c,y) H_E(a,b,c,y),
-// Ws(a,x,c,y) = Wp(a,x,c,y) + Wp(c,y,a,x) (likewise Vs).
-__global__ void focke_part_kernel(int n, const double* __restrict__ Wp,
-                                  const double* __restrict__ HG,
-                                  const double* __restrict__ Vp,
-                                  const double* __restrict__ HE,
-                                  double* __restrict__ part) {
-  extern __shared__ double sm[];
-  double* sS = sm;           // [x][y]
-  double* sH = sm + n * n;   // [b][y]
-  const int a = blockIdx.x / n, c = blockIdx.x - a * n;
-  const int nn = n * n;
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};   // up to 4 outputs per thread (n <= 64, 1024 threads)
-  for (int pass = 0; pass < 2; pass++) {
-    const double* X = pass ? Vp : Wp;
-    const double* H = pass ? HE : HG;
-    __syncthreads();
-    for (int e = threadIdx.x; e < nn; e += blockDim.x) {
-      const int u = e / n, y = e - u * n;
-      sS[e] = X[idx4(n, a, u, c, y)] + X[idx4(n, c, y, a, u)];
-      sH[e] = H[idx4(n, a, u, c, y)];
-    }
-    __syncthreads();
-    int q = 0;
-    for (int e = threadIdx.x; e < nn; e += blockDim.x, q++) {
-      const int x = e / n, b = e - x * n;
-      double s = 0.0;
-      for (int y = 0; y < n; y++) s = fma(sS[x * n + y], sH[b * n + y], s);
-      acc[q] += s;
-    }
+// ---- FP64 build: four launches, a CTA per leg pair (a, c) --------------------
+// Fixing the bra legs a and c of both electron pairs leaves an n x n tile in
+// (b, d) or (x, y), on which every step but the traces is local: the sum over
+// proton pairs, both one-index transforms, the gradient, the back transforms,
+// the dot with GAM_2s and the focke products.  So one kernel goes from GAM_2s
+// and GAM_ee to H and T', one forms the traces, one goes from T' to partial
+// fockp and focke, and one adds the partials up; a tile stays in shared
+// memory in between.  (As fourteen kernels over whole tensors the build at
+// n = 12, np = 8 spent its time on launches and on threads that walked 64
+// proton pairs or 144 partials one load at a time: 109 us; see
+// launch_gam4_factored for the time now.)  At large n the n^5 products and
+// the two FMAs per GAM_2s element are FP64-bound.
+
+// out[i][j] = sum_k A(i, k) B(k, j), the products of n x n tiles below.
+// AT / BT: that factor stored transposed.  Rows are ld = n | 1 doubles apart:
+// with an odd pitch neither rows nor columns of a tile fall on one bank.
+template <bool AT, bool BT>
+__device__ __forceinline__ void tile_mul(int n, int ld, const double* A, const double* B, double* out) {
+  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+    const int i = e / n, j = e - i * n;
+    double s = 0.0;
+#pragma unroll 4
+    for (int k = 0; k < n; k++)
+      s = fma(AT ? A[k * ld + i] : A[i * ld + k], BT ? B[j * ld + k] : B[k * ld + j], s);
+    out[i * ld + j] = s;
   }
-  int q = 0;
-  for (int e = threadIdx.x; e < nn; e += blockDim.x, q++)
-    part[(long long)blockIdx.x * nn + e] = acc[q];
 }
 
-// focke(x,b) (+)= sum_{(a,c)} part[(a,c)][x*n+b]   (column-major focke)
-__global__ void focke_reduce_kernel(int n, const double* __restrict__ part,
-                                    int accumulate, double* __restrict__ focke) {
-  const int nn = n * n;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nn;
-       e += gridDim.x * blockDim.x) {
+// grid (n^2, 2): y = 0: G = sum_p DP(p) GAM_2s(p) -> HG, Gp; y = 1: GAM_ee -> HE, Ep.
+// H(a,b,c,y) = sum_d T(a,b,c,d) DE(y,d), T'(a,x,c,y) = sum_b DE(x,b) H(a,b,c,y).
+constexpr int kForwardThreads = 1024;
+__global__ void __launch_bounds__(kForwardThreads)
+gam4f_forward_kernel(int n, int np, const double* __restrict__ gee,
+                     const double* __restrict__ g2s, const double* __restrict__ DE,
+                     const double* __restrict__ DP, double* __restrict__ HG,
+                     double* __restrict__ Gp, double* __restrict__ HE, double* __restrict__ Ep,
+                     unsigned* __restrict__ counter) {
+  extern __shared__ double sm[];
+  const int n2 = n * n, np2 = np * np, ld = n | 1;
+  const long long n4 = (long long)n2 * n2;
+  double* sDE = sm;            // DE(i,j) at [j][i] (column-major)
+  double* sT = sDE + n * ld;
+  double* sH = sT + n * ld;
+  double* sred = sH + n * ld;  // [blockDim]
+  const int a = blockIdx.x / n, c = blockIdx.x - a * n;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *counter = 0u;
+  for (int e = threadIdx.x; e < n2; e += blockDim.x) sDE[(e / n) * ld + e % n] = DE[e];
+  const long long base = (long long)a * n * n2 + (long long)c * n;   // + b n^2 + d
+  if (blockIdx.y) {
+    for (int e = threadIdx.x; e < n2; e += blockDim.x) {
+      const int b = e / n, d = e - b * n;
+      sT[b * ld + d] = flush(__ldg(gee + base + (long long)b * n2 + d));
+    }
+  } else if (n2 >= (int)blockDim.x) {
+    for (int e = threadIdx.x; e < n2; e += blockDim.x) {
+      const int b = e / n, d = e - b * n;
+      const double* g = g2s + base + (long long)b * n2 + d;
+      double acc = 0.0;
+      int ip = 0, jp = 0;
+#pragma unroll 8
+      for (int p = 0; p < np2; p++) {
+        acc = fma(__ldg(DP + ip + np * jp), flush(__ldg(g + p * n4)), acc);
+        if (++jp == np) { jp = 0; ip++; }
+      }
+      sT[b * ld + d] = acc;
+    }
+  } else {
+    // fewer elements than threads: groups of n^2 threads share the proton pairs
+    const int ng = blockDim.x / n2, grp = threadIdx.x / n2, e = threadIdx.x - grp * n2;
+    double acc = 0.0;
+    if (grp < ng) {
+      const int b = e / n, d = e - b * n;
+      const double* g = g2s + base + (long long)b * n2 + d;
+#pragma unroll 8
+      for (int p = grp; p < np2; p += ng)
+        acc = fma(__ldg(DP + p / np + np * (p % np)), flush(__ldg(g + p * n4)), acc);
+    }
+    sred[threadIdx.x] = acc;
+    __syncthreads();
+    if ((int)threadIdx.x < n2) {
+      double s = 0.0;
+      for (int k = 0; k < ng; k++) s += sred[k * n2 + threadIdx.x];
+      sT[(threadIdx.x / n) * ld + threadIdx.x % n] = s;
+    }
+  }
+  __syncthreads();
+  double* H = blockIdx.y ? HE : HG;
+  double* T = blockIdx.y ? Ep : Gp;
+  // H[b][y] = sum_d T[b][d] DE(y,d), DE(y,d) at [d][y]
+  tile_mul<false, false>(n, ld, sT, sDE, sH);
+  __syncthreads();
+  // T'[x][y] = sum_b DE(x,b) H[b][y], DE(x,b) at [b][x]
+  tile_mul<true, false>(n, ld, sDE, sH, sT);
+  __syncthreads();
+  for (int e = threadIdx.x; e < n2; e += blockDim.x) {
+    const int b = e / n, d = e - b * n;
+    H[base + (long long)b * n2 + d] = sH[b * ld + d];
+    T[base + (long long)b * n2 + d] = sT[b * ld + d];
+  }
+}
+
+// dE/d(the tensor on slots 0, 1) at legs l, from the other tensor T, its leg-pair
+// traces P and its double traces S (sig_code's table)
+__device__ __forceinline__ double grad_term(int n, const int* l, const double* __restrict__ T,
+                                            const double* __restrict__ P, const double* S) {
+  double acc = 0.0;
+#pragma unroll
+  for (int t = 0; t < 24; t++) {
+    const int code = sig_code(t);
+    const int dm = (code >> 2) & 15;
+    if ((dm & 1) && l[0] != l[1]) continue;
+    if ((dm & 2) && l[2] != l[3]) continue;
+    if ((dm & 4) && l[0] != l[3]) continue;
+    if ((dm & 8) && l[1] != l[2]) continue;
+    const int kind = (code >> 6) & 3, tid = (code >> 8) & 7;
+    const int s0 = (code >> 11) & 7, s1 = (code >> 14) & 7,
+              s2 = (code >> 17) & 7, s3 = (code >> 20) & 7;
+    double v;
+    if (kind == 0) {
+      v = __ldg(T + idx4(n, l[s0], l[s1], l[s2], l[s3]));
+    } else if (kind == 1) {
+      int uv[2], q = 0;
+      if (s0 != 7) uv[q++] = l[s0];
+      if (s1 != 7) uv[q++] = l[s1];
+      if (s2 != 7) uv[q++] = l[s2];
+      if (s3 != 7) uv[q++] = l[s3];
+      v = __ldg(P + ((size_t)tid * n + uv[0]) * n + uv[1]);
+    } else {
+      v = S[tid];
+    }
+    acc = fma(sig_coef(code & 3), v, acc);
+  }
+  return acc;
+}
+
+// Sums of v[0..3] over the warp: lane's result is that of v[(lane >> 3) & 3]
+// (six additions instead of twenty).
+__device__ __forceinline__ double warp_sum4(double v0, double v1, double v2, double v3, int lane) {
+  const bool hi = lane & 16, h2 = lane & 8;
+  double a = hi ? v2 : v0, b = hi ? v3 : v1;
+  a += __shfl_xor_sync(0xffffffffu, hi ? v0 : v2, 16);
+  b += __shfl_xor_sync(0xffffffffu, hi ? v1 : v3, 16);
+  double r = h2 ? b : a;
+  r += __shfl_xor_sync(0xffffffffu, h2 ? a : b, 8);
+  r += __shfl_xor_sync(0xffffffffu, r, 4);
+  r += __shfl_xor_sync(0xffffffffu, r, 2);
+  r += __shfl_xor_sync(0xffffffffu, r, 1);
+  return r;
+}
+
+// grid n^2: tile (a, c) of dE/dG', dE/dE' -> epart[(a,c)][x*n + b] and
+// fpart[p][(a,c)] = sum_bd GAM_2s(p; ab; cd) W(ab; cd).
+constexpr int kBackwardThreads = 512;
+__global__ void __launch_bounds__(kBackwardThreads)
+gam4f_backward_kernel(int n, int np, const double* __restrict__ g2s,
+                      const double* __restrict__ DE, const double* __restrict__ HG,
+                      const double* __restrict__ Gp, const double* __restrict__ HE,
+                      const double* __restrict__ Ep, const double* __restrict__ PT,
+                      double* __restrict__ epart, double* __restrict__ fpart) {
+  extern __shared__ double sm[];
+  const int n2 = n * n, np2 = np * np, ld = n | 1, tl = n * ld;
+  const long long n4 = (long long)n2 * n2;
+  double* sDE = sm;
+  double* sW = sDE + tl;       // Wp(a,x,c,y)
+  double* sX = sW + tl;        // Wp(a,x,c,y) + Wp(c,y,a,x)
+  double* sY = sX + tl;        // the same of Vp
+  double* sHG = sY + tl;       // [b][y]
+  double* sHE = sHG + tl;
+  __shared__ double sST[8];
+  const int a = blockIdx.x / n, c = blockIdx.x - a * n;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long base = (long long)a * n * n2 + (long long)c * n;
+  const double* PG = PT;
+  const double* PE = PT + 6 * n2;
+  // double traces (01)(23), (02)(13), (03)(12): traces of the first three tables
+  if (warp < 6) {
+    const double* P = (warp < 3 ? PG : PE) + (size_t)(warp % 3) * n2;
     double s = 0.0;
-    for (int ac = 0; ac < nn; ac++) s += part[(long long)ac * nn + e];
+    for (int u = lane; u < n; u += 32) s += P[u * n + u];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) sST[(warp / 3) * 4 + warp % 3] = s;
+  }
+  for (int e = threadIdx.x; e < n2; e += blockDim.x) {
+    const int b = e / n, d = e - b * n;
+    sDE[b * ld + d] = DE[e];
+    sHG[b * ld + d] = HG[base + (long long)b * n2 + d];
+    sHE[b * ld + d] = HE[base + (long long)b * n2 + d];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < n2; e += blockDim.x) {
+    const int x = e / n, y = e - x * n;
+    const int l[4] = {a, x, c, y}, m[4] = {c, y, a, x};
+    const double w = grad_term(n, l, Ep, PE, sST + 4);
+    sW[x * ld + y] = w;
+    sX[x * ld + y] = w + grad_term(n, m, Ep, PE, sST + 4);
+    sY[x * ld + y] = grad_term(n, l, Gp, PG, sST) + grad_term(n, m, Gp, PG, sST);
+  }
+  __syncthreads();
+  // focke(x,b) of this tile: sum_y X[x][y] HG[b][y] + Y[x][y] HE[b][y]
+  for (int e = threadIdx.x; e < n2; e += blockDim.x) {
     const int x = e / n, b = e - x * n;
-    const int f = x + n * b;
-    focke[f] = accumulate ? focke[f] + s : s;
+    double s = 0.0, t = 0.0;
+#pragma unroll 4
+    for (int y = 0; y < n; y++) {
+      s = fma(sX[x * ld + y], sHG[b * ld + y], s);
+      t = fma(sY[x * ld + y], sHE[b * ld + y], t);
+    }
+    epart[(long long)blockIdx.x * n2 + e] = s + t;
+  }
+  __syncthreads();
+  // W[b][d] = sum_xy Wp[x][y] DE(x,b) DE(y,d), through Ht[x][d] (in sX) into sY;
+  // DE(y,d) at [d][y], DE(x,b) at [b][x]
+  tile_mul<false, true>(n, ld, sW, sDE, sX);
+  __syncthreads();
+  tile_mul<false, false>(n, ld, sDE, sX, sY);
+  __syncthreads();
+  // four proton pairs of a warp at a time
+  const int nw = blockDim.x >> 5;
+  for (int p0 = warp * 4; p0 < np2; p0 += nw * 4) {
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int e = lane; e < n2; e += 32) {
+      const int b = e / n, d = e - b * n;
+      const double* g = g2s + base + (long long)b * n2 + d;
+      const double w = sY[b * ld + d];
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (p0 + k < np2) v[k] = fma(flush(__ldg(g + (p0 + k) * n4)), w, v[k]);
+    }
+    const double r = warp_sum4(v[0], v[1], v[2], v[3], lane);
+    if ((lane & 7) == 0 && p0 + (lane >> 3) < np2)
+      fpart[(long long)(p0 + (lane >> 3)) * n2 + blockIdx.x] = r;
+  }
+}
+
+// CTAs [0, ne_ctas): 32 focke elements each, 32 warps sharing the n^2 tiles; the
+// others: 32 proton pairs each.  The last of those to finish adds E up.
+__global__ void __launch_bounds__(1024)
+gam4f_reduce_kernel(int n, int np, int ne_ctas, const double* __restrict__ epart,
+                    const double* __restrict__ fpart, const double* __restrict__ DP,
+                    int accumulate, double* __restrict__ focke, double* __restrict__ fockp,
+                    double* __restrict__ evals, unsigned* __restrict__ counter,
+                    double* __restrict__ E) {
+  __shared__ double sr[32][33];
+  __shared__ bool last;
+  const int n2 = n * n, np2 = np * np, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if ((int)blockIdx.x < ne_ctas) {
+    const int e = blockIdx.x * 32 + lane;
+    double s = 0.0;
+    if (e < n2) {
+#pragma unroll 8
+      for (int t = warp; t < n2; t += 32) s += epart[(long long)t * n2 + e];
+    }
+    sr[warp][lane] = s;
+    __syncthreads();
+    double v = sr[lane][warp];   // warp = element now, lane = share
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    const int q = blockIdx.x * 32 + warp;
+    if (lane == 0 && q < n2) {
+      const int f = q / n + n * (q % n);   // focke(x,b), column-major
+      focke[f] = accumulate ? focke[f] + v : v;
+    }
+    return;
+  }
+  const int p = (blockIdx.x - ne_ctas) * 32 + warp;
+  double v = 0.0;
+  if (p < np2) {
+    for (int t = lane; t < n2; t += 32) v += fpart[(long long)p * n2 + t];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) {
+      const int f = p / np + np * (p % np);
+      fockp[f] = accumulate ? fockp[f] + v : v;
+      evals[p] = DP[f] * v;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - ne_ctas - 1;
+  __syncthreads();
+  if (last && warp == 0) {
+    __threadfence();
+    double s = 0.0;
+    for (int k = lane; k < np2; k += 32) s += __ldcg(evals + k);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) *E = s;
   }
 }
 
@@ -752,12 +898,13 @@ cudaError_t launch_pair_symmetry_check(int ne, int np, const double* gee,
 }
 
 size_t gam4f_scratch_doubles(int ne, int np) {
-  const size_t n4 = (size_t)ne * ne * ne * ne;
-  const size_t nchunk = (n4 + kDotChunk - 1) / kDotChunk;
-  // G, H_G, G', H_E, E', Wp, Vp + PT(2x6 n^2) + ST(8) + fockp partials
-  return 7 * n4 + 12 * (size_t)ne * ne + 8 + (size_t)np * np * nchunk;
+  const size_t n2 = (size_t)ne * ne, n4 = n2 * n2, p2 = (size_t)np * np;
+  // H_G, G', H_E, E', focke partials; leg-pair traces; fockp partials,
+  // energy terms; counter
+  return 5 * n4 + 12 * n2 + p2 * n2 + p2 + 1;
 }
 
+// Measured (one GB300): n = 12, np = 8: 46 us a call, 71 us by itself (109 us and 301 us as fourteen launches).
 cudaError_t launch_gam4_factored(int ne, int np, const double* gee,
                                  const double* g2s, const double* DE,
                                  const double* DP, double* scratch,
@@ -765,59 +912,35 @@ cudaError_t launch_gam4_factored(int ne, int np, const double* gee,
                                  int accumulate, cudaStream_t s) {
   if (ne < 1 || ne > kGam4FactMaxNE || np < 1 || np > 255)
     return cudaErrorInvalidValue;
-  const int n = ne;
-  const long long n4 = (long long)n * n * n * n, n3 = (long long)n * n * n;
-  const int nchunk = (int)((n4 + kDotChunk - 1) / kDotChunk);
-  double* G = scratch;
-  double* HG = G + n4;
+  const int n = ne, n2 = n * n;
+  const size_t n4 = (size_t)n2 * n2, p2 = (size_t)np * np;
+  double* HG = scratch;
   double* Gp = HG + n4;
   double* HE = Gp + n4;
   double* Ep = HE + n4;
-  double* Wp = Ep + n4;
-  double* Vp = Wp + n4;
-  double* PT = Vp + n4;
-  double* ST = PT + 12 * n * n;
-  double* fpart = ST + 8;
-  // buffers reused once their contents are dead
-  double* Ht = Gp;      // back-transform intermediate (after the gradients)
-  double* W = Ep;       // back-transformed dE/dG'
-  double* epart = G;    // focke partials (n^2 x n^2 = n^4)
-
-  const int TB = 256;
-  const int RB = TB / n;
-  const int TBl = RB * n;                       // threads of xform_last
-  const size_t sm_last = sizeof(double) * ((size_t)n * n + (size_t)RB * n);
-  const size_t sm_second = sizeof(double) * n * n;
-  const int g_last = grid_for((n3 + RB - 1) / RB * TB, TB) ;
-  const int g_n4 = grid_for(n4, TB);
-
-  // 1. G = DP . GAM_2s
-  dp_contract_kernel<<<g_n4, TB, 0, s>>>(n4, np, g2s, DP, G);
-  // 2. H_G = G x DE (last index), G' = DE x H_G (second index); same for GAM_ee
-  xform_last_kernel<false><<<g_last, TBl, sm_last, s>>>(n, n3, G, DE, 1, n, HG);
-  xform_second_kernel<<<g_n4, TB, sm_second, s>>>(n, n * n, HG, DE, 1, n, Gp);
-  xform_last_kernel<true><<<g_last, TBl, sm_last, s>>>(n, n3, gee, DE, 1, n, HE);
-  xform_second_kernel<<<g_n4, TB, sm_second, s>>>(n, n * n, HE, DE, 1, n, Ep);
-  // 3. traces of G' (t=0) and E' (t=1)
-  traces_kernel<<<dim3(grid_for(6LL * n * n, TB), 2), TB, 0, s>>>(n, Gp, Ep, PT);
-  dtraces_kernel<<<1, 64, 0, s>>>(n, PT, ST);
-  // 4. Wp = dE/dG', Vp = dE/dE'
-  gam4f_grad_kernel<<<dim3(g_n4, 2), TB, 0, s>>>(n, Ep, Gp, PT, ST, Wp, Vp);
-  // 5. W = back-transform of Wp:  W(a,b,c,d) = sum_{x,y} Wp(a,x,c,y) DE(x,b) DE(y,d)
-  xform_last_kernel<false><<<g_last, TBl, sm_last, s>>>(n, n3, Wp, DE, n, 1, Ht);
-  xform_second_kernel<<<g_n4, TB, sm_second, s>>>(n, n * n, Ht, DE, n, 1, W);
-  fockp_dot_kernel<<<dim3(nchunk, np * np), kDotTB, 0, s>>>(n4, nchunk, g2s, W, fpart);
-  fockp_reduce_kernel<<<1, 256, 0, s>>>(np, nchunk, fpart, DP, accumulate, fockp, E);
-  // 6. focke
-  const int tbf = n * n < 1024 ? ((n * n + 31) / 32) * 32 : 1024;
-  if (2 * sm_second > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(
-        focke_part_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-        (int)(2 * sm_second));
-    if (e != cudaSuccess) return e;
-  }
-  focke_part_kernel<<<n * n, tbf, 2 * sm_second, s>>>(n, Wp, HG, Vp, HE, epart);
-  focke_reduce_kernel<<<grid_for((long long)n * n, TB), TB, 0, s>>>(n, epart, accumulate, focke);
+  double* epart = Ep + n4;
+  double* PT = epart + n4;
+  double* fpart = PT + 12 * n2;
+  double* evals = fpart + p2 * n2;
+  unsigned* counter = reinterpret_cast<unsigned*>(evals + p2);
+  // Threads beyond the n^2 elements of a tile share its proton pairs, so small
+  // n takes wide CTAs too (n = 12: seven groups of 144; 256 threads, one group
+  // walking all pairs, were 2.5x slower).
+  const size_t tile = (size_t)n * (n | 1);
+  const size_t smf = sizeof(double) * (3 * tile + kForwardThreads), smb = sizeof(double) * 6 * tile;
+  for (const auto& k : {std::make_pair((const void*)gam4f_forward_kernel, smf),
+                        std::make_pair((const void*)gam4f_backward_kernel, smb)})
+    if (k.second > 48 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(k.first, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)k.second);
+      if (e != cudaSuccess) return e;
+    }
+  gam4f_forward_kernel<<<dim3(n2, 2), kForwardThreads, smf, s>>>(n, np, gee, g2s, DE, DP, HG, Gp, HE, Ep, counter);
+  traces_kernel<<<dim3(grid_for(6LL * n2, 128), 2), 128, 0, s>>>(n, Gp, Ep, PT);
+  gam4f_backward_kernel<<<n2, kBackwardThreads, smb, s>>>(n, np, g2s, DE, HG, Gp, HE, Ep, PT, epart, fpart);
+  const int ne_ctas = (n2 + 31) / 32;
+  gam4f_reduce_kernel<<<ne_ctas + (int)((p2 + 31) / 32), 1024, 0, s>>>(
+      n, np, ne_ctas, epart, fpart, DP, accumulate, focke, fockp, evals, counter, E);
   return cudaGetLastError();
 }
 

@@ -180,9 +180,11 @@ cudaError_t launch_t(int ne, long long nipjp, const double* G, const double* W, 
   if (lanes > ne * ne) lanes = ne * ne;
   const int bs = lanes * ne, pt1 = ne | 1, pt0 = (pt1 * ne) | 1;
   const size_t smem = sizeof(double) * ((size_t)pt0 * ne + 3 * NC * (size_t)ne * ne + bs);
-  cudaError_t e = cudaFuncSetAttribute(rank3_kernel<NC, USED>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(rank3_kernel<NC, USED>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
   rank3_kernel<NC, USED><<<(unsigned)(nipjp * ne * ne), bs, smem, s>>>(ne, G, W, DA, DB, part, ppart);
   return cudaGetLastError();
 }
