@@ -162,108 +162,169 @@ __global__ void eg2_kernel(int ne, int np, const double* __restrict__ DE,
 //   FAE[c]     += sum_r DP(ip,jp) DBE(i1,j1) M[r][c]
 //   v[r]        = sum_c DAE[c] M[r][c]
 //   FBE(i1,j1) += sum_{ip,jp} DP v[r];  FP(ip,jp) += sum_{i1,j1} DBE v[r]
-constexpr int kOmgRows = 8;
-__global__ void __launch_bounds__(256)
-omg2_kernel(int ne, int np, long long nrows, int rows_per_cta,
+// Two FP64 FMAs an element are what bounds it (2 per SM and clock: 3.9 ms of
+// FMAs at ne = 40, np = 20 against 1.2 ms of HBM), so everything beside them
+// is kept off the FP64 pipe and out of its way: a warp works alone (no barrier
+// holds back the others' loads) on a panel of 32 * COLS columns, whose DAE and
+// FAE stay in registers; it loads the next column's eight rows while it
+// multiplies this one's, forms 32 row weights at a time, and sums eight rows'
+// dots over its lanes by a transposing butterfly (one addition per row instead
+// of five).  Measured there: 7.75 ms with a CTA of 256 threads per row and a
+// tree per row, 6.5 ms with register columns but barriers every eight rows,
+// 3.7 ms so (96 % of the FP64 pipe).
+constexpr int kOmgRows = 8, kOmgCols = 10, kOmgWarps = 2;
+
+// Columns a lane holds: as many as fit, in panels of even size.
+__host__ __device__ inline int omg2_panels(int n2) {
+  return (n2 + 32 * kOmgCols - 1) / (32 * kOmgCols);
+}
+inline int omg2_cols(int n2) {
+  const int per = (n2 + omg2_panels(n2) - 1) / omg2_panels(n2);
+  return (per + 31) / 32;
+}
+
+// warps: (row block, column panel), the panels of a row block side by side
+template <int COLS>
+__global__ void __launch_bounds__(32 * kOmgWarps, 16 / kOmgWarps)
+omg2_kernel(int ne, int np, long long nrows, int rows_per_block, int nblocks, int npanels,
             const double* __restrict__ DAE, const double* __restrict__ DBE,
             const double* __restrict__ DP, const double* __restrict__ g2,
             double* __restrict__ fae_part, double* __restrict__ vrow) {
-  extern __shared__ double sm[];
-  const int n2 = ne * ne;
-  double* sDAE = sm;
-  double* sFAE = sm + n2;
-  double* swarp = sFAE + n2;   // [8 warps][kOmgRows]
-  for (int k = threadIdx.x; k < n2; k += blockDim.x) {
-    sDAE[k] = DAE[k];
-    sFAE[k] = 0.0;
+  const int n2 = ne * ne, lane = threadIdx.x & 31;
+  const long long w = (long long)blockIdx.x * kOmgWarps + (threadIdx.x >> 5);
+  if (w >= (long long)nblocks * npanels) return;
+  const int panel = (int)(w % npanels), blk = (int)(w / npanels);
+  const int c0 = panel * 32 * COLS + lane;
+  const long long r0 = (long long)blk * rows_per_block;
+  const long long r1 = min(nrows, r0 + rows_per_block);
+  double dae[COLS], fae[COLS];
+#pragma unroll
+  for (int i = 0; i < COLS; i++) {
+    const int c = c0 + i * 32;
+    dae[i] = c < n2 ? DAE[c] : 0.0;
+    fae[i] = 0.0;
   }
-  __syncthreads();
-  const long long r0 = (long long)blockIdx.x * rows_per_cta;
-  const long long r1 = min(nrows, r0 + rows_per_cta);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double u = 0.0;   // weight of row (r - r0) % 32 == lane of the current 32 rows
   for (long long rb = r0; rb < r1; rb += kOmgRows) {
-    double dot[kOmgRows], u[kOmgRows];
+    if (((rb - r0) & 31) == 0) {
+      u = 0.0;
+      long long rr = rb + lane;
+      if (rr < r1) {
+        const int j1 = (int)(rr % ne); rr /= ne;
+        const int i1 = (int)(rr % ne); rr /= ne;
+        const int jp = (int)(rr % np), ip = (int)(rr / np);
+        u = DP[ip + np * jp] * DBE[i1 + ne * j1];
+      }
+    }
+    double su[kOmgRows], dot[kOmgRows];
+    const int sh = (int)((rb - r0) & 31);
 #pragma unroll
     for (int k = 0; k < kOmgRows; k++) {
+      su[k] = __shfl_sync(0xffffffffu, u, sh + k);
       dot[k] = 0.0;
-      long long rr = rb + k;
-      int j1 = (int)(rr % ne); rr /= ne;
-      int i1 = (int)(rr % ne); rr /= ne;
-      int jp = (int)(rr % np);
-      int ip = (int)((rr / np) % np);
-      u[k] = DP[ip + np * jp] * DBE[i1 + ne * j1];
     }
-    for (int c = threadIdx.x; c < n2; c += blockDim.x) {
-      double fa = 0.0;
-      const double dae = sDAE[c];
+    const double* g = g2 + rb * n2 + c0;
+    if (rb + kOmgRows <= r1) {
+      double m[2][kOmgRows];
 #pragma unroll
-      for (int k = 0; k < kOmgRows; k++) {
-        long long r = rb + k;
-        if (r < r1) {
-          double m = __ldg(g2 + r * n2 + c);
-          fa = fma(u[k], m, fa);
-          dot[k] = fma(dae, m, dot[k]);
+      for (int k = 0; k < kOmgRows; k++) m[0][k] = c0 < n2 ? __ldcs(g + (long long)k * n2) : 0.0;
+#pragma unroll
+      for (int i = 0; i < COLS; i++) {
+        if (i + 1 < COLS) {
+#pragma unroll
+          for (int k = 0; k < kOmgRows; k++)
+            m[(i + 1) & 1][k] = c0 + (i + 1) * 32 < n2 ? __ldcs(g + (long long)k * n2 + (i + 1) * 32) : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < kOmgRows; k++) {
+          fae[i] = fma(su[k], m[i & 1][k], fae[i]);
+          dot[k] = fma(dae[i], m[i & 1][k], dot[k]);
         }
       }
-      sFAE[c] += fa;   // column c is owned by exactly one thread
-    }
+    } else {
 #pragma unroll
-    for (int k = 0; k < kOmgRows; k++) {
-      double v = dot[k];
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-      if (lane == 0) swarp[warp * kOmgRows + k] = v;
+      for (int i = 0; i < COLS; i++)
+        if (c0 + i * 32 < n2)
+#pragma unroll
+          for (int k = 0; k < kOmgRows; k++)
+            if (rb + k < r1) {
+              const double m = __ldcs(g + (long long)k * n2 + i * 32);
+              fae[i] = fma(su[k], m, fae[i]);
+              dot[k] = fma(dae[i], m, dot[k]);
+            }
     }
-    __syncthreads();
-    if ((int)threadIdx.x < kOmgRows && rb + threadIdx.x < r1) {
-      double v = 0.0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); w++)
-        v += swarp[w * kOmgRows + threadIdx.x];
-      vrow[rb + threadIdx.x] = v;
+    // eight rows over 32 lanes: halve the rows a lane holds, then the lanes
+#pragma unroll
+    for (int h = 4, o = 16; h >= 1; h >>= 1, o >>= 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int k = 0; k < h; k++) {
+        const double keep = up ? dot[k + h] : dot[k], send = up ? dot[k] : dot[k + h];
+        dot[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
     }
-    __syncthreads();
+    double v = dot[0];   // row 4*(lane bit 4) + 2*(bit 3) + (bit 2)
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    if ((lane & 3) == 0 && rb + (lane >> 2) < r1) vrow[panel * nrows + rb + (lane >> 2)] = v;
   }
-  for (int c = threadIdx.x; c < n2; c += blockDim.x)
-    fae_part[(size_t)blockIdx.x * n2 + c] = sFAE[c];
+#pragma unroll
+  for (int i = 0; i < COLS; i++) {
+    const int c = c0 + i * 32;
+    if (c < n2) fae_part[(size_t)blk * n2 + c] = fae[i];
+  }
 }
 
-__global__ void omg2_reduce(int ne, int np, int nparts,
-                            const double* __restrict__ fae_part,
-                            const double* __restrict__ vrow,
-                            const double* __restrict__ DBE,
-                            const double* __restrict__ DP, double* FAE,
-                            double* FP, double* FBE, double* fp_tmp) {
-  const int n2 = ne * ne, p2 = np * np;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per output over the row blocks (FAE) or the rows (FBE: over p, FP:
+// over (i1,j1)); vrow's column panels are added as they are read.
+__global__ void __launch_bounds__(128)
+omg2_reduce(int ne, int np, int nparts, int npanels, const double* __restrict__ fae_part,
+            const double* __restrict__ vrow, const double* __restrict__ DBE,
+            const double* __restrict__ DP, double* FAE, double* FP, double* FBE,
+            double* __restrict__ fp_tmp) {
+  const int n2 = ne * ne, p2 = np * np, lane = threadIdx.x & 31;
+  const long long nrows = (long long)p2 * n2;
+  const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  double s = 0.0;
+  auto row = [&](long long r) {
+    double v = vrow[r];
+    for (int q = 1; q < npanels; q++) v += vrow[q * nrows + r];
+    return v;
+  };
   if (t < n2) {                       // FAE column c = i2*ne + j2
-    double s = 0.0;
-    for (int k = 0; k < nparts; k++) s += fae_part[(size_t)k * n2 + t];
-    int i2 = t / ne, j2 = t % ne;
-    if (FAE) FAE[i2 + ne * j2] += s;
+    for (int k = lane; k < nparts; k += 32) s += fae_part[(size_t)k * n2 + t];
   } else if (t < 2 * n2) {            // FBE(i1,j1)
-    int c = t - n2, i1 = c / ne, j1 = c % ne;
-    double s = 0.0;
-    for (int ipjp = 0; ipjp < p2; ipjp++) {
-      int ip = ipjp / np, jp = ipjp % np;
-      s = fma(DP[ip + np * jp], vrow[(size_t)ipjp * n2 + i1 * ne + j1], s);
-    }
-    if (FBE) FBE[i1 + ne * j1] += s;
+    for (int p = lane; p < p2; p += 32)
+      s = fma(DP[p / np + np * (p % np)], row((long long)p * n2 + t - n2), s);
   } else if (t < 2 * n2 + p2) {       // FP(ip,jp)
-    int ipjp = t - 2 * n2, ip = ipjp / np, jp = ipjp % np;
-    double s = 0.0;
-    for (int i1 = 0; i1 < ne; i1++)
-      for (int j1 = 0; j1 < ne; j1++)
-        s = fma(DBE[i1 + ne * j1], vrow[(size_t)ipjp * n2 + i1 * ne + j1], s);
-    if (FP) FP[ip + np * jp] += s;
-    fp_tmp[ipjp] = DP[ip + np * jp] * s;
+    const int p = t - 2 * n2;
+    for (int k = lane; k < n2; k += 32)
+      s = fma(DBE[k / ne + ne * (k % ne)], row((long long)p * n2 + k), s);
+  } else {
+    return;
+  }
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane) return;
+  if (t < n2) {
+    if (FAE) FAE[t / ne + ne * (t % ne)] += s;
+  } else if (t < 2 * n2) {
+    const int c = t - n2;
+    if (FBE) FBE[c / ne + ne * (c % ne)] += s;
+  } else {
+    const int p = t - 2 * n2, f = p / np + np * (p % np);
+    if (FP) FP[f] += s;
+    fp_tmp[p] = DP[f] * s;
   }
 }
 
-int omg2_parts(long long nrows) {
-  // a few waves over 152 SMs; each CTA streams a contiguous row range
-  long long want = 152LL * 8;
+// Row blocks: 16 warps a SM (the registers' limit), four rounds of them where
+// the tensor is long.
+int omg2_blocks(long long nrows, int panels) {
+  long long want = 152LL * 16 / panels;
+  if (want < 1) want = 1;
+  if (nrows > want * kOmgRows * 64) want *= 4;
   long long per = (nrows + want - 1) / want;
   per = ((per + kOmgRows - 1) / kOmgRows) * kOmgRows;
-  if (per < kOmgRows) per = kOmgRows;
   return (int)((nrows + per - 1) / per);
 }
 
@@ -383,8 +444,9 @@ cudaError_t launch_eg2_partials(int ne, int np, long long ipjp0,
 }
 
 size_t omg2_partial_doubles(int ne, int np) {
-  long long nrows = (long long)np * np * ne * ne;
-  return (size_t)omg2_parts(nrows) * ne * ne + (size_t)nrows + np * np;
+  const long long nrows = (long long)np * np * ne * ne;
+  const int n2 = ne * ne, panels = omg2_panels(n2);
+  return (size_t)omg2_blocks(nrows, panels) * ne * ne + (size_t)nrows * panels + np * np;
 }
 
 cudaError_t launch_rxchfne_omg2(int ne, int np, const double* DAE,
@@ -393,25 +455,35 @@ cudaError_t launch_rxchfne_omg2(int ne, int np, const double* DAE,
                                 double* FP, double* FBE, double* E,
                                 cudaStream_t s) {
   if (ne < 1 || np < 1 || ne * ne > 16384) return cudaErrorInvalidValue;
-  const long long nrows = (long long)np * np * ne * ne;
-  const int nparts = omg2_parts(nrows);
-  const int per = (int)((nrows + nparts - 1) / nparts);
-  const int rows_per_cta = ((per + kOmgRows - 1) / kOmgRows) * kOmgRows;
-  const int grid = (int)((nrows + rows_per_cta - 1) / rows_per_cta);
+  const int n2 = ne * ne, panels = omg2_panels(n2);
+  const long long nrows = (long long)np * np * n2;
+  const int want = omg2_blocks(nrows, panels);
+  const long long per = (nrows + want - 1) / want;
+  const int rows = (int)(((per + kOmgRows - 1) / kOmgRows) * kOmgRows);
+  const int grid = (int)((nrows + rows - 1) / rows);
   double* fae_part = scratch;
-  double* vrow = scratch + (size_t)nparts * ne * ne;
-  double* fp_tmp = vrow + nrows;
-  const size_t smem = sizeof(double) * (2 * (size_t)ne * ne + 8 * kOmgRows);
-  cudaError_t e = cudaFuncSetAttribute(omg2_kernel,
-      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  double* vrow = scratch + (size_t)want * n2;
+  double* fp_tmp = vrow + nrows * panels;
+  const unsigned ctas = (unsigned)(((long long)grid * panels + kOmgWarps - 1) / kOmgWarps);
+#define OMG(C) omg2_kernel<C><<<ctas, 32 * kOmgWarps, 0, s>>>(ne, np, nrows, rows, grid, panels, DAE, DBE, DP, g2, fae_part, vrow)
+  switch (omg2_cols(n2)) {   // no empty columns in the panels
+    case 1: OMG(1); break;
+    case 2: OMG(2); break;
+    case 3: OMG(3); break;
+    case 4: OMG(4); break;
+    case 5: OMG(5); break;
+    case 6: OMG(6); break;
+    case 7: OMG(7); break;
+    case 8: OMG(8); break;
+    case 9: OMG(9); break;
+    default: OMG(10); break;
+  }
+#undef OMG
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  omg2_kernel<<<grid, 256, smem, s>>>(ne, np, nrows, rows_per_cta, DAE, DBE,
-                                      DP, g2, fae_part, vrow);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  const int nout = 2 * ne * ne + np * np;
-  omg2_reduce<<<(nout + 127) / 128, 128, 0, s>>>(ne, np, grid, fae_part, vrow,
-                                                 DBE, DP, FAE, FP, FBE, fp_tmp);
+  const int nout = 2 * n2 + np * np;
+  omg2_reduce<<<(nout + 3) / 4, 128, 0, s>>>(ne, np, grid, panels, fae_part, vrow, DBE, DP, FAE,
+                                             FP, FBE, fp_tmp);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   sum_vec_kernel<<<1, 256, 0, s>>>(np * np, fp_tmp, E);
