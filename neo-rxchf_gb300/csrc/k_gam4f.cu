@@ -146,57 +146,84 @@ __device__ __forceinline__ double sig_coef(int k) {
   return k == 0 ? 0.5 : (k == 1 ? -0.25 : (k == 2 ? 0.125 : -0.0625));
 }
 
-// blockIdx.y = 0: Wp = dE/dG' from (E', PT_E, ST_E);
-// blockIdx.y = 1: Vp = dE/dE' from (G', PT_G, ST_G).
-__global__ void gam4f_grad_kernel(int n, const double* __restrict__ Ep,
-                                  const double* __restrict__ Gp,
-                                  const double* __restrict__ PT,
-                                  const double* __restrict__ ST,
-                                  double* __restrict__ Wp,
-                                  double* __restrict__ Vp) {
-  const int which = blockIdx.y;
-  const double* T = which ? Gp : Ep;                       // the other tensor
+// dE/d(the tensor on slots 0, 1) at legs l, from the other tensor T, its leg-pair
+// traces P and its double traces S (sig_code's table)
+__device__ __forceinline__ double grad_term(int n, const int* l, const double* __restrict__ T,
+                                            const double* __restrict__ P, const double* S) {
+  double acc = 0.0;
+#pragma unroll
+  for (int t = 0; t < 24; t++) {
+    const int code = sig_code(t);
+    const int dm = (code >> 2) & 15;
+    if ((dm & 1) && l[0] != l[1]) continue;
+    if ((dm & 2) && l[2] != l[3]) continue;
+    if ((dm & 4) && l[0] != l[3]) continue;
+    if ((dm & 8) && l[1] != l[2]) continue;
+    const int kind = (code >> 6) & 3, tid = (code >> 8) & 7;
+    const int s0 = (code >> 11) & 7, s1 = (code >> 14) & 7,
+              s2 = (code >> 17) & 7, s3 = (code >> 20) & 7;
+    double v;
+    if (kind == 0) {
+      v = __ldg(T + idx4(n, l[s0], l[s1], l[s2], l[s3]));
+    } else if (kind == 1) {
+      int uv[2], q = 0;
+      if (s0 != 7) uv[q++] = l[s0];
+      if (s1 != 7) uv[q++] = l[s1];
+      if (s2 != 7) uv[q++] = l[s2];
+      if (s3 != 7) uv[q++] = l[s3];
+      v = __ldg(P + ((size_t)tid * n + uv[0]) * n + uv[1]);
+    } else {
+      v = S[tid];
+    }
+    acc = fma(sig_coef(code & 3), v, acc);
+  }
+  return acc;
+}
+
+// Tensor-core build, Wp = dE/dG' from (E', PT_E, ST_E) and Vp = dE/dE' from (G',
+// PT_G, ST_G), in two kernels: off every delta an element is four gathers and
+// four FMAs; the 4 n^3 elements on a delta are done over by gam4f_delta_kernel.
+// (In one kernel the rare delta terms, up to twenty of them one lane at a time,
+// filled the FP64 pipe of whole warps: n = 48, 472 us; 146 us so.)
+// grid (n, ceil(n/4), 2 * kGradSplit): a CTA owns (x, four consecutive a, a
+// share of c), a thread (a, y): two of the gathers read the four a of one
+// 32-byte sector in one request, the other two the four c of one.
+constexpr int kGradSplit = 4;
+__global__ void __launch_bounds__(256)
+gam4f_gather_kernel(int n, const double* __restrict__ Ep, const double* __restrict__ Gp,
+                    double* __restrict__ Wp, double* __restrict__ Vp) {
+  const int which = blockIdx.z / kGradSplit, part = blockIdx.z % kGradSplit;
+  const double* T = which ? Gp : Ep;   // the other tensor
+  double* out = which ? Vp : Wp;
+  const int x = blockIdx.x, a = blockIdx.y * 4 + (threadIdx.x & 3), y = threadIdx.x >> 2;
+  if (a >= n || y >= n) return;
+  const int nb = (n + 3) / 4, c1 = min(n, nb * (part + 1) / kGradSplit * 4);
+#pragma unroll 4
+  for (int c = nb * part / kGradSplit * 4; c < c1; c++) {
+    double acc = 0.125 * __ldg(T + idx4(n, x, a, y, c));   // grad_term's order
+    acc = fma(-0.0625, __ldg(T + idx4(n, x, c, y, a)), acc);
+    acc = fma(-0.0625, __ldg(T + idx4(n, y, a, x, c)), acc);
+    out[idx4(n, a, x, c, y)] = fma(0.125, __ldg(T + idx4(n, y, c, x, a)), acc);
+  }
+}
+
+// grid (x, 4 deltas, 2 tensors); an element on several deltas is written
+// with the same value by each
+__global__ void gam4f_delta_kernel(int n, const double* __restrict__ Ep,
+                                   const double* __restrict__ Gp, const double* __restrict__ PT,
+                                   const double* __restrict__ ST, double* __restrict__ Wp,
+                                   double* __restrict__ Vp) {
+  const int which = blockIdx.z, d = blockIdx.y;
+  const double* T = which ? Gp : Ep;
   const double* P = PT + (size_t)(which ? 0 : 1) * 6 * n * n;
   const double* S = ST + (which ? 0 : 4);
   double* out = which ? Vp : Wp;
-  const long long n4 = (long long)n * n * n * n;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < n4;
-       o += stride) {
-    int l[4];
-    long long r = o;
-    l[3] = (int)(r % n); r /= n;
-    l[2] = (int)(r % n); r /= n;
-    l[1] = (int)(r % n); r /= n;
-    l[0] = (int)r;
-    double acc = 0.0;
-#pragma unroll
-    for (int t = 0; t < 24; t++) {
-      const int code = sig_code(t);
-      const int dm = (code >> 2) & 15;
-      if ((dm & 1) && l[0] != l[1]) continue;
-      if ((dm & 2) && l[2] != l[3]) continue;
-      if ((dm & 4) && l[0] != l[3]) continue;
-      if ((dm & 8) && l[1] != l[2]) continue;
-      const int kind = (code >> 6) & 3, tid = (code >> 8) & 7;
-      const int s0 = (code >> 11) & 7, s1 = (code >> 14) & 7,
-                s2 = (code >> 17) & 7, s3 = (code >> 20) & 7;
-      double v;
-      if (kind == 0) {
-        v = T[idx4(n, l[s0], l[s1], l[s2], l[s3])];
-      } else if (kind == 1) {
-        int uv[2], q = 0;
-        if (s0 != 7) uv[q++] = l[s0];
-        if (s1 != 7) uv[q++] = l[s1];
-        if (s2 != 7) uv[q++] = l[s2];
-        if (s3 != 7) uv[q++] = l[s3];
-        v = P[((size_t)tid * n + uv[0]) * n + uv[1]];
-      } else {
-        v = S[tid];
-      }
-      acc = fma(sig_coef(code & 3), v, acc);
-    }
-    out[o] = acc;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n * n * n; t += gridDim.x * blockDim.x) {
+    const int u = t / (n * n), v = t / n % n, w = t % n;
+    // legs (0,1), (2,3), (0,3), (1,2) equal
+    const int l[4] = {u, d == 0 ? u : v, d == 1 ? w : (d == 3 ? v : (d == 0 ? v : w)),
+                      d == 2 ? u : w};
+    out[idx4(n, l[0], l[1], l[2], l[3])] = grad_term(n, l, T, P, S);
   }
 }
 
@@ -218,21 +245,25 @@ __device__ __forceinline__ double block_sum(double v, double* sw) {
   return t;   // valid in thread 0
 }
 
-// One CTA: fockp(ip,jp) (+)= sum_chunk part; E = sum_p DP(p) * (new part).
-__global__ void fockp_reduce_kernel(int np, int nchunk,
-                                    const double* __restrict__ part,
-                                    const double* __restrict__ DP,
-                                    int accumulate, double* __restrict__ fockp,
-                                    double* __restrict__ E) {
+// One CTA, a warp per p: fockp(ip,jp) (+)= sum_chunk part; E = sum_p DP(p) *
+// (new part).
+__global__ void __launch_bounds__(1024)
+fockp_reduce_kernel(int np, int nchunk, const double* __restrict__ part,
+                    const double* __restrict__ DP, int accumulate,
+                    double* __restrict__ fockp, double* __restrict__ E) {
   __shared__ double sw[32];
+  const int lane = threadIdx.x & 31;
   double e = 0.0;
-  for (int p = threadIdx.x; p < np * np; p += blockDim.x) {
+  for (int p = threadIdx.x >> 5; p < np * np; p += 32) {
     double s = 0.0;
-    for (int c = 0; c < nchunk; c++) s += part[(long long)p * nchunk + c];
-    const int ip = p / np, jp = p - ip * np;
-    const int f = ip + np * jp;                  // column-major fockp(ip,jp)
-    fockp[f] = accumulate ? fockp[f] + s : s;
-    e = fma(DP[f], s, e);
+    for (int c = lane; c < nchunk; c += 32) s += part[(long long)p * nchunk + c];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+      const int ip = p / np, jp = p - ip * np;
+      const int f = ip + np * jp;                  // column-major fockp(ip,jp)
+      fockp[f] = accumulate ? fockp[f] + s : s;
+      e = fma(DP[f], s, e);
+    }
   }
   const double t = block_sum(e, sw);
   if (threadIdx.x == 0) *E = t;
@@ -264,9 +295,11 @@ __global__ void dp_contract_mixed_kernel(long long n4, int np, const double* __r
       sdp[p] = tc::narrow_f64(DP[ip + np * jp]);
     }
   __syncthreads();
-  const long long stride = (long long)gridDim.x * blockDim.x;
   const long long nv = (n4 & 1) ? n4 : n4 / 2;
-  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nv; v += stride) {
+  // one item a thread: a grid-strided loop of four and a quarter rounds left
+  // the last one three quarters empty
+  const long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (v < nv) {
     double acc0 = 0.0, acc1 = 0.0;
     for (int p0 = 0; p0 < np2; p0 += kMixChunk) {
       const int p1 = p0 + kMixChunk < np2 ? p0 + kMixChunk : np2;
@@ -278,7 +311,7 @@ __global__ void dp_contract_mixed_kernel(long long n4, int np, const double* __r
           a0 = fmaf(d, tc::narrow_f64(__ldcs(g2s + (long long)p * n4 + v)), a0);
         }
       } else {
-#pragma unroll 8
+#pragma unroll 16
         for (int p = p0; p < p1; p++) {
           const float d = staged ? sdp[p] : tc::narrow_f64(DP[(p / np) + np * (p % np)]);
           const double2 g = __ldcs(reinterpret_cast<const double2*>(g2s + (long long)p * n4) + v);
@@ -313,7 +346,7 @@ __global__ void narrow_kernel(long long n, const double* __restrict__ in,
 // A CTA takes kDotP consecutive p (grid (nchunk, ceil(np^2 / kDotP))) so
 // that each Wf element it loads serves kDotP products.
 static_assert(kDotChunk / kDotTB == kMixChunk, "one FP32 partial sum per thread");
-constexpr int kDotP = 2;
+constexpr int kDotP = 2, kDotBatch = 8;
 __global__ void __launch_bounds__(kDotTB)
 fockp_dot_mixed_kernel(long long n4, int nchunk, int np2,
                        const double* __restrict__ g2s,
@@ -327,11 +360,32 @@ fockp_dot_mixed_kernel(long long n4, int nchunk, int np2,
   float a[kDotP];
 #pragma unroll
   for (int j = 0; j < kDotP; j++) a[j] = 0.0f;
-  for (long long r = base + threadIdx.x; r < end; r += blockDim.x) {
-    const float w = __ldg(Wf + r);
+  if (pn == kDotP && end - base == kDotChunk) {
+    // whole chunks: kDotBatch steps' loads in flight before the first product
+    const double* g = g2s + (long long)p0 * n4 + base + threadIdx.x;
+    const float* w = Wf + base + threadIdx.x;
+#pragma unroll 1
+    for (int k = 0; k < kMixChunk; k += kDotBatch) {
+      double x[kDotP][kDotBatch];
+      float v[kDotBatch];
 #pragma unroll
-    for (int j = 0; j < kDotP; j++)
-      if (j < pn) a[j] = fmaf(tc::narrow_f64(__ldcs(g2s + (long long)(p0 + j) * n4 + r)), w, a[j]);
+      for (int q = 0; q < kDotBatch; q++) {
+#pragma unroll
+        for (int j = 0; j < kDotP; j++) x[j][q] = __ldcs(g + j * n4 + (k + q) * kDotTB);
+        v[q] = __ldg(w + (k + q) * kDotTB);
+      }
+#pragma unroll
+      for (int q = 0; q < kDotBatch; q++)
+#pragma unroll
+        for (int j = 0; j < kDotP; j++) a[j] = fmaf(tc::narrow_f64(x[j][q]), v[q], a[j]);
+    }
+  } else {
+    for (long long r = base + threadIdx.x; r < end; r += kDotTB) {
+      const float w = __ldg(Wf + r);
+#pragma unroll
+      for (int j = 0; j < kDotP; j++)
+        if (j < pn) a[j] = fmaf(tc::narrow_f64(__ldcs(g2s + (long long)(p0 + j) * n4 + r)), w, a[j]);
+    }
   }
   // kDotP block sums in FP64: warp shuffles, then one warp over the warps
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -450,38 +504,12 @@ gam4f_forward_kernel(int n, int np, const double* __restrict__ gee,
   }
 }
 
-// dE/d(the tensor on slots 0, 1) at legs l, from the other tensor T, its leg-pair
-// traces P and its double traces S (sig_code's table)
-__device__ __forceinline__ double grad_term(int n, const int* l, const double* __restrict__ T,
-                                            const double* __restrict__ P, const double* S) {
-  double acc = 0.0;
-#pragma unroll
-  for (int t = 0; t < 24; t++) {
-    const int code = sig_code(t);
-    const int dm = (code >> 2) & 15;
-    if ((dm & 1) && l[0] != l[1]) continue;
-    if ((dm & 2) && l[2] != l[3]) continue;
-    if ((dm & 4) && l[0] != l[3]) continue;
-    if ((dm & 8) && l[1] != l[2]) continue;
-    const int kind = (code >> 6) & 3, tid = (code >> 8) & 7;
-    const int s0 = (code >> 11) & 7, s1 = (code >> 14) & 7,
-              s2 = (code >> 17) & 7, s3 = (code >> 20) & 7;
-    double v;
-    if (kind == 0) {
-      v = __ldg(T + idx4(n, l[s0], l[s1], l[s2], l[s3]));
-    } else if (kind == 1) {
-      int uv[2], q = 0;
-      if (s0 != 7) uv[q++] = l[s0];
-      if (s1 != 7) uv[q++] = l[s1];
-      if (s2 != 7) uv[q++] = l[s2];
-      if (s3 != 7) uv[q++] = l[s3];
-      v = __ldg(P + ((size_t)tid * n + uv[0]) * n + uv[1]);
-    } else {
-      v = S[tid];
-    }
-    acc = fma(sig_coef(code & 3), v, acc);
-  }
-  return acc;
+// Off every delta only its four gathers are left (terms 16, 17, 22, 23).
+__device__ __forceinline__ double grad_gather(int n, const int* l, const double* __restrict__ T) {
+  double acc = 0.125 * __ldg(T + idx4(n, l[1], l[0], l[3], l[2]));
+  acc = fma(-0.0625, __ldg(T + idx4(n, l[1], l[2], l[3], l[0])), acc);
+  acc = fma(-0.0625, __ldg(T + idx4(n, l[3], l[0], l[1], l[2])), acc);
+  return fma(0.125, __ldg(T + idx4(n, l[3], l[2], l[1], l[0])), acc);
 }
 
 // Sums of v[0..3] over the warp: lane's result is that of v[(lane >> 3) & 3]
@@ -540,6 +568,18 @@ gam4f_backward_kernel(int n, int np, const double* __restrict__ g2s,
   __syncthreads();
   for (int e = threadIdx.x; e < n2; e += blockDim.x) {
     const int x = e / n, y = e - x * n;
+    const int l[4] = {a, x, c, y}, m[4] = {c, y, a, x};
+    const double w = grad_gather(n, l, Ep);
+    sW[x * ld + y] = w;
+    sX[x * ld + y] = w + grad_gather(n, m, Ep);
+    sY[x * ld + y] = grad_gather(n, l, Gp) + grad_gather(n, m, Gp);
+  }
+  __syncthreads();
+  // the rows x = a, x = c and columns y = a, y = c lie on deltas (a lane with
+  // delta terms in the loop above would hold up its whole warp)
+  for (int e = threadIdx.x; e < 4 * n; e += blockDim.x) {
+    const int k = e / n, u = e - k * n, q = (k & 1) ? c : a;
+    const int x = k < 2 ? q : u, y = k < 2 ? u : q;
     const int l[4] = {a, x, c, y}, m[4] = {c, y, a, x};
     const double w = grad_term(n, l, Ep, PE, sST + 4);
     sW[x * ld + y] = w;
@@ -690,13 +730,80 @@ __global__ void flush_copy_kernel(long long n, const double* __restrict__ in,
 }
 
 // ---- mixed-precision variant: the transforms and focke on tensor cores -----
-// C[m*ldc + n] = alpha sum_{k in split} A[m*lda + k] B[n*ldb + k]
+// Rows [0, rows) x K [kt, kt + 64) of an operand into its two TF32 halves in
+// the canonical layout, by warps [w0, nw) of the CTA: a warp takes 8 rows x 8
+// k, a lane two neighbouring k, so that its two 8-byte stores per half fill
+// whole 128-byte core matrices (a lane per k hit four banks eight times over)
+// and eight such loads are in flight before the first is converted.  VEC: the
+// pairs are 16-byte aligned.
+template <bool VEC>
+__device__ __forceinline__ void tc_load(const double* __restrict__ X, long long ld, long long x0,
+                                        int rows, long long kt, int kv, unsigned char* hi,
+                                        unsigned char* lo) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int nw = tc::kThreads / 32, kBatch = 8;
+  const int kh = (kv + 7) / 8, nt = ((rows + 7) / 8) * kh;
+  const int r = (lane >> 1) & 7, k = ((lane >> 4) << 2) + ((lane & 1) << 1);
+  for (int t0 = warp; t0 < nt; t0 += nw * kBatch) {
+    double2 v[kBatch];
+#pragma unroll
+    for (int q = 0; q < kBatch; q++) {
+      const int t = t0 + q * nw;
+      v[q] = make_double2(0.0, 0.0);
+      if (t < nt) {
+        const int rr = (t / kh) * 8 + r, kk = (t % kh) * 8 + k;
+        const double* p = X + (x0 + rr) * ld + kt + kk;
+        if (rr < rows) {
+          if (VEC && kk + 1 < kv) {
+            v[q] = __ldg(reinterpret_cast<const double2*>(p));
+          } else {
+            if (kk < kv) v[q].x = __ldg(p);
+            if (kk + 1 < kv) v[q].y = __ldg(p + 1);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kBatch; q++) {
+      const int t = t0 + q * nw;
+      if (t < nt) {
+        uint2 h, l;
+        tc::split_tf32(v[q].x, h.x, l.x);
+        tc::split_tf32(v[q].y, h.y, l.y);
+        const int off = tc::canon_off((t / kh) * 8 + r, (t % kh) * 8 + k);
+        *reinterpret_cast<uint2*>(hi + off) = h;
+        *reinterpret_cast<uint2*>(lo + off) = l;
+      }
+    }
+  }
+}
+
+// 2^ea v in FP64 by integer operations, for normal numbers and zeros: their
+// fields move over.  (A conversion, an addition and a multiplication per
+// result, all on the FP64 pipe, were a transform's largest part.)
+__device__ __forceinline__ double widen(float v, int ea) {
+  const uint32_t u = __float_as_uint(v), e = (u >> 23) & 255u;
+  const uint32_t hi = (u & 0x80000000u) | (e == 0u ? 0u : (((e + 896u + (uint32_t)ea) << 20) | ((u & 0x7fffffu) >> 3)));
+  return __hiloint2double((int)hi, (int)(u << 29));
+}
+// subnormal, infinite or NaN: what widen does not carry over
+__device__ __forceinline__ bool not_plain(float v) {
+  const uint32_t u = __float_as_uint(v) & 0x7fffffffu;
+  return u - 0x00800000u >= 0x7f000000u && u != 0u;
+}
+
+// C[m*ldc + n] = 2^ea sum_{k in split} A[m*lda + k] B[n*ldb + k]
 // grid (ceil(M/128), ceil(N/64), nsplit); split z covers K range
 // [z*kchunk, min(K, (z+1)*kchunk)) and writes C + z*split_stride.
-__global__ void __launch_bounds__(tc::kThreads, 1)
+// Rows past M or N are not loaded (their results are not stored), K steps past
+// the end not multiplied; a K tail inside a step is zero.
+// Measured at n = 48 (M = 110592, N = K = 48): 257 us a call with 128 threads
+// loading one element at a time and converting on the FP64 pipe, 65 us so.
+template <bool VEC>
+__global__ void __launch_bounds__(tc::kThreads, 2)
 tc_gemm_kernel(const double* __restrict__ A, long long lda, long long M,
                const double* __restrict__ B, long long ldb, long long N, long long K,
-               long long kchunk, double alpha, double* __restrict__ C, long long ldc,
+               long long kchunk, int ea, double* __restrict__ C, long long ldc,
                long long split_stride, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char tc_sm[];
   unsigned char* a_hi = tc_sm;
@@ -708,6 +815,8 @@ tc_gemm_kernel(const double* __restrict__ A, long long lda, long long M,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const long long m0 = (long long)blockIdx.x * tc::kTileM;
   const long long n0 = (long long)blockIdx.y * tc::kTileN;
+  const int mv = (int)(M - m0 < tc::kTileM ? M - m0 : tc::kTileM);
+  const int nv = (int)(N - n0 < tc::kTileN ? N - n0 : tc::kTileN);
   const long long kbeg = (long long)blockIdx.z * kchunk;
   const long long kend = kbeg + kchunk < K ? kbeg + kchunk : K;
   if (warp == 0) {
@@ -719,6 +828,10 @@ tc_gemm_kernel(const double* __restrict__ A, long long lda, long long M,
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(tc::smem_u32(mbar))
                  : "memory");
   }
+  // rows that are never loaded are multiplied all the same: give them a value
+  if (mv < tc::kTileM || nv < tc::kTileN)
+    for (int e = tid * 16; e < 2 * (tc::kABytes + tc::kBBytes); e += tc::kThreads * 16)
+      *reinterpret_cast<uint4*>(tc_sm + e) = make_uint4(0u, 0u, 0u, 0u);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -727,43 +840,32 @@ tc_gemm_kernel(const double* __restrict__ A, long long lda, long long M,
   uint32_t phase = 0;
   bool ok = true;
   const uint32_t idesc = tc::instr_desc();
-  // kFoldTiles 64-wide K tiles are accumulated in TMEM (FP32) and then
-  // folded into this thread's FP64 row of the result
-  double acc[tc::kTileN];
+  // kFoldTiles 64-wide K tiles are accumulated in TMEM (FP32) and then folded
+  // into FP64: this thread's half row of the result (a warp reads the 32
+  // tensor-memory lanes of its number modulo four)
+  constexpr int kHalf = tc::kTileN / 2;
+  const int half = warp >> 2, rloc = (warp & 3) * 32 + lane;
+  const bool used = (warp & 3) * 32 < mv && half * kHalf < nv;   // any result of this warp stored
+  const bool one = kend - kbeg <= tc::kTileK * tc::kFoldTiles;   // a single fold
+  const double scale = ldexp(1.0, ea);
+  double acc[kHalf];
 #pragma unroll
-  for (int i = 0; i < tc::kTileN; i++) acc[i] = 0.0;
-  const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
+  for (int i = 0; i < kHalf; i++) acc[i] = 0.0;
+  const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(half * kHalf);
   int tile = 0;
   for (long long kt = kbeg; kt < kend && ok; kt += tc::kTileK, tile++) {
     const bool first = tile % tc::kFoldTiles == 0;
     const bool fold = (tile + 1) % tc::kFoldTiles == 0 || kt + tc::kTileK >= kend;
-    for (int e = tid; e < tc::kTileM * tc::kTileK; e += tc::kThreads) {
-      const int r = e / tc::kTileK, k = e - r * tc::kTileK;
-      const long long gm = m0 + r, gk = kt + k;
-      const double v = (gm < M && gk < kend) ? A[gm * lda + gk] : 0.0;
-      uint32_t hi, lo;
-      tc::split_tf32(v, hi, lo);
-      const int off = tc::canon_off(r, k);
-      *reinterpret_cast<uint32_t*>(a_hi + off) = hi;
-      *reinterpret_cast<uint32_t*>(a_lo + off) = lo;
-    }
-    for (int e = tid; e < tc::kTileN * tc::kTileK; e += tc::kThreads) {
-      const int r = e / tc::kTileK, k = e - r * tc::kTileK;
-      const long long gn = n0 + r, gk = kt + k;
-      const double v = (gn < N && gk < kend) ? B[gn * ldb + gk] : 0.0;
-      uint32_t hi, lo;
-      tc::split_tf32(v, hi, lo);
-      const int off = tc::canon_off(r, k);
-      *reinterpret_cast<uint32_t*>(b_hi + off) = hi;
-      *reinterpret_cast<uint32_t*>(b_lo + off) = lo;
-    }
+    const int kv = (int)(kend - kt < tc::kTileK ? kend - kt : tc::kTileK);
+    tc_load<VEC>(A, lda, m0, mv, kt, kv, a_hi, a_lo);
+    tc_load<VEC>(B, ldb, n0, nv, kt, kv, b_hi, b_lo);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t ah = tc::smem_u32(a_hi), al = tc::smem_u32(a_lo);
       const uint32_t bh = tc::smem_u32(b_hi), bl = tc::smem_u32(b_lo);
-      for (int st = 0; st < tc::kTileK / 8; st++) {
+      for (int st = 0; st < (kv + 7) / 8; st++) {
         const uint32_t o = st * 256;   // two 128-byte core matrices per K step
         tc::mma_tf32(tmem, tc::smem_desc(ah + o), tc::smem_desc(bh + o), idesc,
                      (st > 0 || !first) ? 1 : 0);
@@ -775,13 +877,22 @@ tc_gemm_kernel(const double* __restrict__ A, long long lda, long long M,
     ok = __syncthreads_and(tc::mbar_wait(mb, phase) ? 1 : 0) != 0;
     phase ^= 1u;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ok && fold) {
+    if (ok && fold && used) {
 #pragma unroll
-      for (int c = 0; c < tc::kTileN / 16; c++) {
+      for (int c = 0; c < kHalf / 16; c++) {
         float v[16];
         tc::tmem_ld16(trow + (uint32_t)(c * 16), v);
+        bool odd = !one;
 #pragma unroll
-        for (int i = 0; i < 16; i++) acc[c * 16 + i] += (double)v[i];
+        for (int i = 0; i < 16; i++) odd = odd || not_plain(v[i]);
+        if (__any_sync(0xffffffffu, odd)) {
+          const double f = one ? scale : 1.0;
+#pragma unroll
+          for (int i = 0; i < 16; i++) acc[c * 16 + i] = fma((double)v[i], f, acc[c * 16 + i]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; i++) acc[c * 16 + i] = widen(v[i], ea);
+        }
       }
     }
     // every lane's reads are done before the next tile's MMA overwrites TMEM
@@ -795,15 +906,14 @@ tc_gemm_kernel(const double* __restrict__ A, long long lda, long long M,
     // stage the 128 x 64 FP64 tile in their shared memory (row stride 65)
     // and write it row-segment by row-segment, coalesced
     double* sc = reinterpret_cast<double*>(tc_sm);
-    const int rloc = warp * 32 + lane;
 #pragma unroll
-    for (int i = 0; i < tc::kTileN; i++) sc[rloc * (tc::kTileN + 1) + i] = alpha * acc[i];
+    for (int i = 0; i < kHalf; i++)
+      sc[rloc * (tc::kTileN + 1) + half * kHalf + i] = one ? acc[i] : scale * acc[i];
     __syncthreads();
     double* out = C + (long long)blockIdx.z * split_stride;
-    for (int e = tid; e < tc::kTileM * tc::kTileN; e += tc::kThreads) {
-      const int r = e / tc::kTileN, c = e - r * tc::kTileN;
-      const long long row = m0 + r, n = n0 + c;
-      if (row < M && n < N) out[row * ldc + n] = sc[r * (tc::kTileN + 1) + c];
+    for (int e = tid; e < mv * nv; e += tc::kThreads) {
+      const int r = e / nv, c = e - r * nv;
+      out[(m0 + r) * ldc + n0 + c] = sc[r * (tc::kTileN + 1) + c];
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -854,33 +964,39 @@ __global__ void transpose_n_kernel(int n, const double* __restrict__ DE, double*
   }
 }
 
-// focke(x,b) (+)= sum_split part[split][x*64 + b]
+// focke(x,b) (+)= sum_split part[split][x*64 + b], a warp per output
 __global__ void focke_tc_reduce_kernel(int n, int nsplit, const double* __restrict__ part,
                                        int accumulate, double* __restrict__ focke) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * n; e += gridDim.x * blockDim.x) {
-    const int x = e / n, b = e - x * n;
-    double s = 0.0;
-    for (int z = 0; z < nsplit; z++) s += part[(long long)z * 128 * 64 + x * 64 + b];
+  const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (e >= n * n) return;
+  const int x = e / n, b = e - x * n;
+  double s = 0.0;
+  for (int z = lane; z < nsplit; z += 32) s += part[(long long)z * 128 * 64 + x * 64 + b];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0) {
     const int f = x + n * b;
     focke[f] = accumulate ? focke[f] + s : s;
   }
 }
 
-constexpr long long kFockeKChunk = 1024;
+// Two 256-wide FP32 folds a CTA: enough of them for the SMs at n = 48 (216)
+constexpr long long kFockeKChunk = 512;
 
 cudaError_t tc_gemm(const double* A, long long lda, long long M, const double* B,
-                    long long ldb, long long N, long long K, long long kchunk, double alpha,
+                    long long ldb, long long N, long long K, long long kchunk, int ea,
                     double* C, long long ldc, long long split_stride, int* err,
                     cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(tc_gemm_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const bool vec = !(lda & 1) && !(ldb & 1) && !(kchunk & 1) &&
+                   !((uintptr_t)A & 15) && !((uintptr_t)B & 15);
+  const auto fn = vec ? tc_gemm_kernel<true> : tc_gemm_kernel<false>;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        tc::kSmemBytes);
   if (e != cudaSuccess) return e;
   const long long nsplit = (K + kchunk - 1) / kchunk;
   const dim3 grid((unsigned)((M + tc::kTileM - 1) / tc::kTileM),
                   (unsigned)((N + tc::kTileN - 1) / tc::kTileN), (unsigned)(nsplit < 1 ? 1 : nsplit));
-  tc_gemm_kernel<<<grid, tc::kThreads, tc::kSmemBytes, s>>>(A, lda, M, B, ldb, N, K, kchunk,
-                                                           alpha, C, ldc, split_stride, err);
+  fn<<<grid, tc::kThreads, tc::kSmemBytes, s>>>(A, lda, M, B, ldb, N, K, kchunk, ea, C, ldc,
+                                               split_stride, err);
   return cudaGetLastError();
 }
 
@@ -991,14 +1107,15 @@ cudaError_t launch_gam4_factored_tc(int ne, int np, const double* gee,
   transpose_n_kernel<<<grid_for(n2, TB), TB, 0, s>>>(n, DE, DEt);
   // last-index transforms: T'(..,y) = sum_d T(..,d) DE(y,d)  [B = DE^T rows]
   auto last_f = [&](const double* in, double* out) {
-    return tc_gemm(in, n, n3, DEt, n, n, n, n, 1.0, out, n, 0, err, s);
+    return tc_gemm(in, n, n3, DEt, n, n, n, n, 0, out, n, 0, err, s);
   };
   // back transforms: T'(..,d) = sum_y T(..,y) DE(y,d)  [B = DE rows]
-  auto last_b = [&](const double* in, double* out, double alpha) {
-    return tc_gemm(in, n, n3, DE, n, n, n, n, alpha, out, n, 0, err, s);
+  auto last_b = [&](const double* in, double* out, int ea) {
+    return tc_gemm(in, n, n3, DE, n, n, n, n, ea, out, n, 0, err, s);
   };
   // 1. G = DP . GAM_2s (FP32 products, HBM)
-  dp_contract_mixed_kernel<<<g_n4, 256, np * np <= kDpShared ? sizeof(float) * np * np : 0, s>>>(
+  const long long nv = (n4 & 1) ? n4 : n4 / 2;
+  dp_contract_mixed_kernel<<<(unsigned)((nv + 255) / 256), 256, np * np <= kDpShared ? sizeof(float) * np * np : 0, s>>>(
       n4, np, g2s, DP, buf[0]);
   // 2. H_G, G' and H_E, E'
   TRY(last_f(buf[0], buf[1]));                                        // H_G
@@ -1011,28 +1128,29 @@ cudaError_t launch_gam4_factored_tc(int ne, int np, const double* gee,
   // 3-4. traces and gradients (FP64)
   traces_kernel<<<dim3(grid_for(6LL * n * n, TB), 2), TB, 0, s>>>(n, buf[3], buf[5], PT);
   dtraces_kernel<<<1, 64, 0, s>>>(n, PT, ST);
-  gam4f_grad_kernel<<<dim3(g_n4, 2), TB, 0, s>>>(n, buf[5], buf[3], PT, ST, buf[6], buf[7]);
+  gam4f_gather_kernel<<<dim3(n, (n + 3) / 4, 2 * kGradSplit), 4 * n, 0, s>>>(n, buf[5], buf[3], buf[6], buf[7]);
+  gam4f_delta_kernel<<<dim3((unsigned)((n3 + 127) / 128), 4, 2), 128, 0, s>>>(n, buf[5], buf[3], PT, ST, buf[6], buf[7]);
   // Ws = Wp + Wp^swap, Vs = Vp + Vp^swap
   pair_swap_kernel<<<tgrid, tblk, 0, s>>>((int)n2, buf[6], 1.0, buf[0]);
   pair_swap_kernel<<<tgrid, tblk, 0, s>>>((int)n2, buf[7], 1.0, buf[2]);
   // 5. W = back(Ws / 2), fockp = <GAM_2s, W>, E
-  TRY(last_b(buf[0], buf[3], 0.5));
+  TRY(last_b(buf[0], buf[3], -1));
   pair_swap_kernel<<<tgrid, tblk, 0, s>>>((int)n2, buf[3], 0.0, buf[5]);
-  TRY(last_b(buf[5], buf[6], 1.0));                                   // W
+  TRY(last_b(buf[5], buf[6], 0));                                   // W
   float* Wf = reinterpret_cast<float*>(buf[7]);   // free until swap12 below
   narrow_kernel<<<g_n4, TB, 0, s>>>(n4, buf[6], Wf);
   fockp_dot_mixed_kernel<<<dim3(nchunk, (np * np + kDotP - 1) / kDotP), kDotTB, 0, s>>>(
       n4, nchunk, np * np, g2s, Wf, fpart);
-  fockp_reduce_kernel<<<1, 256, 0, s>>>(np, nchunk, fpart, DP, accumulate, fockp, E);
+  fockp_reduce_kernel<<<1, 1024, 0, s>>>(np, nchunk, fpart, DP, accumulate, fockp, E);
   // 6. focke(x,b) = sum_{a,c,y} Ws(a,x,c,y) H_G(a,b,c,y) + Vs(a,x,c,y) H_E(a,b,c,y)
   swap12_kernel<<<g_n4, TB, 0, s>>>(n, buf[0], buf[3]);   // Ws  -> [x][a][c][y]
   swap12_kernel<<<g_n4, TB, 0, s>>>(n, buf[1], buf[5]);   // H_G -> [b][a][c][y]
   swap12_kernel<<<g_n4, TB, 0, s>>>(n, buf[2], buf[7]);   // Vs
   swap12_kernel<<<g_n4, TB, 0, s>>>(n, buf[4], buf[1]);   // H_E
-  TRY(tc_gemm(buf[3], n3, n, buf[5], n3, n, n3, kFockeKChunk, 1.0, epart, 64, 128 * 64, err, s));
-  TRY(tc_gemm(buf[7], n3, n, buf[1], n3, n, n3, kFockeKChunk, 1.0, epart + nsplit * 128 * 64,
+  TRY(tc_gemm(buf[3], n3, n, buf[5], n3, n, n3, kFockeKChunk, 0, epart, 64, 128 * 64, err, s));
+  TRY(tc_gemm(buf[7], n3, n, buf[1], n3, n, n3, kFockeKChunk, 0, epart + nsplit * 128 * 64,
               64, 128 * 64, err, s));
-  focke_tc_reduce_kernel<<<grid_for(n2, TB), TB, 0, s>>>(n, (int)(2 * nsplit), epart,
+  focke_tc_reduce_kernel<<<(unsigned)((n2 * 32 + TB - 1) / TB), TB, 0, s>>>(n, (int)(2 * nsplit), epart,
                                                         accumulate, focke);
 #undef TRY
   return cudaGetLastError();

@@ -4,7 +4,7 @@
 // ("3xTF32": a = a_hi + a_lo with a_hi = tf32(a), a_lo = tf32(a - a_hi);
 // a b ~ a_hi b_hi + a_hi b_lo + a_lo b_hi, ~2^-21 relative), and FP64 output.
 //
-// One CTA of 128 threads owns one 128-row tile of A and one 64-row tile of B
+// One CTA of 256 threads owns one 128-row tile of A and one 64-row tile of B
 // and loops over K in steps of 64 (the FP32 accumulator in tensor memory
 // is folded into FP64 registers every kFoldTiles tiles):
 //   * every thread loads FP64 elements, splits them and stores the TF32
@@ -18,10 +18,9 @@
 //     tcgen05.commit to an mbarrier;
 //   * every thread waits on the mbarrier (bounded: after kSpinLimit polls the
 //     kernel records an error flag instead of hanging);
-// and finally each warp reads its 32 accumulator lanes with tcgen05.ld and
-// the CTA writes the FP64 tile through shared memory, coalesced.  Tensor memory (64 columns) is allocated
-// and freed by warp 0.  Operand rows past M or N and K past the end read as
-// zero.
+// and finally each warp reads half the columns of its 32 accumulator lanes
+// (its number modulo four) with tcgen05.ld and the CTA writes the FP64 tile through shared memory, coalesced.  Tensor memory (64 columns) is allocated
+// and freed by warp 0.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -34,7 +33,7 @@ namespace tc {
 constexpr int kTileM = 128, kTileN = 64, kTileK = 64;
 // K tiles accumulated in tensor memory (FP32) between two FP64 folds
 constexpr int kFoldTiles = 4;
-constexpr int kThreads = 128;
+constexpr int kThreads = 256;
 constexpr long long kSpinLimit = 1LL << 26;
 
 // shared-memory bytes of one operand half: rows x 64 TF32 values
