@@ -68,6 +68,8 @@
 // grid drains through a device counter (gam3_fb_persistent); the per-block
 // arithmetic is that of gam3_fb_kernel, so each system's R4 is bit-identical
 // to its separate build.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <type_traits>
 #include <vector>
@@ -123,20 +125,42 @@ __global__ void g3_records_kernel(DevSystem S, double* __restrict__ rec, double*
 
 constexpr int kFbThreads = 128;   // threads (and bras per chunk) of a CTA
 constexpr int kFbShares = 4;      // shares of a chunk's bras that warps take
+constexpr int kFbMinPart = 16;    // fewest bras of a part
 
 __host__ __device__ __forceinline__ int nPe_of(int ne) { return ne * (ne + 1) / 2; }
+
+// Parts that the bras of a block are cut into, one CTA of a cluster each, for
+// systems with too few blocks to fill the chip: a block of contracted
+// functions has many times the bras of one of primitives, and the longest one
+// was the pass.  Measured (one GB300, a pass): examples/xchf (441 blocks of 9
+// to 729 bras) 2340 -> 500 (Vep) and 2310 -> 850 us (Vee); nebf = 4, npbf = 2 of
+// two primitives (300 blocks, FP32) 940 -> 670 and 800 -> 600 us.  From 152 x 16
+// blocks on the chip is full (4410 blocks: the build takes 1.55 ms with one
+// part, 2.93 with four), and with fewer than kFbMinPart bras a part the CTAs
+// are mostly empty (nebf = 6, npbf = 2 of one primitive, 9 bras: 1.07, 1.37 ms with eight).
+__host__ __device__ __forceinline__ int fb_parts(const DevSystem& S) {
+  const long long nPe = nPe_of(S.nebf);
+  const long long blocks = nPe * nPe * nPe_of(S.npbf) * S.g3_ntile;
+  const long long bras = (long long)S.g3_nket * S.g3_nket * S.ngtg * S.ngtg / (nPe * nPe);   // mean
+  int n = 1;
+  while (n < 8 && blocks * n < 152 * 16 && bras > n * kFbMinPart) n *= 2;
+  return n;
+}
 
 // One CTA's work: block blk (Pp, Pa, Pb) and ket tile `tile` of one pass.
 // MODE 0: G4Vep, (Pp, P1, P2), kets e3 -> R4[Pp][P1][P2][P3]  = -sum
 // MODE 1: G4Vee, (Pp, P1, P3), kets e2 -> R4[Pp][P1][P2][P3] += 2 sum
 //         (or = 2 sum when store1: the batched launch keeps the two passes
 //         in separate arrays and adds them afterwards).
-// Each element has one owner CTA per pass, so results are deterministic.
-template <bool F32, int LE, int LN, int MODE>
+// Each element has one owner CTA per pass, and the parts of its bras are added
+// in their order, so results are deterministic.  CLUSTER: the parts are the
+// CTAs of a cluster, and the first adds the others' sums from their shared
+// memory; otherwise one CTA takes one part after the other.
+template <bool F32, int LE, int LN, int MODE, bool CLUSTER>
 __device__ __forceinline__ void fb_block(const DevSystem& S, const double* __restrict__ erec,
                                          const double* __restrict__ prec, double screen,
                                          double* __restrict__ r4, long long blk, int tile,
-                                         unsigned char* smraw, bool store1) {
+                                         int nparts, unsigned char* smraw, bool store1) {
   using R = typename std::conditional<F32, float, double>::type;
   constexpr int NW = 4 * LE + 2 * LN;   // bra Hermite order per direction
   constexpr int NK = 2 * LE;            // ket Hermite order per direction
@@ -165,100 +189,122 @@ __device__ __forceinline__ void fb_block(const DevSystem& S, const double* __res
   const int kb = kofs[Pb], nb = kofs[Pb + 1] - kb;
   const int ng = S.ngtg;
   const int nbra = na * nb * ng * ng;
+  int plen = (nbra + nparts - 1) / nparts;   // bras of a part
+  if (plen < kFbMinPart) plen = kFbMinPart;
+  nparts = (nbra + plen - 1) / plen;
+  const int z0 = CLUSTER ? (int)blockIdx.z : 0;
+  if (z0 >= nparts) return;   // (the cluster's barriers count only CTAs that have not exited)
   const double* rp = prec + (size_t)kRLen * Pp;
   double wsum = 0.0;
   if (screen > 0.0)
     for (int k = 0; k < ng; k++)
       for (int l = 0; l < ng; l++) wsum += fabs(S.bgem[k] * S.bgem[l]);
 
-  // Lane sums of ket kk, one row per bra share: acc_s[share * nkt + kk]
+  // Lane sums of ket kk, one row per bra share: acc_s[share * nkt + kk];
+  // sums of the tile's electron pairs: tot
+  double* tot = acc_s + kFbShares * nkt;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ngrp = (nkt + 31) / 32;
-  for (int k = threadIdx.x; k < kFbShares * nkt; k += blockDim.x) acc_s[k] = 0.0;
-  for (int c0 = 0; c0 < nbra; c0 += kFbThreads) {
-    const int nvalid = nbra - c0 < kFbThreads ? nbra - c0 : kFbThreads;
-    __syncthreads();
-    if ((int)threadIdx.x < nvalid) {
-      int q = c0 + threadIdx.x;
-      const int l = q % ng; q /= ng;
-      const int k = q % ng; q /= ng;
-      const int ub = q % nb;
-      const int ua = q / nb;
-      const double* ra = erec + (size_t)kRLen * (ka + ua);
-      const double* rb = erec + (size_t)kRLen * (kb + ub);
-      Bra<R, NW> b;
-      if constexpr (MODE == 0)
-        build_bra_vep<R, LE, LN, NW>(ra, rb, rp, (R)S.ggem[k], (R)S.ggem[l], b);
-      else
-        build_bra_vee<R, LE, LN, NW>(ra, rb, rp, (R)S.ggem[k], (R)S.ggem[l], b);
-      if constexpr (!F32) finish_bra<NW>(b);
-      b.wgt = (MODE == 0 ? -1.0 : 2.0) * (S.bgem[k] * S.bgem[l]) * ra[kRC] * rb[kRC] *
-              rp[kRC];
-      // Vep: S1 S2 Qp (x Q3 of the ket); Vee: Q1 S3 Sp (x Q2 of the ket)
-      b.est = wsum * (MODE == 0 ? ra[kRS] * rb[kRS] * rp[kRQ]
-                                : 2.0 * ra[kRQ] * rb[kRS] * rp[kRS]);
-      bras[threadIdx.x] = b;
-    }
-    __syncthreads();
-    // Warps take (32 kets, share of the bras): with all the kets on the CTA's
-    // threads, a last round of few kets left most of its warps idle.
-    const int nsh = nvalid >= 16 ? kFbShares : (nvalid >= 8 ? 2 : 1);
-    for (int unit = warp; unit < ngrp * nsh; unit += kFbThreads / 32) {
-      const int grp = unit / nsh, sh = unit - grp * nsh;
-      const int i0 = nvalid * sh / nsh, i1 = nvalid * (sh + 1) / nsh;
-      const int kk = grp * 32 + lane;
-      if (kk >= nkt) continue;
-      const int kid = kperm[k0 + kk];
-      const double* rk = erec + (size_t)kRLen * kid;
-      const double qk = rk[kRQ];
-      const double rkc = rk[kRC];
-      double part = 0.0;
-      if constexpr (F32) {
-        const R pk = (R)rk[kRP];
-        R Xk[3], Ek[3][NK + 1];
-        int tk[3];
-        for (int d = 0; d < 3; d++) {
-          Xk[d] = (R)rk[kRX + d];
-          tk[d] = (int)rk[kRT + d];
-          for (int t = 0; t <= NK; t++)
-            Ek[d][t] = (t & 1) ? -(R)rk[kRE + 5 * d + t] : (R)rk[kRE + 5 * d + t];
-        }
-        for (int bi = i0; bi < i1; bi++) {
-          const Bra<R, NW>& b = bras[bi];
-          if (screen > 0.0 && b.est * qk < screen) continue;
-          double v = fb_eval<R, NW, NK>(b, pk, Xk, Ek, tk);
-          if (MODE == 0) v = underflow_bits(v);   // zz = underflow(G4_MD_xgVepg)
-          part += b.wgt * v;
-        }
-      } else {
-        Ket<NK> ket;
-        load_ket<NK>(rk, ket);
-        for (int bi = i0; bi < i1; bi++) {
-          const Bra<R, NW>& b = bras[bi];
-          if (screen > 0.0 && b.est * qk < screen) continue;
-          double v = fb_value<NW, NK>(b, ket);
-          if (MODE == 0) v = underflow_bits(v);
-          part = fma(b.wgt, v, part);
-        }
+  for (int z = z0; z < (CLUSTER ? z0 + 1 : nparts); z++) {
+    if (z > z0) __syncthreads();   // the previous part's sums are taken
+    const int zend = (z + 1) * plen < nbra ? (z + 1) * plen : nbra;
+    for (int k = threadIdx.x; k < kFbShares * nkt; k += blockDim.x) acc_s[k] = 0.0;
+    for (int c0 = z * plen; c0 < zend; c0 += kFbThreads) {
+      const int nvalid = zend - c0 < kFbThreads ? zend - c0 : kFbThreads;
+      __syncthreads();
+      if ((int)threadIdx.x < nvalid) {
+        int q = c0 + threadIdx.x;
+        const int l = q % ng; q /= ng;
+        const int k = q % ng; q /= ng;
+        const int ub = q % nb;
+        const int ua = q / nb;
+        const double* ra = erec + (size_t)kRLen * (ka + ua);
+        const double* rb = erec + (size_t)kRLen * (kb + ub);
+        Bra<R, NW> b;
+        if constexpr (MODE == 0)
+          build_bra_vep<R, LE, LN, NW>(ra, rb, rp, (R)S.ggem[k], (R)S.ggem[l], b);
+        else
+          build_bra_vee<R, LE, LN, NW>(ra, rb, rp, (R)S.ggem[k], (R)S.ggem[l], b);
+        if constexpr (!F32) finish_bra<NW>(b);
+        b.wgt = (MODE == 0 ? -1.0 : 2.0) * (S.bgem[k] * S.bgem[l]) * ra[kRC] * rb[kRC] *
+                rp[kRC];
+        // Vep: S1 S2 Qp (x Q3 of the ket); Vee: Q1 S3 Sp (x Q2 of the ket)
+        b.est = wsum * (MODE == 0 ? ra[kRS] * rb[kRS] * rp[kRQ]
+                                  : 2.0 * ra[kRQ] * rb[kRS] * rp[kRS]);
+        bras[threadIdx.x] = b;
       }
-      acc_s[sh * nkt + kid - k0] += part * rkc;
+      __syncthreads();
+      // Warps take (32 kets, share of the bras): with all the kets on the CTA's
+      // threads, a last round of few kets left most of its warps idle.
+      const int nsh = nvalid >= 16 ? kFbShares : (nvalid >= 8 ? 2 : 1);
+      for (int unit = warp; unit < ngrp * nsh; unit += kFbThreads / 32) {
+        const int grp = unit / nsh, sh = unit - grp * nsh;
+        const int i0 = nvalid * sh / nsh, i1 = nvalid * (sh + 1) / nsh;
+        const int kk = grp * 32 + lane;
+        if (kk >= nkt) continue;
+        const int kid = kperm[k0 + kk];
+        const double* rk = erec + (size_t)kRLen * kid;
+        const double qk = rk[kRQ];
+        const double rkc = rk[kRC];
+        double part = 0.0;
+        if constexpr (F32) {
+          const R pk = (R)rk[kRP];
+          R Xk[3], Ek[3][NK + 1];
+          int tk[3];
+          for (int d = 0; d < 3; d++) {
+            Xk[d] = (R)rk[kRX + d];
+            tk[d] = (int)rk[kRT + d];
+            for (int t = 0; t <= NK; t++)
+              Ek[d][t] = (t & 1) ? -(R)rk[kRE + 5 * d + t] : (R)rk[kRE + 5 * d + t];
+          }
+          for (int bi = i0; bi < i1; bi++) {
+            const Bra<R, NW>& b = bras[bi];
+            if (screen > 0.0 && b.est * qk < screen) continue;
+            double v = fb_eval<R, NW, NK>(b, pk, Xk, Ek, tk);
+            if (MODE == 0) v = underflow_bits(v);   // zz = underflow(G4_MD_xgVepg)
+            part += b.wgt * v;
+          }
+        } else {
+          Ket<NK> ket;
+          load_ket<NK>(rk, ket);
+          for (int bi = i0; bi < i1; bi++) {
+            const Bra<R, NW>& b = bras[bi];
+            if (screen > 0.0 && b.est * qk < screen) continue;
+            double v = fb_value<NW, NK>(b, ket);
+            if (MODE == 0) v = underflow_bits(v);
+            part = fma(b.wgt, v, part);
+          }
+        }
+        acc_s[sh * nkt + kid - k0] += part * rkc;
+      }
+    }
+    __syncthreads();
+    for (int P = P0 + threadIdx.x; P < P1t; P += blockDim.x) {
+      double s = 0.0;
+      for (int sh = 0; sh < kFbShares; sh++)
+        for (int k = kofs[P]; k < kofs[P + 1]; k++) s += acc_s[sh * nkt + k - k0];
+      tot[P - P0] = z > z0 ? tot[P - P0] + s : s;
     }
   }
-  __syncthreads();
   const long long nP = nPe;
-  for (int P = P0 + threadIdx.x; P < P1t; P += blockDim.x) {
-    double s = 0.0;
-    for (int sh = 0; sh < kFbShares; sh++)
-      for (int k = kofs[P]; k < kofs[P + 1]; k++) s += acc_s[sh * nkt + k - k0];
-    if (MODE == 0) {
-      r4[((Pp * nP + Pa) * nP + Pb) * nP + P] = s;
-      if (kHalf && Pa != Pb) r4[((Pp * nP + Pb) * nP + Pa) * nP + P] = s;
-    } else if (store1) {
-      r4[((Pp * nP + Pa) * nP + P) * nP + Pb] = s;
-    } else {
-      r4[((Pp * nP + Pa) * nP + P) * nP + Pb] += s;
+  if (CLUSTER && nparts > 1) cooperative_groups::this_cluster().sync();
+  if (z0 == 0)
+    for (int P = P0 + threadIdx.x; P < P1t; P += blockDim.x) {
+      double s = tot[P - P0];
+      if (CLUSTER)
+        for (int z = 1; z < nparts; z++)
+          s += cooperative_groups::this_cluster().map_shared_rank(tot, z)[P - P0];
+      if (MODE == 0) {
+        r4[((Pp * nP + Pa) * nP + Pb) * nP + P] = s;
+        if (kHalf && Pa != Pb) r4[((Pp * nP + Pb) * nP + Pa) * nP + P] = s;
+      } else if (store1) {
+        r4[((Pp * nP + Pa) * nP + P) * nP + Pb] = s;
+      } else {
+        r4[((Pp * nP + Pa) * nP + P) * nP + Pb] += s;
+      }
     }
-  }
+  // the other parts' sums stay until they are read
+  if (CLUSTER && nparts > 1) cooperative_groups::this_cluster().sync();
 }
 
 template <bool F32, int LE, int LN, int MODE>
@@ -267,8 +313,8 @@ gam3_fb_kernel(DevSystem S, const double* __restrict__ erec,
                const double* __restrict__ prec, double screen,
                double* __restrict__ r4) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  fb_block<F32, LE, LN, MODE>(S, erec, prec, screen, r4, (long long)blockIdx.x, blockIdx.y,
-                              smraw, false);
+  fb_block<F32, LE, LN, MODE, true>(S, erec, prec, screen, r4, (long long)blockIdx.x, blockIdx.y,
+                                    (int)gridDim.z, smraw, false);
 }
 
 // ---- many systems in one persistent launch ----------------------------------
@@ -302,9 +348,11 @@ gam3_fb_persistent(const G3BatchSys* __restrict__ sys, const long long* __restri
       const int tile = (int)(local % b.S.g3_ntile);
       const long long blk = local / b.S.g3_ntile;
       if ((lo & 1) == 0)
-        fb_block<F32, LE, LN, 0>(b.S, b.erec, b.prec, screen, b.r4a, blk, tile, smraw, false);
+        fb_block<F32, LE, LN, 0, false>(b.S, b.erec, b.prec, screen, b.r4a, blk, tile,
+                                        fb_parts(b.S), smraw, false);
       else
-        fb_block<F32, LE, LN, 1>(b.S, b.erec, b.prec, screen, b.r4b, blk, tile, smraw, true);
+        fb_block<F32, LE, LN, 1, false>(b.S, b.erec, b.prec, screen, b.r4b, blk, tile,
+                                        fb_parts(b.S), smraw, true);
     }
   }
 }
@@ -354,7 +402,7 @@ __global__ void gam3_expand_kernel(int ne, int np, const double* __restrict__ au
 // kets: the most kets of a tile
 template <class R, int NW>
 size_t fb_smem(int kets) {
-  return sizeof(Bra<R, NW>) * kFbThreads + sizeof(double) * (size_t)kFbShares * kets;
+  return sizeof(Bra<R, NW>) * kFbThreads + sizeof(double) * (size_t)(kFbShares + 1) * kets;
 }
 
 template <bool F32, int LE, int LN>
@@ -400,6 +448,26 @@ cudaError_t persistent_dispatch(int kets, int le, int lp, const G3BatchSys* d_sy
 #undef PD
 }
 
+template <bool F32, int LE, int LN, int MODE>
+cudaError_t fb_pass(dim3 grid, size_t smem, const DevSystem& sys, const double* erec,
+                    const double* prec, double screen, double* r4, cudaStream_t s) {
+  auto* kernel = gam3_fb_kernel<F32, LE, LN, MODE>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kFbThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = at.val.clusterDim.y = 1;
+  at.val.clusterDim.z = grid.z;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, sys, erec, prec, screen, r4);
+}
+
 template <bool F32, int LE, int LN>
 cudaError_t fb_t(const DevSystem& sys, const double* erec, const double* prec,
                  double screen, double* r4, cudaStream_t s) {
@@ -410,19 +478,10 @@ cudaError_t fb_t(const DevSystem& sys, const double* erec, const double* prec,
   const int nPp = sys.npbf * (sys.npbf + 1) / 2;
   const long long nblk = (long long)nPp * nPe * nPe;
   if (nblk > 0x7fffffffLL || sys.g3_ntile > 65535) return cudaErrorInvalidValue;
-  const dim3 grid((unsigned)nblk, (unsigned)sys.g3_ntile);
-  cudaError_t e = cudaFuncSetAttribute(gam3_fb_kernel<F32, LE, LN, 0>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+  const dim3 grid((unsigned)nblk, (unsigned)sys.g3_ntile, (unsigned)fb_parts(sys));
+  cudaError_t e = fb_pass<F32, LE, LN, 0>(grid, smem, sys, erec, prec, screen, r4, s);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(gam3_fb_kernel<F32, LE, LN, 1>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  gam3_fb_kernel<F32, LE, LN, 0><<<grid, kFbThreads, smem, s>>>(sys, erec, prec, screen, r4);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  gam3_fb_kernel<F32, LE, LN, 1><<<grid, kFbThreads, smem, s>>>(sys, erec, prec, screen, r4);
-  return cudaGetLastError();
+  return fb_pass<F32, LE, LN, 1>(grid, smem, sys, erec, prec, screen, r4, s);
 }
 
 template <bool F32>
