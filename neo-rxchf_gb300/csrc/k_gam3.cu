@@ -124,7 +124,9 @@ __global__ void g3_records_kernel(DevSystem S, double* __restrict__ rec, double*
 }
 
 constexpr int kFbThreads = 128;   // threads (and bras per chunk) of a CTA
-constexpr int kFbShares = 4;      // shares of a chunk's bras that warps take
+// Shares of a chunk's bras that lanes take (with eight, loading the kets for
+// each showed: nebf = 5 of two primitives, npbf = 2: 3.5 -> 3.8 ms)
+constexpr int kFbShares = 4;
 constexpr int kFbMinPart = 16;    // fewest bras of a part
 
 __host__ __device__ __forceinline__ int nPe_of(int ne) { return ne * (ne + 1) / 2; }
@@ -202,9 +204,9 @@ __device__ __forceinline__ void fb_block(const DevSystem& S, const double* __res
 
   // Lane sums of ket kk, one row per bra share: acc_s[share * nkt + kk];
   // sums of the tile's electron pairs: tot
+  const int full = (nkt + 31) / 32 * 32;
+  const int pitch = LE == 0 || 4 * nkt < 3 * full ? nkt : full;   // lanes of a share
   double* tot = acc_s + kFbShares * nkt;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int ngrp = (nkt + 31) / 32;
   for (int z = z0; z < (CLUSTER ? z0 + 1 : nparts); z++) {
     if (z > z0) __syncthreads();   // the previous part's sums are taken
     const int zend = (z + 1) * plen < nbra ? (z + 1) * plen : nbra;
@@ -234,14 +236,17 @@ __device__ __forceinline__ void fb_block(const DevSystem& S, const double* __res
         bras[threadIdx.x] = b;
       }
       __syncthreads();
-      // Warps take (32 kets, share of the bras): with all the kets on the CTA's
-      // threads, a last round of few kets left most of its warps idle.
+      // Lanes take (share of the bras, ket), the kets of a share from a warp's
+      // first lane on, or beside each other where that left lanes empty: always
+      // with s functions (examples/xchf, 78 kets: 846 -> 792 us a Vee
+      // pass), with more than a quarter of them empty where warps then hold kets
+      // of different orders (36 kets, FP32: 669 -> 602 and 605 -> 551 us; 55 kets
+      // would lose 7 %).
       const int nsh = nvalid >= 16 ? kFbShares : (nvalid >= 8 ? 2 : 1);
-      for (int unit = warp; unit < ngrp * nsh; unit += kFbThreads / 32) {
-        const int grp = unit / nsh, sh = unit - grp * nsh;
-        const int i0 = nvalid * sh / nsh, i1 = nvalid * (sh + 1) / nsh;
-        const int kk = grp * 32 + lane;
+      for (int item = threadIdx.x; item < pitch * nsh; item += kFbThreads) {
+        const int sh = item / pitch, kk = item - sh * pitch;
         if (kk >= nkt) continue;
+        const int i0 = nvalid * sh / nsh, i1 = nvalid * (sh + 1) / nsh;
         const int kid = kperm[k0 + kk];
         const double* rk = erec + (size_t)kRLen * kid;
         const double qk = rk[kRQ];

@@ -208,8 +208,14 @@ NX_HD double boys_sum(int L, TT Tin, double alpha, BF&& b) {
   const double T = (double)Tin;
   const double ma = -alpha;
   if (!(T <= 20.0)) {
+#if defined(__CUDA_ARCH__)
+    // one FP64 reciprocal square root instead of two divisions and a root
+    const double rs = rsqrt(T), rT = rs * rs;
+    double f = 0.88622692545275801365 * rs;
+#else
     const double rT = 1.0 / T;
     double f = 0.88622692545275801365 / sqrt(T);
+#endif
     double s = f * (double)b(0), pw = 1.0;
     for (int m = 1; m <= L; m++) {
       f = f * ((double)m - 0.5) * rT;
