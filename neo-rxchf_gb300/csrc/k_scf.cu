@@ -23,6 +23,13 @@ namespace {
 // part[c*nt + t]: c = 0 E_ecore, 1 E_pcore, 2 E_ep, 3 E_ee, 4 E_gam1, 5 S_gam1.
 // xfocke / xfockp (optional): the NEO-HF part without GAM_1 (xchf1_fock.f's
 // Xfocke / Xfockp, :218-219).
+// A warp per t: one thread's chain of dependent FP64 adds over the density was
+// the kernel (nebf = 6, npbf = 1: 20.7 us; @FK@ so).
+__device__ __forceinline__ double lanes_sum(double v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 __global__ void fock1_kernel(int ne, int np, int nelec,
                              const double* __restrict__ Hce,
                              const double* __restrict__ Hcp,
@@ -37,36 +44,38 @@ __global__ void fock1_kernel(int ne, int np, int nelec,
                              double* __restrict__ part,
                              double* __restrict__ xfocke,
                              double* __restrict__ xfockp) {
-  const int nt = ne * ne + np * np;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int n2 = ne * ne, p2 = np * np, nt = n2 + p2;
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= nt) return;
-  const int n2 = ne * ne;
   double e[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  double fep = 0.0, fg1 = 0.0, s1 = 0.0;
   if (t < n2) {
     const int i = t / ne, j = t - i * ne;
-    const double fc = Hce[i * ne + j];
-    double fep = 0.0, fg1 = 0.0, s1 = 0.0;
-    for (int p = 0; p < np; p++)
-      for (int q = 0; q < np; q++) {
-        const double dp = DP[p + np * q];
-        const long long o = ((long long)(p * np + q) * ne + i) * ne + j;
-        fep = fep + dp * Gep[o];
-        fg1 = fg1 + dp * G1[o];
-        s1 = s1 + dp * G1s[o];
-      }
-    double fee = 0.0;
-    if (nelec > 1) {
-      for (int k = 0; k < ne; k++)
-        for (int l = 0; l < ne; l++) {
-          const double v1 = Gee[(((long long)i * ne + j) * ne + k) * ne + l];
-          const double v2 = Gee[(((long long)i * ne + l) * ne + k) * ne + j];
-          fee = fee + 2.0 * DE[k + ne * l] * ((v1 - 0.5 * v2) * 0.5);
-        }
+    for (int k = lane; k < p2; k += 32) {
+      const int p = k / np, q = k - p * np;
+      const double dp = DP[p + np * q];
+      const long long o = (long long)k * n2 + t;
+      fep = fma(dp, Gep[o], fep);
+      fg1 = fma(dp, G1[o], fg1);
+      s1 = fma(dp, G1s[o], s1);
     }
+    double fee = 0.0;
+    if (nelec > 1)
+      for (int m = lane; m < n2; m += 32) {
+        const int k = m / ne, l = m - k * ne;
+        const double v1 = Gee[(long long)t * n2 + m];
+        const double v2 = Gee[(((long long)i * ne + l) * ne + k) * ne + j];
+        fee = fma(DE[k + ne * l], fma(-0.5, v2, v1), fee);
+      }
+    fep = lanes_sum(fep);
+    fg1 = lanes_sum(fg1);
+    s1 = lanes_sum(s1);
+    fee = lanes_sum(fee);
+    if (lane) return;
+    const double fc = Hce[t], d = DE[i + ne * j];
     focke[i + ne * j] = fc + fep + fee + fg1;
     if (xfocke) xfocke[i + ne * j] = fc + fep + fee;
     se1[i + ne * j] = s1;
-    const double d = DE[i + ne * j];
     e[0] = d * fc;
     e[2] = d * fep;
     e[3] = d * (0.5 * fee);
@@ -74,16 +83,19 @@ __global__ void fock1_kernel(int ne, int np, int nelec,
     e[5] = d * s1;
   } else {
     const int k = t - n2, p = k / np, q = k - p * np;
-    const double fc = Hcp[p * np + q];
-    double fep = 0.0, fg1 = 0.0, s1 = 0.0;
-    for (int i = 0; i < ne; i++)
-      for (int j = 0; j < ne; j++) {
-        const double de = DE[i + ne * j];
-        const long long o = ((long long)(p * np + q) * ne + i) * ne + j;
-        fep = fep + de * Gep[o];
-        fg1 = fg1 + de * G1[o];
-        s1 = s1 + de * G1s[o];
-      }
+    for (int m = lane; m < n2; m += 32) {
+      const int i = m / ne, j = m - i * ne;
+      const double de = DE[i + ne * j];
+      const long long o = (long long)k * n2 + m;
+      fep = fma(de, Gep[o], fep);
+      fg1 = fma(de, G1[o], fg1);
+      s1 = fma(de, G1s[o], s1);
+    }
+    fep = lanes_sum(fep);
+    fg1 = lanes_sum(fg1);
+    s1 = lanes_sum(s1);
+    if (lane) return;
+    const double fc = Hcp[k];
     fockp[p + np * q] = fc + fep + fg1;
     if (xfockp) xfockp[p + np * q] = fc + fep;
     sp1[p + np * q] = s1;
@@ -103,20 +115,19 @@ __device__ double block_sum(double v, double* sw) {
   return r;   // every thread gets the same value
 }
 
-// en[2..6], en[11] from the partials; the later slots (gam_2..4) are zeroed
+// en[2..6], en[11] from the partials, a warp per channel (one channel after the
+// other: 11.9 us at nt = 37, @FE@ so); the later slots (gam_2..4) are zeroed
 // here and filled by their contractions when the electron count has them.
 __global__ void fock1_energy_kernel(int nt, const double* __restrict__ part,
                                     double* __restrict__ en) {
-  __shared__ double sw[32];
-  const int slot[6] = {2, 3, 4, 5, 6, 11};
-  for (int c = 0; c < 6; c++) {
-    double v = 0.0;
-    for (int t = threadIdx.x; t < nt; t += blockDim.x) v += part[(long long)c * nt + t];
-    const double s = block_sum(v, sw);
-    if (threadIdx.x == 0) en[slot[c]] = s;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) en[7] = en[8] = en[9] = en[12] = 0.0;
+  const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double v = 0.0;
+#pragma unroll 4
+  for (int t = lane; t < nt; t += 32) v += part[(long long)c * nt + t];
+  v = lanes_sum(v);
+  if (lane) return;
+  en[c < 5 ? c + 2 : 11] = v;
+  if (c == 0) en[7] = en[8] = en[9] = en[12] = 0.0;
 }
 
 // S_total, E_total, H_expect (xchf1_fock.f:311-319) and XCfock_correction
@@ -296,7 +307,27 @@ __global__ void uhf_dendif_kernel(int ne, int np, const double* __restrict__ DA,
 // diagonal to working precision and V holds the eigenvectors as columns.
 // Sweeps are bounded; *sweeps_out = sweeps used (kJacobiMaxSweeps + 1 when
 // the off-diagonal norm did not converge).
+// What bounds it at these sizes is the latency of dependent FP64 instructions:
+// a rotation comes from two reciprocal square roots (the tangent's two roots
+// and three divisions took twice the time), and rows and columns turn in one
+// pass over 2 x 2 blocks between two barriers.  roothan_kernel at n = 6: @JB@.
 constexpr int kJacobiMaxSweeps = 40;
+
+// Rotation of rows p < q from d = a_qq - a_pp and a_pq: t = tan of the smaller
+// angle with (1 - t^2) / (2 t) = d / (2 a_pq), c = 1 / sqrt(1 + t^2), s = t c
+__device__ __forceinline__ void jacobi_rotation(double d, double apq, double* c, double* s) {
+  const double h = apq + apq, w = fma(d, d, h * h);
+  if (w > 1e-280 && w < 1e280) {   // cos 2 angle = |d| / sqrt(w), sin 2 angle = |h| / sqrt(w)
+    const double r = rsqrt(w), c2 = fma(0.5 * fabs(d), r, 0.5), rc = rsqrt(c2);
+    *c = c2 * rc;
+    *s = (d == 0.0 ? fabs(h) : (d > 0.0 ? h : -h)) * (0.5 * r * rc);
+    return;
+  }
+  const double th = d / h;
+  const double t = (th >= 0.0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
+  *c = 1.0 / sqrt(t * t + 1.0);
+  *s = t * *c;
+}
 
 __device__ int jacobi_eig(int n, double* A, double* V, double* rc, double* rs,
                           int* rp, int* rq, double* sw) {
@@ -314,9 +345,21 @@ __device__ int jacobi_eig(int n, double* A, double* V, double* rc, double* rs,
       if (k / n == k % n) dia += a * a;
       else off += a * a;
     }
-    off = block_sum(off, sw);
+    const int nw = min((n * n + 31) >> 5, (int)blockDim.x >> 5);   // warps with elements
+    if ((int)threadIdx.x >> 5 < nw) {
+      off = lanes_sum(off);
+      dia = lanes_sum(dia);
+      if ((threadIdx.x & 31) == 0) {
+        sw[threadIdx.x >> 5] = off;
+        sw[16 + (threadIdx.x >> 5)] = dia;
+      }
+    }
     __syncthreads();
-    dia = block_sum(dia, sw);
+    off = dia = 0.0;
+    for (int k = 0; k < nw; k++) {
+      off += sw[k];
+      dia += sw[16 + k];
+    }
     __syncthreads();
     if (!(off == off) || !(dia == dia)) return kJacobiMaxSweeps + 2;   // NaN input
     if (off <= 1e-30 * dia || off == 0.0) break;
@@ -336,14 +379,9 @@ __device__ int jacobi_eig(int n, double* A, double* V, double* rc, double* rs,
         double c = 1.0, s = 0.0;
         if (q < n) {
           const double apq = A[p * n + q];
-          if (apq != 0.0) {
-            const double th = (A[q * n + q] - A[p * n + p]) / (2.0 * apq);
-            const double t = (th >= 0.0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
-            c = 1.0 / sqrt(t * t + 1.0);
-            s = t * c;
-          }
+          if (apq != 0.0) jacobi_rotation(A[q * n + q] - A[p * n + p], apq, &c, &s);
         } else {
-          p = q = -1;   // pair with the dummy index: no rotation
+          q = -1;   // p is paired with the dummy index: no rotation
         }
         rp[k] = p;
         rq[k] = q;
@@ -351,27 +389,37 @@ __device__ int jacobi_eig(int n, double* A, double* V, double* rc, double* rs,
         rs[k] = s;
       }
       __syncthreads();
-      // rows: A <- J^T A
-      for (int e = threadIdx.x; e < (m / 2) * n; e += blockDim.x) {
-        const int k = e / n, j = e - k * n, p = rp[k], q = rq[k];
-        if (p < 0) continue;
+      // A <- J^T A J, a thread per pair of pairs; V <- V J
+      const int h = m / 2;
+      for (int e = threadIdx.x; e < h * (h + n); e += blockDim.x) {
+        const int k = e % h, f = e / h, p = rp[k], q = rq[k];
         const double c = rc[k], s = rs[k];
-        const double apj = A[p * n + j], aqj = A[q * n + j];
-        A[p * n + j] = c * apj - s * aqj;
-        A[q * n + j] = s * apj + c * aqj;
-      }
-      __syncthreads();
-      // columns: A <- A J, V <- V J
-      for (int e = threadIdx.x; e < (m / 2) * n; e += blockDim.x) {
-        const int k = e / n, i = e - k * n, p = rp[k], q = rq[k];
-        if (p < 0) continue;
-        const double c = rc[k], s = rs[k];
-        const double aip = A[i * n + p], aiq = A[i * n + q];
-        A[i * n + p] = c * aip - s * aiq;
-        A[i * n + q] = s * aip + c * aiq;
-        const double vip = V[i * n + p], viq = V[i * n + q];
-        V[i * n + p] = c * vip - s * viq;
-        V[i * n + q] = s * vip + c * viq;
+        if (f >= h) {
+          double* v = V + (f - h) * n;
+          if (q < 0) continue;
+          const double vp = v[p], vq = v[q];
+          v[p] = c * vp - s * vq;
+          v[q] = s * vp + c * vq;
+          continue;
+        }
+        const int p1 = rp[f], q1 = rq[f];
+        const double c1 = rc[f], s1 = rs[f];
+        double* a = A + p1 * n;
+        double* b = A + (q1 < 0 ? p1 : q1) * n;
+        const double app = a[p], aqp = b[p];
+        const double xp = c1 * app - s1 * aqp, yp = s1 * app + c1 * aqp;
+        double xq = 0.0, yq = 0.0;
+        if (q >= 0) {
+          const double apq = a[q], aqq = b[q];
+          xq = c1 * apq - s1 * aqq;
+          yq = s1 * apq + c1 * aqq;
+        }
+        a[p] = c * xp - s * xq;
+        if (q >= 0) a[q] = s * xp + c * xq;
+        if (q1 >= 0) {
+          b[p] = c * yp - s * yq;
+          if (q >= 0) b[q] = s * yp + c * yq;
+        }
       }
       __syncthreads();
     }
@@ -583,63 +631,61 @@ __global__ void diis_kernel(int n, double* __restrict__ F,
   }
   __syncthreads();
   const int cnt = s_cnt + 1 < kDiisMax ? s_cnt + 1 : kDiisMax;
-  // new row of B: <e_slot, e_j> for the occupied slots
-  for (int j = 0; j < cnt; j++) {
+  // new row of B: <e_slot, e_j> for the occupied slots, a warp each
+  for (int j = threadIdx.x >> 5; j < cnt; j += blockDim.x >> 5) {
     const double* ej = Eh + (size_t)j * nn;
     double acc = 0.0;
-    for (int k = threadIdx.x; k < nn; k += blockDim.x) acc += e[k] * ej[k];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) sw[threadIdx.x / 32] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double r = 0.0;
-      for (int k = 0; k < (int)(blockDim.x + 31) / 32; k++) r += sw[k];
-      B[slot * kDiisMax + j] = r;
-      B[j * kDiisMax + slot] = r;
+    for (int k = threadIdx.x & 31; k < nn; k += 32) acc += e[k] * ej[k];
+    acc = lanes_sum(acc);
+    if ((threadIdx.x & 31) == 0) {
+      B[slot * kDiisMax + j] = acc;
+      B[j * kDiisMax + slot] = acc;
     }
-    __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    state[0] = cnt;
-    state[1] = (slot + 1) % kDiisMax;
-    s_ok = 0;
-    if (cnt >= 2) {
-      const int m = cnt + 1;
-      double A[(kDiisMax + 1) * (kDiisMax + 2)];
-      const int w = m + 1;
-      for (int i = 0; i < cnt; i++) {
-        for (int j = 0; j < cnt; j++) A[i * w + j] = B[i * kDiisMax + j];
-        A[i * w + cnt] = -1.0;
-        A[i * w + m] = 0.0;
-      }
-      for (int j = 0; j < cnt; j++) A[cnt * w + j] = -1.0;
-      A[cnt * w + cnt] = 0.0;
-      A[cnt * w + m] = -1.0;
+  __syncthreads();
+  // Gauss-Jordan, a row per lane (one thread: @DI@ a call, most of it the
+  // latency of some 700 dependent FP64 instructions)
+  if (threadIdx.x < 32) {
+    const int r = threadIdx.x, m = cnt + 1, w = m + 1;
+    __shared__ double A[(kDiisMax + 1) * (kDiisMax + 2)];
+    bool ok = cnt >= 2;
+    if (ok) {
       double scale = 0.0;
       for (int i = 0; i < cnt; i++) scale = fmax(scale, fabs(B[i * kDiisMax + i]));
-      bool ok = scale > 0.0;
+      ok = scale > 0.0;
+      if (r < m) {
+        for (int j = 0; j < cnt; j++) A[r * w + j] = r < cnt ? B[r * kDiisMax + j] : -1.0;
+        A[r * w + cnt] = r < cnt ? -1.0 : 0.0;
+        A[r * w + m] = r < cnt ? 0.0 : -1.0;
+      }
+      __syncwarp();
       for (int c = 0; c < m && ok; c++) {
         int piv = c;
-        for (int r = c + 1; r < m; r++)
-          if (fabs(A[r * w + c]) > fabs(A[piv * w + c])) piv = r;
-        if (fabs(A[piv * w + c]) < 1e-14 * fmax(scale, 1.0)) { ok = false; break; }
-        if (piv != c)
-          for (int k = 0; k <= m; k++) {
-            const double t = A[c * w + k];
-            A[c * w + k] = A[piv * w + k];
-            A[piv * w + k] = t;
-          }
-        for (int r = 0; r < m; r++) {
-          if (r == c) continue;
+        for (int k = c + 1; k < m; k++)
+          if (fabs(A[k * w + c]) > fabs(A[piv * w + c])) piv = k;
+        if (fabs(A[piv * w + c]) < 1e-14 * fmax(scale, 1.0)) {
+          ok = false;
+          break;
+        }
+        __syncwarp();
+        if (piv != c && r <= m) {
+          const double t = A[c * w + r];
+          A[c * w + r] = A[piv * w + r];
+          A[piv * w + r] = t;
+        }
+        __syncwarp();
+        if (r < m && r != c) {
           const double fct = A[r * w + c] / A[c * w + c];
           for (int k = c; k <= m; k++) A[r * w + k] -= fct * A[c * w + k];
         }
+        __syncwarp();
       }
-      if (ok) {
-        for (int i = 0; i < cnt; i++) coef[i] = A[i * w + m] / A[i * w + i];
-        s_ok = 1;
-      }
+      if (ok && r < cnt) coef[r] = A[r * w + m] / A[r * w + r];
+    }
+    if (r == 0) {
+      state[0] = cnt;
+      state[1] = (slot + 1) % kDiisMax;
+      s_ok = ok;
     }
   }
   __syncthreads();
@@ -883,10 +929,10 @@ cudaError_t launch_scf_fock1(int ne, int np, int nelec, const double* Hce,
                              double* se1, double* sp1, double* part, double* en,
                              cudaStream_t s, double* xfocke, double* xfockp) {
   const int nt = ne * ne + np * np;
-  fock1_kernel<<<(nt + 127) / 128, 128, 0, s>>>(ne, np, nelec, Hce, Hcp, Gep, G1,
+  fock1_kernel<<<(nt + 3) / 4, 128, 0, s>>>(ne, np, nelec, Hce, Hcp, Gep, G1,
                                                 G1s, Gee, DE, DP, focke, fockp,
                                                 se1, sp1, part, xfocke, xfockp);
-  fock1_energy_kernel<<<1, 256, 0, s>>>(nt, part, en);
+  fock1_energy_kernel<<<1, 6 * 32, 0, s>>>(nt, part, en);
   return cudaGetLastError();
 }
 
@@ -978,7 +1024,7 @@ cudaError_t launch_uhf_fock1(int ne, int np, const double* Hce, const double* Hc
   uhf_fock1_kernel<<<(nt + 127) / 128, 128, 0, s>>>(ne, np, Hce, Hcp, Gep, G1, G1s, Gee,
                                                     DAE, DBE, DP, FAE, FBE, FP, SAE1,
                                                     SBE1, SP1, part);
-  fock1_energy_kernel<<<1, 256, 0, s>>>(nt, part, en);
+  fock1_energy_kernel<<<1, 6 * 32, 0, s>>>(nt, part, en);
   return cudaGetLastError();
 }
 
