@@ -380,6 +380,13 @@ G3_HD double pair_coulomb(const double* r, const double* s) {
   return (2.0 * kPi * kPi * sqrt(kPi)) * rs / pq * coulomb_sum<NT>(n, W, R, alpha * R2, alpha);
 }
 
+// |c_a c_b| sqrt((ab|ab)) of a pair record.  (As an integral over four
+// primitives this was the longest chain of g3_records_kernel: examples/xchf,
+// 86 us, and nebf = 4 s/p, 128 us; 63 on average from the record.)
+G3_HD double schwarz_factor(const double* r) {
+  return fabs(r[kRC]) * sqrt(fabs(pair_coulomb<8>(r, r)));
+}
+
 // The multiplicative terms of xcalc_GAM1_MD's integrand (gam_1_OMP.f:398-836)
 // for an electron and a proton pair density coupled by exp(-g r^2):
 // *e = -Z/r_eC + Z/r_pC - 1/r_ep, *ov = the overlap.

@@ -36,7 +36,8 @@ G3_HD int pair_index(int i, int j) {
   return i >= j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i;
 }
 
-// Record of one primitive pair (A, B) with contraction coefficients ca, cb.
+// Record of one primitive pair (A, B) with contraction coefficients ca, cb
+// (without Q, which comes from the record itself: g2::schwarz_factor).
 G3_HD void fill_pair_record(const md::Prim& A, const md::Prim& B, double ca, double cb,
                             double* out) {
   md::Pair pr;
@@ -58,8 +59,7 @@ G3_HD void fill_pair_record(const md::Prim& A, const md::Prim& B, double ca, dou
   const double cab = fabs(ca * cb);
   const double pi = 3.14159265358979323846;
   out[kRS] = cab * pow(pi / pr.p, 1.5) * pr.K[0] * pr.K[1] * pr.K[2] * ang;
-  out[kRQ] = cab * sqrt(fabs(md::gfvee(A, A, B, B)));
-  for (int k = 25; k < kRLen; k++) out[k] = 0.0;
+  for (int k = kRQ; k < kRLen; k++) out[k] = 0.0;
 }
 
 // ---- composite bra -----------------------------------------------------------

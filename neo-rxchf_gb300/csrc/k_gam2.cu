@@ -237,6 +237,7 @@ gam2_triple_kernel(DevSystem S, int Pp0, long long nunit,
   int* que = s_q[wid];
   int nq = 0;
   const long long o = ((long long)split * nunit + row) * v.nket;
+  int turn = 0;   // the warps of grid z take every gridDim.z-th 32 kets
   for (int p0 = 0; p0 < v.nket || nq > 0;) {
     while (nq < 32 && p0 < v.nket) {
       const int pos = p0 + lane;
@@ -249,7 +250,8 @@ gam2_triple_kernel(DevSystem S, int Pp0, long long nunit,
       __syncwarp();
     }
     const int nv = nq < 32 ? nq : 32;
-    if (lane < nv) {
+    const bool mine = turn++ % gridDim.z == blockIdx.z;
+    if (lane < nv && mine) {
       const int kid = que[lane];
       const double* r2 = v.erec + (size_t)kRLen * kid;
       const double* e2 = v.egrad + (size_t)kGLen * kid;
@@ -279,24 +281,39 @@ gam2_triple_kernel(DevSystem S, int Pp0, long long nunit,
   }
 }
 
-// out[row][P] = sum_split sum_{ket of P} in[split][row][ket]; lower = only P <= row % nPe
-__global__ void gam2_contract_kernel(DevSystem S, long long nrow, int nsplit, int lower,
+// out[row][P] = sum_split sum_{ket of P} in[split][row][ket]; lower = only P <= row % nPe.
+// lanes (a power of two) threads share a sum over the splits: with one, a small
+// system's 64 splits were 57 us of dependent adds (examples/xchf; 6 so).
+__global__ void gam2_contract_kernel(DevSystem S, long long nrow, int nsplit, int lower, int lanes,
                                      const double* __restrict__ in, double* __restrict__ out) {
   const int nPe = S.nebf * (S.nebf + 1) / 2, nket = S.g3_nket;
   const int* kofs = S.g3i + 2 * nket;
-  const long long n = nrow * nPe;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int P = (int)(t % nPe);
+  const long long n = nrow * nPe * lanes;
+  const int sub = threadIdx.x & (lanes - 1);
+  // (a warp's threads stay in the loop together)
+  for (long long u0 = blockIdx.x * (long long)blockDim.x; u0 < n; u0 += (long long)gridDim.x * blockDim.x) {
+    const long long t = (u0 + threadIdx.x) / lanes;
     const long long row = t / nPe;
-    if (lower && P > (int)(row % nPe)) continue;
+    const int P = (int)(t - row * nPe);
+    const bool on = row < nrow && !(lower && P > (int)(row % nPe));
     double s = 0.0;
-    for (int q = 0; q < nsplit; q++) {
-      const double* x = in + ((long long)q * nrow + row) * nket;
-      for (int k = kofs[P]; k < kofs[P + 1]; k++) s += x[k];
-    }
-    out[t] = s;
+    if (on)
+      for (int q = sub; q < nsplit; q += lanes) {
+        const double* x = in + ((long long)q * nrow + row) * nket;
+        for (int k = kofs[P]; k < kofs[P + 1]; k++) s += x[k];
+      }
+    for (int o = lanes >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (on && sub == 0) out[t] = s;
   }
+}
+
+void contract(const DevSystem& S, long long nrow, int nsplit, int lower, const double* in,
+              double* out, cudaStream_t s) {
+  const int nPe = S.nebf * (S.nebf + 1) / 2;
+  int lanes = 1;
+  while (lanes < 32 && 2 * lanes < nsplit) lanes *= 2;
+  const unsigned nb = (unsigned)std::min<long long>((nrow * nPe * lanes + 127) / 128, 152 * 16);
+  gam2_contract_kernel<<<nb, 128, 0, s>>>(S, nrow, nsplit, lower, lanes, in, out);
 }
 
 // The contracted canonical arrays onto the packed order: block y is the
@@ -389,13 +406,16 @@ cudaError_t build_t(const DevSystem& S, const Plan& p, double* scratch, int Pp0,
     double* R1c = Yc + (size_t)units * p.nPe;
     double* R2c = R1c + (size_t)units * p.nPe;
     const unsigned nb = (unsigned)((units + kWarps - 1) / kWarps);
-    gam2_triple_kernel<LE, LN, RX ? kCoulomb12 : kAll><<<dim3(nb, p.spR), 32 * kWarps, 0, s>>>(S, c0, units, R1, R2);
+    // too few warps even with a bra each: the 32-ket turns of one over several
+    // (examples/xchf, 1344 warps of three turns: 283 us, 150 so)
+    const unsigned nz = units * p.spR < kWantWarps ? std::min((p.nket + 31) / 32, 4) : 1;
+    gam2_triple_kernel<LE, LN, RX ? kCoulomb12 : kAll><<<dim3(nb, p.spR, nz), 32 * kWarps, 0, s>>>(
+        S, c0, units, R1, R2);
     gam2_pair_kernel<LE, LN, RX><<<dim3(nb, (p.nket + 31) / 32, p.spY), 32 * kWarps, 0, s>>>(
         S, c0, units, Y);
-    const unsigned cb = (unsigned)std::min<long long>((units * p.nPe + 127) / 128, 152 * 16);
-    gam2_contract_kernel<<<cb, 128, 0, s>>>(S, units, p.spY, 0, Y, Yc);
-    if (!RX) gam2_contract_kernel<<<cb, 128, 0, s>>>(S, units, p.spR, 1, R1, R1c);
-    gam2_contract_kernel<<<cb, 128, 0, s>>>(S, units, p.spR, 1, R2, R2c);
+    contract(S, units, p.spY, 0, Y, Yc, s);
+    if (!RX) contract(S, units, p.spR, 1, R1, R1c, s);
+    contract(S, units, p.spR, 1, R2, R2c, s);
     const long long n4 = (long long)ne * ne * ne * ne;
     const dim3 eg((unsigned)std::min<long long>((n4 + 255) / 256, 1024), (unsigned)nc);
     if (one)
@@ -494,8 +514,7 @@ cudaError_t launch_gam3_factors(const DevSystem& S, double* scratch, const doubl
       case 8: overlap_t<2, 2>(S, p, c0, units, R2, s); break;
       default: return cudaErrorInvalidValue;
     }
-    const unsigned cb = (unsigned)std::min<long long>((units * p.nPe + 127) / 128, 152 * 16);
-    gam2_contract_kernel<<<cb, 128, 0, s>>>(S, units, p.spR, 1, R2, R2c);
+    contract(S, units, p.spR, 1, R2, R2c, s);
     overlap_expand_kernel<<<dim3((unsigned)std::min<long long>((n4 + 255) / 256, 1024), nc), 256, 0, s>>>(
         ne, np, c0, R2c, W3);
   }

@@ -118,8 +118,11 @@ __global__ void g3_records_kernel(DevSystem S, double* __restrict__ rec, double*
       pa = S.pprim + ip;
       pb = S.pprim + jp;
     }
-    if (u < n) fill_pair_record(to_md(*pa), to_md(*pb), pa->coef, pb->coef, rec + (size_t)kRLen * t);
-    else g2::fill_gradient_record(to_md(*pa), to_md(*pb), grad + (size_t)g2::kGLen * t);
+    double* r = rec + (size_t)kRLen * t;
+    if (u < n) {
+      fill_pair_record(to_md(*pa), to_md(*pb), pa->coef, pb->coef, r);
+      r[kRQ] = g2::schwarz_factor(r);
+    } else g2::fill_gradient_record(to_md(*pa), to_md(*pb), grad + (size_t)g2::kGLen * t);
   }
 }
 
