@@ -266,7 +266,7 @@ def run_reference(args):
 
 
 FACTORED_LARGE = (60, 24)   # nebf, npbf of the mixed-precision XCHF shape
-FACTORED_LAUNCHES = 14      # kernels of one factorised build (k_gam4f.cu)
+FACTORED_LAUNCHES = 4       # kernels of one factorised build (k_gam4f.cu)
 
 
 def time_factored(neoxc, torch, dev, stream, ne, np_, d_gee, d_g2s, d_DE, d_DP,
@@ -453,7 +453,7 @@ def open_shell_section(neoxc, torch, dev, stream):
                                     "frac": gbs / peak if peak else None,
                                     "algorithmic_bytes": nbytes},
                             "bound": "fp64",
-                            "launches_per_call": 5}
+                            "launches_per_call": 7 if k == 3 else 6}
         del G, Gs
         torch.cuda.empty_cache()
     return out
@@ -578,13 +578,10 @@ def scf_section(neoxc, with_cpu: bool):
                      "E_err_vs_log": r["final"]["E_total"] - E_log}
         if mixed:
             out[name]["E_err_vs_fp64_Eh"] = r["final"]["E_total"] - E_fp64
-            out[name]["precision"] = ("%s MD tables FP32 (Boys function, seeds, sums over "
-                                      "primitives and geminal terms FP64%s); one-body, "
-                                      "GAM_1, GAM_ee, contractions, Fock assembly and "
-                                      "diagonalisation FP64"
-                                      % (("gam_3", "") if mixed == "gam3" else
-                                         ("gam_2, gam_3", "; gam_2 items above the "
-                                          "recompute threshold in FP64")))
+            out[name]["precision"] = ("gam_3 MD tables FP32 (Boys function, seeds, sums over "
+                                      "primitives and geminal terms FP64); one-body, GAM_1, "
+                                      "GAM_ee, gam_2, contractions, Fock assembly and "
+                                      "diagonalisation FP64")
         else:
             E_fp64 = r["final"]["E_total"]
     out["config1"] = config1_section(neoxc)
@@ -609,10 +606,9 @@ def config1_section(neoxc):
     solve = every integral built on the GPU (gam_2 and the 1.9e8-element
     gam_3 tensor included) from core-Hamiltonian guesses and DIIS SCF to
     the reference's convergence rule, through neoxc_xchf_scf with host
-    arrays.  Mixed (FP32 McMurchie-Davidson tables for gam_2 and gam_3 with
-    FP64 Boys function, seeds and sums, the large gam_2 items re-evaluated
-    in FP64; Fock assembly and diagonalisation FP64), then FP64; the mixed
-    energy is reported against the FP64 one."""
+    arrays.  Mixed (FP32 McMurchie-Davidson tables for gam_3 with FP64 Boys
+    function, seeds and sums; gam_2, Fock assembly and diagonalisation FP64),
+    then FP64; the mixed energy is reported against the FP64 one."""
     from neoxc import basis
     s = basis.synthetic(**CONFIG1)
     out = {"workload": "XCHF RHF, seeded synthetic system (seed %d): nebf=%d (s/p, 3 primitives), "
@@ -736,10 +732,7 @@ def gam3_batch_section(neoxc, nsys=48):
 
 
 # Precision of the mixed arms of the examples/xchf scans: gam_3 in FP32
-# tables (0.15 microhartree from FP64 on this system), gam_2 in FP64.  Most
-# gam_2 items of this basis (tight s primitives) lie above the dynamic-
-# precision threshold, where the mixed gam_2 build costs more than the FP64
-# one (52.0 vs 43.7 ms per DIIS solve).
+# tables (0.15 microhartree from FP64 on this system), gam_2 in FP64.
 SCAN_MIXED = "gam3"
 
 

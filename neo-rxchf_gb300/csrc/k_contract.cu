@@ -2,13 +2,14 @@
 // deterministic partial-sum reducer shared by every contraction kernel.
 //
 // Reference: gam2_IC1_OMP.f:339-570 (EG2IC1 / thread_EG2ICR),
-// gam3_IC1_OMP.f:433-725 (EG3IC1 / thread_EG3ICR), rxchfne/rxchfne_omg2.f
-// (RXCHFne_FAE/FP/FBE_OMG2), xchf1_independent/xchf1_fock.f:728-783
-// (XCfock_correction), CS_Integrals/Spot_Check/pack_GAM.f (index maps).
+// gam3_IC1_OMP.f:433-725 (EG3IC1 / thread_EG3ICR; its kernel: k_rank3.cu),
+// rxchfne/rxchfne_omg2.f (RXCHFne_FAE/FP/FBE_OMG2),
+// xchf1_independent/xchf1_fock.f:728-783 (XCfock_correction),
+// CS_Integrals/Spot_Check/pack_GAM.f (index maps).
 //
-// All kernels here are HBM-bound streams over the stored integral tensor:
-// every element is read from HBM once, permuted partners are gathered from
-// shared memory, and partial sums are written per CTA and reduced by a
+// All kernels here stream over the stored integral tensor: every element is
+// read from HBM once (FP64 instructions bound the wider ones, see each), and
+// partial sums are written per CTA and reduced by a
 // second, deterministic kernel (no floating-point atomics), so repeated
 // calls give bit-identical results.
 #include <algorithm>

@@ -30,8 +30,8 @@
 //
 // Measured (one GB300, neoxc_gam2_ic1 / _rxchfne_gam2_ic1 from host arrays):
 // nebf = 8 s/p of 2 primitives, npbf = 3 s/p/d, NG = 3: 494 ms element by
-// element, 6.4 ms so; RXCHF-ne, nebf = 9 s/p/d, npbf = 4, NG = 4: 815 ms and
-// 13.7 ms.  The former FP32-first form (dynamic precision) was 1.8x faster
+// element, 5.6 ms so; RXCHF-ne, nebf = 9 s/p/d, npbf = 4, NG = 4: 815 ms and
+// 11.7 ms.  The former FP32-first form (dynamic precision) was 1.8x faster
 // than the first of each pair, so it is gone.
 //
 // A warp owns one canonical (proton pair, electron pair) and a share of its

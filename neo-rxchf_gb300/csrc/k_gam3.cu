@@ -42,11 +42,11 @@
 //
 // FP64 instructions bound the FP64 build (2 per SM and clock): fb_value takes
 // about half of fb_eval's, G4Vep runs over unordered (e1, e2) pairs, the bras
-// fold one particle at a time, and warps share (32 kets, a quarter of the
-// bras) units so that none idles in a last round of few kets.  Measured (one
+// fold one particle at a time, lanes take (share of the bras, ket) items, and
+// small systems cut a block's bras into parts.  Measured (one
 // GB300, neoxc_gam3_ic1): nebf = 6 s/p of 3 primitives, npbf = 4 s/p/d,
 // NG = 3: 516 -> 279 ms, 253 ms with the overlap-only W3 of k_gam2.cu; FP32
-// tables at nebf = 4, npbf = 2: 6.5 -> 3.8 -> 2.1 ms.
+// tables at nebf = 4, npbf = 2: 6.5 -> 2.1 -> 1.6 ms (parts and packed lanes).
 //
 // The prefactors, exponents and centres follow G4_MD_xgVepg / G4_MD_xgVeeg
 // (truncated pi, the reference's underflow on every G4Vep value); only the

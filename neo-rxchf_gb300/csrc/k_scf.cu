@@ -644,8 +644,8 @@ __global__ void diis_kernel(int n, double* __restrict__ F,
     }
   }
   __syncthreads();
-  // Gauss-Jordan, a row per lane (one thread: 37 us a call of the kernel, 16 so; most of it was the
-  // latency of some 700 dependent FP64 instructions)
+  // Gauss-Jordan, a row per lane (one thread: 37 us a call of the kernel, 16
+  // so; most of it was the latency of some 700 dependent FP64 instructions)
   if (threadIdx.x < 32) {
     const int r = threadIdx.x, m = cnt + 1, w = m + 1;
     __shared__ double A[(kDiisMax + 1) * (kDiisMax + 2)];

@@ -14,7 +14,7 @@
 //   class A = the alpha Fock row (FAE) and the alpha-weighted proton term,
 //   class B = the same with alpha and beta exchanged (FBE, beta weights).
 // The flag sets of the reference (LAA, LAB, ... / L4A, L3A1B, ...) arrive
-// as bit masks, so FAE with swapped arguments (the reference's beta call)
+// as bit masks (rank 3 has its kernel in k_rank3.cu), so FAE with swapped arguments (the reference's beta call)
 // and UFP's class B are the same code.  Per-CTA partials are reduced by a
 // second deterministic kernel (no floating-point atomics).
 #include <type_traits>

@@ -5,8 +5,7 @@
 // the mixed-precision path).  In both instances the Boys function, the
 // seeds (-alpha)^m F_m(T) and the final Hermite-Coulomb sum are FP64; md32's
 // Gaussian-product set-up, Hermite and derivative tables and the Hermite
-// folds are FP32.  The mixed gam_2 build re-evaluates every md32 result
-// whose contribution is large with md (dynamic precision, k_md.cu).
+// folds are FP32 (the mixed gam_3 build).
 //
 // The reference evaluates each primitive integral as a 9- or 12-deep loop
 // over Hermite indices, and inside every iteration re-derives the Boys'

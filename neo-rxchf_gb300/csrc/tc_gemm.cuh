@@ -19,7 +19,8 @@
 //   * every thread waits on the mbarrier (bounded: after kSpinLimit polls the
 //     kernel records an error flag instead of hanging);
 // and finally each warp reads half the columns of its 32 accumulator lanes
-// (its number modulo four) with tcgen05.ld and the CTA writes the FP64 tile through shared memory, coalesced.  Tensor memory (64 columns) is allocated
+// (its number modulo four) with tcgen05.ld and the CTA writes the FP64 tile
+// through shared memory, coalesced.  Tensor memory (64 columns) is allocated
 // and freed by warp 0.
 #pragma once
 #include <cuda_runtime.h>
