@@ -70,6 +70,7 @@ G3_HD void fill_gradient_record(const md::Prim& A, const md::Prim& B, double* ou
 template <int NT>
 G3_HD double coulomb_sum(const int* n, const double (*W)[NT + 1], const double* R, double T,
                          double alpha) {
+  static_assert(NT <= g3::kHermMax, "hermite_scaled's tables");
   const double z = -(alpha + alpha);
   double B[3 * NT + 1], A[NT + 1];
   g3::hermite_scaled(n[0], W[0], z * R[0], z, B);

@@ -445,38 +445,46 @@ G3_HD double asym(int L) {
 #endif
 }
 
-// t! / ((2i-t)! (t-i)! 2^(t-i)), t, i <= 12 (zero unless i <= t <= 2i)
+// Largest Hermite order of one direction: d electrons in the bra's two pairs
+// and the ket (4 each) and a d proton pair (4).
+constexpr int kHermMax = 16;
+
+// t! / ((2i-t)! (t-i)! 2^(t-i)), t, i <= kHermMax (zero unless i <= t <= 2i)
 #define NX_HERMX_VALUES \
-    1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
-    0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
-    0, 1.0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
-    0, 0, 3.0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
-    0, 0, 3.0, 6.0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, \
-    0, 0, 0, 15.0, 10.0, 1.0, 0, 0, 0, 0, 0, 0, 0, \
-    0, 0, 0, 15.0, 45.0, 15.0, 1.0, 0, 0, 0, 0, 0, 0, \
-    0, 0, 0, 0, 105.0, 105.0, 21.0, 1.0, 0, 0, 0, 0, 0, \
-    0, 0, 0, 0, 105.0, 420.0, 210.0, 28.0, 1.0, 0, 0, 0, 0, \
-    0, 0, 0, 0, 0, 945.0, 1260.0, 378.0, 36.0, 1.0, 0, 0, 0, \
-    0, 0, 0, 0, 0, 945.0, 4725.0, 3150.0, 630.0, 45.0, 1.0, 0, 0, \
-    0, 0, 0, 0, 0, 0, 10395.0, 17325.0, 6930.0, 990.0, 55.0, 1.0, 0, \
-    0, 0, 0, 0, 0, 0, 10395.0, 62370.0, 51975.0, 13860.0, 1485.0, 66.0, 1.0
+    1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 1.0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 0, 3.0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 0, 3.0, 6.0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 0, 0, 15.0, 10.0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 0, 0, 15.0, 45.0, 15.0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 0, 0, 0, 105.0, 105.0, 21.0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 0, 0, 0, 105.0, 420.0, 210.0, 28.0, 1.0, 0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 0, 0, 0, 0, 945.0, 1260.0, 378.0, 36.0, 1.0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 0, 0, 0, 0, 945.0, 4725.0, 3150.0, 630.0, 45.0, 1.0, 0, 0, 0, 0, 0, 0, \
+    0, 0, 0, 0, 0, 0, 10395.0, 17325.0, 6930.0, 990.0, 55.0, 1.0, 0, 0, 0, 0, 0, \
+    0, 0, 0, 0, 0, 0, 10395.0, 62370.0, 51975.0, 13860.0, 1485.0, 66.0, 1.0, 0, 0, 0, 0, \
+    0, 0, 0, 0, 0, 0, 0, 135135.0, 270270.0, 135135.0, 25740.0, 2145.0, 78.0, 1.0, 0, 0, 0, \
+    0, 0, 0, 0, 0, 0, 0, 135135.0, 945945.0, 945945.0, 315315.0, 45045.0, 3003.0, 91.0, 1.0, 0, 0, \
+    0, 0, 0, 0, 0, 0, 0, 0, 2027025.0, 4729725.0, 2837835.0, 675675.0, 75075.0, 4095.0, 105.0, 1.0, 0, \
+    0, 0, 0, 0, 0, 0, 0, 0, 2027025.0, 16216200.0, 18918900.0, 7567560.0, 1351350.0, 120120.0, 5460.0, 120.0, 1.0
 #if defined(__CUDACC__)
-static __device__ const double kHermXDev[13 * 13] = {NX_HERMX_VALUES};
+static __device__ const double kHermXDev[(kHermMax + 1) * (kHermMax + 1)] = {NX_HERMX_VALUES};
 #endif
-static const double kHermXHost[13 * 13] = {NX_HERMX_VALUES};
+static const double kHermXHost[(kHermMax + 1) * (kHermMax + 1)] = {NX_HERMX_VALUES};
 #undef NX_HERMX_VALUES
 G3_HD double hermx(int t, int i) {
 #if defined(__CUDA_ARCH__)
-  return __ldg(&kHermXDev[t * 13 + i]);
+  return __ldg(&kHermXDev[t * (kHermMax + 1) + i]);
 #else
-  return kHermXHost[t * 13 + i];
+  return kHermXHost[t * (kHermMax + 1) + i];
 #endif
 }
 
 // The factors of F_i(alpha R^2) in sum_t W[t] d^t/dR^t F_0(alpha R^2), i <= n:
 //   A[i] = sum_t W[t] t! / ((2i-t)! (t-i)!) (-2 alpha R)^(2i-t) (-alpha)^(t-i)
-// with y = -2 alpha R and z = -2 alpha.  Orders up to 4 straight (s, p and
-// most d pairs), beyond by Horner in y.
+// with y = -2 alpha R and z = -2 alpha, n <= kHermMax.  Orders up to 4 straight
+// (s, p and most d pairs), beyond by Horner in y.
 G3_HD void hermite_scaled(int n, const double* W, double y, double z, double* A) {
   A[0] = W[0];
   if (n == 0) return;
@@ -505,7 +513,7 @@ G3_HD void hermite_scaled(int n, const double* W, double y, double z, double* A)
     A[4] = w4 * y2 * y2;
     return;
   }
-  double zp[7];
+  double zp[kHermMax / 2 + 1];
   zp[0] = 1.0;
   for (int k = 1; k <= n / 2; k++) zp[k] = zp[k - 1] * z;
   double yp = 1.0;   // y^(2i - min(2i, n))
@@ -627,6 +635,7 @@ G3_HD void load_ket(const double* rk, Ket<NK>& k) {
 template <int NW, int NK>
 G3_HD double fb_value(const Bra<double, NW>& b, const Ket<NK>& k) {
   constexpr int NT = NW + NK;
+  static_assert(NT <= kHermMax, "hermite_scaled's tables");
   const double rs = rsqrt64(b.Z + k.p), z = b.Z * k.p * (rs * rs);   // z: alpha
   double R[3], R2 = 0.0;
   for (int d = 0; d < 3; d++) {
