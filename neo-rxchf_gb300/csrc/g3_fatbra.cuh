@@ -622,8 +622,11 @@ G3_HD void load_ket(const double* rk, Ket<NK>& k) {
     const double* E = rk + kRE + 5 * d;
     k.X[d] = rk[kRX + d];
     k.t[d] = n;
-    const double top = E[n];   // K / (2p)^n: zero only where K underflowed
-    const double r = top != 0.0 ? 1.0 / top : 0.0;
+    // E[n] = K / (2p)^n.  With K underflowing its reciprocal would overflow and
+    // the coefficients lose their digits: the whole density, K times a few
+    // powers of its widths, is then far below 1e-250 and is left out.
+    const bool on = n == 0 || !(fabs(E[n]) < 1e-280);   // (NaN goes on)
+    const double top = on ? E[n] : 0.0, r = on ? 1.0 / top : 0.0;
     f *= (n & 1) ? -top : top;
     if (NK > 0)
       for (int q = 0; q < n; q++) k.e[d][q] = ((n - q) & 1) ? -(E[q] * r) : E[q] * r;
