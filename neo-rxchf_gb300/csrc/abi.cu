@@ -2026,10 +2026,13 @@ static size_t xchf_job_bytes(const neoxc_xchf_job& j, int64_t options) {
   const size_t ne = (size_t)j.nebf, np = (size_t)j.npbf;
   const size_t e2 = ne * ne, p2 = np * np;
   size_t d = 4 * e2 + 4 * p2 + 3 * e2 * p2 + e2 * e2 + 32 * (e2 + p2);
-  if (j.nelec > 1) {
-    d += 2 * e2 * e2 * p2 + eg2_partial_doubles((int)ne, (int)np);
-    // the gam_2 build's scratch: primitive pairs of the canonical pairs
-    // (a range that stage_system will refuse counts as one primitive)
+  if (j.nelec > 1) d += 2 * e2 * e2 * p2 + eg2_partial_doubles((int)ne, (int)np);
+  // the gam_2 build's scratch, for sizes that the solve will not refuse:
+  // primitive pairs of the canonical pairs (a range that stage_system will
+  // refuse counts as one primitive)
+  const bool sizes = j.nebf >= 1 && j.nebf <= kScfMaxN && j.npbf >= 1 && j.npbf <= kScfMaxN &&
+                     j.npebf <= 65536 && j.ngtg1 >= 1 && j.ngtg1 <= kMaxNG;
+  if (j.nelec > 1 && sizes) {
     int64_t nket = 0, most = 1;
     auto prims = [&](int64_t i) -> int64_t {
       if (!j.KPESTR || !j.KPEEND) return 1;
@@ -2042,7 +2045,9 @@ static size_t xchf_job_bytes(const neoxc_xchf_job& j, int64_t options) {
         nket += n;
         most = std::max(most, n);
       }
-    d += gam2_scratch_bound((int)ne, (int)np, (int)nket, (int)most, (int)j.ngtg1);
+    const int64_t cap = 1 << 28;   // (far beyond what fits)
+    d += gam2_scratch_bound((int)ne, (int)np, (int)std::min(nket, cap), (int)std::min(most, cap),
+                            (int)j.ngtg1);
   }
   if (j.nelec > 2) {
     d += e2 * e2 * e2 * p2 + gam3_aux_doubles((int)ne, (int)np) +
