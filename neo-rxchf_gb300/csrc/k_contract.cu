@@ -389,7 +389,7 @@ cudaError_t launch_eg3_partials(int ne, int np, long long ipjp0, long long nipjp
                                 const double* g3_slice, double* scratch, cudaStream_t s) {
   if (ne < 1 || ne > 20 || np < 1) return cudaErrorInvalidValue;
   double* part = scratch + rank3_weight_doubles(ne, 1) + (size_t)ipjp0 * ne * ne * ne;
-  return launch_rank3(ne, nipjp, 1, 1u, g3_slice, scratch, nullptr, nullptr, part, nullptr, s);
+  return launch_rank3_closed(ne, nipjp, g3_slice, scratch, part, s);
 }
 
 cudaError_t launch_eg3_reduce(int ne, int np, double* scratch, const double* DE, const double* DP,

@@ -10,11 +10,11 @@
 // densities:
 //   row[j] += sum_uv G(j,u,v) W0(u,v) + G(u,j,v) W1(u,v) + G(u,v,j) W2(u,v).
 // The weights are tabulated once per call (they serve every proton pair and
-// i1), so an element costs 3 FP64 FMAs a class instead of the 9 to 14 FP64
+// i1; see kFormNE for the smallest calls), so an element costs 3 FP64 FMAs a class instead of the 9 to 14 FP64
 // operations of forming the combinations.  FP64 issue (2 per SM and clock)
 // is still what bounds it: 3 FMAs take 4.4x the time of the element's 8
-// bytes from HBM.  A CTA owns (p, i1, i2) and walks i3, so one partial row
-// is written per (p, i1, i2).
+// bytes from HBM.  A CTA owns (p, i1, i2) and walks i3 or a share of it, so one
+// partial row is written per (p, i1, i2) and share.
 // Measured (one GB300, whole call): EG3IC1 at ne = 12, np = 8 (1.5 GB) 6.69 ms
 // with the combinations formed per ket tuple and a serial reduction, 1.12 ms
 // so (3 FMAs an element at the measured FP64 rate: 1.08 ms); open shell at
@@ -25,6 +25,18 @@ namespace neoxc {
 namespace {
 
 constexpr int kThreads = 256;
+
+// Open shell with few protons: a CTA per (p, i1, i2) that walks all of i3 leaves
+// most of the chip idle (np = 1: 16 CTAs at ne = 4, 100 at ne = 10), so the walk
+// is cut into shares until there are kFillCtas of them; up to kFormNE the CTAs
+// then form the weights themselves, for the table is one launch more.  Whole
+// calls (one GB300, us; the kernel without tables, one step per CTA / one share /
+// shares / shares that form the weights): ne = 4, np = 1 40 / 45 / 39 / 33;
+// ne = 6, np = 2 50 / 54 / 45 / 41; ne = 8, np = 1 46 / 60 / 43 / 39; ne = 10, np = 1
+// 74 / 76 / 54 / 54; ne = 12, np = 1 131 / 105 / 76 / 82.  Cut for 152 x 8 CTAs instead,
+// ne = 8, np = 2 takes 64 us for 56, ne = 12, np = 1 83 for 76.
+constexpr long long kFillCtas = 152 * 4;
+constexpr int kFormNE = 8;
 
 // x / d for x < 65536, 2 <= d <= 256, by one multiply-high
 struct DivN {
@@ -51,8 +63,34 @@ __global__ void weights_closed_kernel(int ne, const double* __restrict__ DE,
   }
 }
 
-// bit 0: the six-term set, bit 1: the two mixed pairs, bit 2: the 23 pair
-// (FAE_OMG3's LAA, LAB, LBB); class B exchanges the spins
+// Weights of the ket pair (u,v) of electrons (i2,i3) for one class with flags f
+// (bit 0: the six-term set, bit 1: the two mixed pairs, bit 2: the 23 pair;
+// FAE_OMG3's LAA, LAB, LBB); A, B: the class's densities of its own and of the
+// other spin
+__device__ __forceinline__ void open_weights(int ne, const double* __restrict__ A,
+                                             const double* __restrict__ B, unsigned f, int i2,
+                                             int i3, int u, int v, double* w) {
+  const double a2u = A[i2 + ne * u], a2v = A[i2 + ne * v], a3u = A[i3 + ne * u], a3v = A[i3 + ne * v];
+  const double b2u = B[i2 + ne * u], b2v = B[i2 + ne * v], b3u = B[i3 + ne * u], b3v = B[i3 + ne * v];
+  double w0 = 0.0, w1 = 0.0, w2 = 0.0;
+  if (f & 1u) {
+    const double x = a2u * a3v - a2v * a3u;
+    w0 += x;
+    w1 -= x;
+    w2 += x;
+  }
+  if (f & 2u) {
+    w0 += a2u * b3v + b2u * a3v;
+    w1 -= a2u * b3v;
+    w2 -= b2v * a3u;
+  }
+  if (f & 4u) w0 += b2u * b3v - b2v * b3u;
+  w[0] = w0;
+  w[1] = w1;
+  w[2] = w2;
+}
+
+// class B exchanges the spins
 __global__ void weights_open_kernel(int ne, const double* __restrict__ DA,
                                     const double* __restrict__ DB, unsigned fa, unsigned fb,
                                     double* __restrict__ W) {
@@ -63,39 +101,21 @@ __global__ void weights_open_kernel(int ne, const double* __restrict__ DA,
     const int c = t >= n4;
     const long long r = t - c * n4;
     const int uv = (int)(r % n2), i = (int)(r / n2);
-    const int u = uv / ne, v = uv - u * ne, i2 = i / ne, i3 = i - i2 * ne;
-    const double* A = c ? DB : DA;
-    const double* B = c ? DA : DB;
-    const unsigned f = c ? fb : fa;
-    const double a2u = A[i2 + ne * u], a2v = A[i2 + ne * v], a3u = A[i3 + ne * u], a3v = A[i3 + ne * v];
-    const double b2u = B[i2 + ne * u], b2v = B[i2 + ne * v], b3u = B[i3 + ne * u], b3v = B[i3 + ne * v];
-    double w0 = 0.0, w1 = 0.0, w2 = 0.0;
-    if (f & 1u) {
-      const double x = a2u * a3v - a2v * a3u;
-      w0 += x;
-      w1 -= x;
-      w2 += x;
-    }
-    if (f & 2u) {
-      w0 += a2u * b3v + b2u * a3v;
-      w1 -= a2u * b3v;
-      w2 -= b2v * a3u;
-    }
-    if (f & 4u) w0 += b2u * b3v - b2v * b3u;
-    double* o = W + (size_t)c * 3 * n4 + r;
-    o[0] = w0;
-    o[n4] = w1;
-    o[2 * n4] = w2;
+    double w[3];
+    open_weights(ne, c ? DB : DA, c ? DA : DB, c ? fb : fa, i / ne, i % ne, uv / ne, uv % ne, w);
+    for (int s = 0; s < 3; s++) W[((size_t)c * 3 + s) * n4 + r] = w[s];
   }
 }
 
 // NC classes; USED: bit c = class c has weights.  Threads (j, q): ket j of the
-// row, q strides the pairs (u,v).
+// row, q strides the pairs (u,v).  CTA y of a (p, i1, i2) takes its share of i3
+// and writes a partial row of its own.  W null (NC = 2): the weights are formed
+// here, of flags fa and fb.
 template <int NC, unsigned USED>
 __global__ void __launch_bounds__(kThreads)
 rank3_kernel(int ne, const double* __restrict__ G, const double* __restrict__ W,
-             const double* __restrict__ DA, const double* __restrict__ DB,
-             double* __restrict__ part, double* __restrict__ ppart) {
+             const double* __restrict__ DA, const double* __restrict__ DB, unsigned fa,
+             unsigned fb, double* __restrict__ part, double* __restrict__ ppart) {
   extern __shared__ double sm[];
   const int n2 = ne * ne, n3 = n2 * ne;
   const long long n4 = (long long)n2 * n2;
@@ -115,18 +135,30 @@ rank3_kernel(int ne, const double* __restrict__ G, const double* __restrict__ W,
   double acc[NC];
 #pragma unroll
   for (int c = 0; c < NC; c++) acc[c] = 0.0;
-  for (int i3 = 0; i3 < ne; i3++) {
+  const int i3end = ne * ((int)blockIdx.y + 1) / (int)gridDim.y;
+  for (int i3 = ne * (int)blockIdx.y / (int)gridDim.y; i3 < i3end; i3++) {
     __syncthreads();
     for (int k = threadIdx.x; k < n3; k += blockDim.x) {
       const int xy = (int)dv((unsigned)k), z = k - xy * ne;
       const int x = (int)dv((unsigned)xy), y = xy - x * ne;
       sG[x * pt0 + y * pt1 + z] = __ldg(g0 + (long long)x * n4 + (long long)y * n2 + i3 * ne + z);
     }
-    const double* w = W + (long long)(i2 * ne + i3) * n2;
+    bool formed = false;
+    if constexpr (NC == 2) formed = !W;
+    if (formed) {
+      for (int k = threadIdx.x; k < NC * n2; k += blockDim.x) {
+        const int c = k >= n2, uv = k - c * n2, u = (int)dv((unsigned)uv);
+        double w[3];
+        open_weights(ne, c ? DB : DA, c ? DA : DB, c ? fb : fa, i2, i3, u, uv - u * ne, w);
+        for (int s = 0; s < 3; s++) sW[(3 * c + s) * n2 + uv] = w[s];
+      }
+    } else {
+      const double* w = W + (long long)(i2 * ne + i3) * n2;
 #pragma unroll
-    for (int s = 0; s < 3 * NC; s++)
-      if (USED & (1u << (s / 3)))
-        for (int k = threadIdx.x; k < n2; k += blockDim.x) sW[s * n2 + k] = __ldg(w + s * n4 + k);
+      for (int s = 0; s < 3 * NC; s++)
+        if (USED & (1u << (s / 3)))
+          for (int k = threadIdx.x; k < n2; k += blockDim.x) sW[s * n2 + k] = __ldg(w + s * n4 + k);
+    }
     __syncthreads();
     if (q0 < lanes) {
 #pragma unroll 2
@@ -146,6 +178,7 @@ rank3_kernel(int ne, const double* __restrict__ G, const double* __restrict__ W,
     }
   }
   double row[NC];
+  const long long out = cta * gridDim.y + blockIdx.y;
 #pragma unroll
   for (int c = 0; c < NC; c++) {
     __syncthreads();
@@ -154,7 +187,7 @@ rank3_kernel(int ne, const double* __restrict__ G, const double* __restrict__ W,
     row[c] = 0.0;
     if ((int)threadIdx.x < ne) {
       for (int t = threadIdx.x; t < lanes * ne; t += ne) row[c] += sred[t];
-      part[(cta * NC + c) * ne + threadIdx.x] = row[c];
+      part[(out * NC + c) * ne + threadIdx.x] = row[c];
     }
   }
   if constexpr (NC == 2) {
@@ -167,14 +200,15 @@ rank3_kernel(int ne, const double* __restrict__ G, const double* __restrict__ W,
     if (threadIdx.x == 0) {
       double s = 0.0;
       for (int k = 0; k < ne; k++) s += sred[k];
-      ppart[cta * 2] = s;
+      ppart[out * 2] = s;
     }
   }
 }
 
 template <int NC, unsigned USED>
-cudaError_t launch_t(int ne, long long nipjp, const double* G, const double* W, const double* DA,
-                     const double* DB, double* part, double* ppart, cudaStream_t s) {
+cudaError_t launch_t(int ne, long long nipjp, int split, const double* G, const double* W,
+                     const double* DA, const double* DB, unsigned fa, unsigned fb, double* part,
+                     double* ppart, cudaStream_t s) {
   // no more groups of ne threads than ket pairs: small ne takes small CTAs
   int lanes = kThreads / ne;
   if (lanes > ne * ne) lanes = ne * ne;
@@ -185,7 +219,8 @@ cudaError_t launch_t(int ne, long long nipjp, const double* G, const double* W, 
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  rank3_kernel<NC, USED><<<(unsigned)(nipjp * ne * ne), bs, smem, s>>>(ne, G, W, DA, DB, part, ppart);
+  rank3_kernel<NC, USED><<<dim3((unsigned)(nipjp * ne * ne), split), bs, smem, s>>>(
+      ne, G, W, DA, DB, fa, fb, part, ppart);
   return cudaGetLastError();
 }
 
@@ -202,22 +237,34 @@ cudaError_t launch_rank3_weights_closed(int ne, const double* DE, double* W, cud
   return cudaGetLastError();
 }
 
-cudaError_t launch_rank3_weights_open(int ne, const double* DA, const double* DB, unsigned fa,
-                                      unsigned fb, double* W, cudaStream_t s) {
-  weights_open_kernel<<<wgrid(2LL * ne * ne * ne * ne), 256, 0, s>>>(ne, DA, DB, fa, fb, W);
-  return cudaGetLastError();
+int rank3_split(int ne, long long nipjp) {
+  const long long fill = kFillCtas / (nipjp * ne * ne);
+  return (int)(fill < 1 ? 1 : (fill > ne ? ne : fill));
 }
 
-cudaError_t launch_rank3(int ne, long long nipjp, int ncls, unsigned used, const double* G,
-                         const double* W, const double* DA, const double* DB, double* part,
-                         double* ppart, cudaStream_t s) {
-  if (ne < 1 || ne > 28 || nipjp < 1 || ncls < 1 || ncls > 2) return cudaErrorInvalidValue;
-  if (ncls == 1) return launch_t<1, 1u>(ne, nipjp, G, W, DA, DB, part, ppart, s);
-  switch (used & 3u) {
-    case 0: return launch_t<2, 0u>(ne, nipjp, G, W, DA, DB, part, ppart, s);
-    case 1: return launch_t<2, 1u>(ne, nipjp, G, W, DA, DB, part, ppart, s);
-    case 2: return launch_t<2, 2u>(ne, nipjp, G, W, DA, DB, part, ppart, s);
-    default: return launch_t<2, 3u>(ne, nipjp, G, W, DA, DB, part, ppart, s);
+cudaError_t launch_rank3_closed(int ne, long long nipjp, const double* G, const double* W,
+                                double* part, cudaStream_t s) {
+  if (ne < 1 || ne > 28 || nipjp < 1) return cudaErrorInvalidValue;
+  return launch_t<1, 1u>(ne, nipjp, 1, G, W, nullptr, nullptr, 0u, 0u, part, nullptr, s);
+}
+
+cudaError_t launch_rank3_open(int ne, long long nipjp, const double* G, const double* DA,
+                              const double* DB, unsigned fa, unsigned fb, double* W, double* part,
+                              double* ppart, cudaStream_t s) {
+  if (ne < 1 || ne > 28 || nipjp < 1) return cudaErrorInvalidValue;
+  const int n = rank3_split(ne, nipjp);
+  if (n > 1 && ne <= kFormNE) {
+    W = nullptr;
+  } else {
+    weights_open_kernel<<<wgrid(2LL * ne * ne * ne * ne), 256, 0, s>>>(ne, DA, DB, fa, fb, W);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  switch ((fa ? 1u : 0u) | (fb ? 2u : 0u)) {
+    case 0: return launch_t<2, 0u>(ne, nipjp, n, G, W, DA, DB, fa, fb, part, ppart, s);
+    case 1: return launch_t<2, 1u>(ne, nipjp, n, G, W, DA, DB, fa, fb, part, ppart, s);
+    case 2: return launch_t<2, 2u>(ne, nipjp, n, G, W, DA, DB, fa, fb, part, ppart, s);
+    default: return launch_t<2, 3u>(ne, nipjp, n, G, W, DA, DB, fa, fb, part, ppart, s);
   }
 }
 

@@ -449,9 +449,14 @@ cudaError_t launch_spin_kernel(int ne, int np, const double* G, const double* Gs
 
 }  // namespace
 
+// partial rows of an (ipjp, i1)
+static int spin_nsub(int K, int ne, int np) {
+  return K == 4 ? ne * ne : (K == 3 ? ne * rank3_split(ne, (long long)np * np) : ne);
+}
+
 size_t spin_scratch_doubles(int K, int ne, int np) {
   const int nacc = K == 2 ? 4 : 2;
-  const size_t ncta = (size_t)np * np * ne * ne * (K == 4 ? ne : 1);
+  const size_t ncta = (size_t)np * np * ne * spin_nsub(K, ne, np);
   return ncta * nacc * ne + ncta * 2 + (K == 3 ? rank3_weight_doubles(ne, 2) : 0);
 }
 
@@ -462,7 +467,8 @@ cudaError_t launch_spin_omg(int K, int ne, int np, const double* G, const double
   if (ne < 1 || ne > kSpinThreads || np < 1 || K < 2 || K > 4 || (K != 2 && Gs))
     return cudaErrorInvalidValue;
   const int nacc = (K == 2 && Gs) ? 4 : 2;
-  const size_t ncta = (size_t)np * np * ne * ne * (K == 4 ? ne : 1);
+  const int nsub = spin_nsub(K, ne, np);
+  const size_t ncta = (size_t)np * np * ne * nsub;
   double* part = scratch;
   double* ppart = scratch + ncta * (K == 2 ? 4 : 2) * ne;
   cudaError_t e;
@@ -473,15 +479,10 @@ cudaError_t launch_spin_omg(int K, int ne, int np, const double* G, const double
   else if (!fits)   // ranks 3 and 4 stage the whole ket block
     return cudaErrorInvalidValue;
   else if (K == 3) {
-    double* W = ppart + ncta * 2;
-    e = launch_rank3_weights_open(ne, DA, DB, fa, fb, W, s);
-    if (e != cudaSuccess) return e;
-    e = launch_rank3(ne, (long long)np * np, 2, (fa ? 1u : 0u) | (fb ? 2u : 0u), G, W, DA, DB,
-                     part, ppart, s);
+    e = launch_rank3_open(ne, (long long)np * np, G, DA, DB, fa, fb, ppart + ncta * 2, part, ppart, s);
   } else
     e = launch_spin_kernel<4, true>(ne, np, G, nullptr, DA, DB, fa, fb, part, ppart, s);
   if (e != cudaSuccess) return e;
-  const int nsub = K == 4 ? ne * ne : ne;
   const int ne_out = nacc * ne * ne;
   spin_reduce_e_kernel<<<(ne_out + 3) / 4, 128, 0, s>>>(ne, np, nacc, nsub, part, DP,
                                                         fe_out);

@@ -71,14 +71,17 @@ cudaError_t launch_fock_reduce(int ne, int np, int nsub, double* part,
 // (EG3IC1, one class) or open shell (two classes, flag bits as below).
 size_t rank3_weight_doubles(int ne, int ncls);
 cudaError_t launch_rank3_weights_closed(int ne, const double* DE, double* W, cudaStream_t s);
-cudaError_t launch_rank3_weights_open(int ne, const double* DA, const double* DB, unsigned fa,
-                                      unsigned fb, double* W, cudaStream_t s);
-// part[((p*ne + i1)*ne + i2)*ncls + c][j1]; with DA / DB (two classes) also
-// ppart[2*((p*ne + i1)*ne + i2)] = sum_j1 (DA row_A + DB row_B).  used: bit c
-// set when class c has any nonzero weight (else its rows are zeros).
-cudaError_t launch_rank3(int ne, long long nipjp, int ncls, unsigned used, const double* g3,
-                         const double* W, const double* DA, const double* DB, double* part,
-                         double* ppart, cudaStream_t s);
+// part[((p*ne + i1)*ne + i2)*ne + j1]
+cudaError_t launch_rank3_closed(int ne, long long nipjp, const double* g3, const double* W,
+                                double* part, cudaStream_t s);
+// The open-shell rows, with the weights (into W where they are tabulated, a
+// scratch of rank3_weight_doubles(ne, 2)): with n = rank3_split partial rows of
+// each, o = ((p*ne + i1)*ne + i2)*n + share, part[(o*2 + c)*ne + j1] and
+// ppart[2*o] = sum_j1 (DA row_A + DB row_B).
+int rank3_split(int ne, long long nipjp);
+cudaError_t launch_rank3_open(int ne, long long nipjp, const double* g3, const double* DA,
+                              const double* DB, unsigned fa, unsigned fb, double* W, double* part,
+                              double* ppart, cudaStream_t s);
 
 // ---- open-shell XCUHF contractions (k_spin.cu, xcuhf/xcuhf_omg*.f) ------
 // Rank K = 2 (GM2ICR, optional GM2sICR as Gs), 3 (GM3ICR) or 4 (OMG4_ICR).
