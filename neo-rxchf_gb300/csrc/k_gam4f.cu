@@ -1041,7 +1041,24 @@ cudaError_t launch_gam4_factored(int ne, int np, const double* gee,
   unsigned* counter = reinterpret_cast<unsigned*>(evals + p2);
   // Threads beyond the n^2 elements of a tile share its proton pairs, so small
   // n takes wide CTAs too (n = 12: seven groups of 144; 256 threads, one group
-  // walking all pairs, were 2.5x slower).
+  // walking all pairs, were 2.5x slower).  But one CTA of that width fills an SM,
+  // whose memory and FP64 phases then wait for each other, and from n = 33 its
+  // loops over the n^2 elements take a second, nearly empty turn: 640 threads
+  // there, so that two CTAs share an SM.  The backward kernel (128 registers)
+  // has two of 256 threads up to n = 48, by their shared memory, which pays
+  // while its sums over proton pairs, which want all 16 warps, are short: up to
+  // np = 5, where the narrow forward pays from n = 23 too.  Whole calls, us,
+  // (1024, 512), (640, 512), (640, 256) threads:
+  //   n = 24, np = 3   247  235  200     n = 33, np = 3  1093  992  840
+  //   n = 24, np = 10  472  404  443     n = 33, np = 6  1266 1092 1042
+  //   n = 28, np = 3   478  456  406     n = 36, np = 6  1666 1515 1577
+  //   n = 28, np = 10  823  856  834     n = 40, np = 1  2127 2052 1883
+  //   n = 30, np = 8   783  797  774     n = 40, np = 10 3594 3272 3326
+  //   n = 32, np = 5   882  844  789     n = 49, np = 3  5458 5222 5353
+  // The results do not depend on the choice.
+  const bool two = np <= 5 && n > 22 && n <= 48;
+  const int tforward = two || n > 32 ? 640 : kForwardThreads;
+  const int tbackward = two ? 256 : kBackwardThreads;
   const size_t tile = (size_t)n * (n | 1);
   const size_t smf = sizeof(double) * (3 * tile + kForwardThreads), smb = sizeof(double) * 6 * tile;
   for (const auto& k : {std::make_pair((const void*)gam4f_forward_kernel, smf),
@@ -1051,9 +1068,9 @@ cudaError_t launch_gam4_factored(int ne, int np, const double* gee,
                                            (int)k.second);
       if (e != cudaSuccess) return e;
     }
-  gam4f_forward_kernel<<<dim3(n2, 2), kForwardThreads, smf, s>>>(n, np, gee, g2s, DE, DP, HG, Gp, HE, Ep, counter);
+  gam4f_forward_kernel<<<dim3(n2, 2), tforward, smf, s>>>(n, np, gee, g2s, DE, DP, HG, Gp, HE, Ep, counter);
   traces_kernel<<<dim3(grid_for(6LL * n2, 128), 2), 128, 0, s>>>(n, Gp, Ep, PT);
-  gam4f_backward_kernel<<<n2, kBackwardThreads, smb, s>>>(n, np, g2s, DE, HG, Gp, HE, Ep, PT, epart, fpart);
+  gam4f_backward_kernel<<<n2, tbackward, smb, s>>>(n, np, g2s, DE, HG, Gp, HE, Ep, PT, epart, fpart);
   const int ne_ctas = (n2 + 31) / 32;
   gam4f_reduce_kernel<<<ne_ctas + (int)((p2 + 31) / 32), 1024, 0, s>>>(
       n, np, ne_ctas, epart, fpart, DP, accumulate, focke, fockp, evals, counter, E);
