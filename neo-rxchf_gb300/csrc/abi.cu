@@ -363,7 +363,8 @@ int build_gam2(const DevSystem& d, int rx, double* x1, double* x2, cudaStream_t 
 int build_gam3_aux(const DevSystem& d, double* aux, cudaStream_t s, const double* gee_in = nullptr,
                    const double* hc_in = nullptr, const double* w3_in = nullptr) {
   DBuf scr;
-  RC(dalloc(scr, sizeof(double) * gam2_scratch_doubles(d, 1, d.npbf * (d.npbf + 1) / 2), s));
+  RC(dalloc(scr, sizeof(double) * gam3_factors_scratch(d.nebf, d.npbf, d.g3_nket, d.g3_max_prim,
+                                                       d.ngtg, w3_in != nullptr), s));
   CU(launch_gam3_aux(d, aux, scr.as<double>(), s, gee_in, hc_in, w3_in));
   return NEOXC_OK;
 }
@@ -2027,9 +2028,10 @@ static size_t xchf_job_bytes(const neoxc_xchf_job& j, int64_t options) {
   const size_t e2 = ne * ne, p2 = np * np;
   size_t d = 4 * e2 + 4 * p2 + 3 * e2 * p2 + e2 * e2 + 32 * (e2 + p2);
   if (j.nelec > 1) d += 2 * e2 * e2 * p2 + eg2_partial_doubles((int)ne, (int)np);
-  // the gam_2 build's scratch, for sizes that the solve will not refuse:
-  // primitive pairs of the canonical pairs (a range that stage_system will
-  // refuse counts as one primitive)
+  // the pair records and the gam_2 build's scratch (the gam_3 factors take
+  // less), for sizes that the solve will not refuse: primitive pairs of the
+  // canonical pairs (a range that stage_system will refuse counts as one
+  // primitive)
   const bool sizes = j.nebf >= 1 && j.nebf <= kScfMaxN && j.npbf >= 1 && j.npbf <= kScfMaxN &&
                      j.npebf <= 65536 && j.ngtg1 >= 1 && j.ngtg1 <= kMaxNG;
   if (j.nelec > 1 && sizes) {
@@ -2047,7 +2049,9 @@ static size_t xchf_job_bytes(const neoxc_xchf_job& j, int64_t options) {
       }
     const int64_t cap = 1 << 28;   // (far beyond what fits)
     d += gam2_scratch_bound((int)ne, (int)np, (int)std::min(nket, cap), (int)std::min(most, cap),
-                            (int)j.ngtg1);
+                            (int)j.ngtg1) +
+         g3_record_doubles((int)std::min(nket, cap), (int)np) +
+         g3_gradient_doubles((int)std::min(nket, cap), (int)np);
   }
   if (j.nelec > 2) {
     d += e2 * e2 * e2 * p2 + gam3_aux_doubles((int)ne, (int)np) +

@@ -531,6 +531,11 @@ size_t gam2_scratch_bound(int ne, int np, int nket, int max_prim, int ng) {
   return p.fac + p.per * (size_t)p.chunk;
 }
 
+size_t gam3_factors_scratch(int ne, int np, int nket, int max_prim, int ng, bool w3_given) {
+  const Plan p = make_plan(ne, np, nket, max_prim, ng, true, np * (np + 1) / 2);
+  return w3_given ? p.fac : p.fac + p.per * (size_t)p.chunk;
+}
+
 cudaError_t launch_gam2_prepare(const DevSystem& S, double* scratch, cudaStream_t s) {
   if (S.nebf < 1 || S.npbf < 1 || !S.g3i || !S.g3rec || !S.g3grad) return cudaErrorInvalidValue;
   const int nPe = S.nebf * (S.nebf + 1) / 2, nPp = S.npbf * (S.npbf + 1) / 2;

@@ -234,7 +234,9 @@ size_t gam3_r4_doubles(int ne, int np);
 // gee_in / hc_in (optional, device): GAM_ee and Hcore already built by the
 // caller (C-order [i][j][k][l] and [i][j]); copied instead of recomputed.
 // w3_in: GM2sICR, which is W3 (the overlaps of the same geminal pairs).
-// scratch: gam2_scratch_doubles(sys, 1, npbf(npbf+1)/2).
+// scratch: gam3_factors_scratch of the system's sizes (with w3_in no more than
+// the gam_2 build of an XCHF solve has taken and given back before).
+size_t gam3_factors_scratch(int ne, int np, int nket, int max_prim, int ng, bool w3_given);
 cudaError_t launch_gam3_aux(const DevSystem& sys, double* aux, double* scratch, cudaStream_t s,
                             const double* gee_in = nullptr, const double* hc_in = nullptr,
                             const double* w3_in = nullptr);
