@@ -528,8 +528,11 @@ __device__ __forceinline__ double warp_sum4(double v0, double v1, double v2, dou
 }
 
 // grid n^2: tile (a, c) of dE/dG', dE/dE' -> epart[(a,c)][x*n + b] and
-// fpart[p][(a,c)] = sum_bd GAM_2s(p; ab; cd) W(ab; cd).
+// fpart[p][(a,c)] = sum_bd GAM_2s(p; ab; cd) W(ab; cd).  LEAN: three tiles of
+// shared memory for six; DE, H_G and H_E are read from memory, an element at a
+// time for all lanes of a warp, and epart is [(a,c)][b*n + x].
 constexpr int kBackwardThreads = 512;
+template <bool LEAN>
 __global__ void __launch_bounds__(kBackwardThreads)
 gam4f_backward_kernel(int n, int np, const double* __restrict__ g2s,
                       const double* __restrict__ DE, const double* __restrict__ HG,
@@ -539,11 +542,11 @@ gam4f_backward_kernel(int n, int np, const double* __restrict__ g2s,
   extern __shared__ double sm[];
   const int n2 = n * n, np2 = np * np, ld = n | 1, tl = n * ld;
   const long long n4 = (long long)n2 * n2;
-  double* sDE = sm;
-  double* sW = sDE + tl;       // Wp(a,x,c,y)
+  double* sW = sm;             // Wp(a,x,c,y)
   double* sX = sW + tl;        // Wp(a,x,c,y) + Wp(c,y,a,x)
   double* sY = sX + tl;        // the same of Vp
-  double* sHG = sY + tl;       // [b][y]
+  double* sDE = sY + tl;
+  double* sHG = sDE + tl;      // [b][y]
   double* sHE = sHG + tl;
   __shared__ double sST[8];
   const int a = blockIdx.x / n, c = blockIdx.x - a * n;
@@ -559,12 +562,13 @@ gam4f_backward_kernel(int n, int np, const double* __restrict__ g2s,
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if (lane == 0) sST[(warp / 3) * 4 + warp % 3] = s;
   }
-  for (int e = threadIdx.x; e < n2; e += blockDim.x) {
-    const int b = e / n, d = e - b * n;
-    sDE[b * ld + d] = DE[e];
-    sHG[b * ld + d] = HG[base + (long long)b * n2 + d];
-    sHE[b * ld + d] = HE[base + (long long)b * n2 + d];
-  }
+  if (!LEAN)
+    for (int e = threadIdx.x; e < n2; e += blockDim.x) {
+      const int b = e / n, d = e - b * n;
+      sDE[b * ld + d] = DE[e];
+      sHG[b * ld + d] = HG[base + (long long)b * n2 + d];
+      sHE[b * ld + d] = HE[base + (long long)b * n2 + d];
+    }
   __syncthreads();
   for (int e = threadIdx.x; e < n2; e += blockDim.x) {
     const int x = e / n, y = e - x * n;
@@ -589,21 +593,41 @@ gam4f_backward_kernel(int n, int np, const double* __restrict__ g2s,
   __syncthreads();
   // focke(x,b) of this tile: sum_y X[x][y] HG[b][y] + Y[x][y] HE[b][y]
   for (int e = threadIdx.x; e < n2; e += blockDim.x) {
-    const int x = e / n, b = e - x * n;
+    const int q = e / n, r = e - q * n, x = LEAN ? r : q, b = LEAN ? q : r;
+    const double* hg = LEAN ? HG + base + (long long)b * n2 : sHG + b * ld;
+    const double* he = LEAN ? HE + base + (long long)b * n2 : sHE + b * ld;
     double s = 0.0, t = 0.0;
 #pragma unroll 4
     for (int y = 0; y < n; y++) {
-      s = fma(sX[x * ld + y], sHG[b * ld + y], s);
-      t = fma(sY[x * ld + y], sHE[b * ld + y], t);
+      s = fma(sX[x * ld + y], LEAN ? __ldg(hg + y) : hg[y], s);
+      t = fma(sY[x * ld + y], LEAN ? __ldg(he + y) : he[y], t);
     }
     epart[(long long)blockIdx.x * n2 + e] = s + t;
   }
   __syncthreads();
   // W[b][d] = sum_xy Wp[x][y] DE(x,b) DE(y,d), through Ht[x][d] (in sX) into sY;
   // DE(y,d) at [d][y], DE(x,b) at [b][x]
-  tile_mul<false, true>(n, ld, sW, sDE, sX);
-  __syncthreads();
-  tile_mul<false, false>(n, ld, sDE, sX, sY);
+  if (LEAN) {
+    for (int e = threadIdx.x; e < n2; e += blockDim.x) {
+      const int d = e / n, x = e - d * n;
+      double s = 0.0;
+#pragma unroll 4
+      for (int y = 0; y < n; y++) s = fma(sW[x * ld + y], __ldg(DE + d * n + y), s);
+      sX[x * ld + d] = s;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < n2; e += blockDim.x) {
+      const int b = e / n, d = e - b * n;
+      double s = 0.0;
+#pragma unroll 4
+      for (int x = 0; x < n; x++) s = fma(__ldg(DE + b * n + x), sX[x * ld + d], s);
+      sY[b * ld + d] = s;
+    }
+  } else {
+    tile_mul<false, true>(n, ld, sW, sDE, sX);
+    __syncthreads();
+    tile_mul<false, false>(n, ld, sDE, sX, sY);
+  }
   __syncthreads();
   // four proton pairs of a warp at a time
   const int nw = blockDim.x >> 5;
@@ -623,10 +647,10 @@ gam4f_backward_kernel(int n, int np, const double* __restrict__ g2s,
   }
 }
 
-// CTAs [0, ne_ctas): 32 focke elements each, 32 warps sharing the n^2 tiles; the
+// lean: the layout of epart.  CTAs [0, ne_ctas): 32 focke elements each, 32 warps sharing the n^2 tiles; the
 // others: 32 proton pairs each.  The last of those to finish adds E up.
 __global__ void __launch_bounds__(1024)
-gam4f_reduce_kernel(int n, int np, int ne_ctas, const double* __restrict__ epart,
+gam4f_reduce_kernel(int n, int np, int ne_ctas, bool lean, const double* __restrict__ epart,
                     const double* __restrict__ fpart, const double* __restrict__ DP,
                     int accumulate, double* __restrict__ focke, double* __restrict__ fockp,
                     double* __restrict__ evals, unsigned* __restrict__ counter,
@@ -647,7 +671,7 @@ gam4f_reduce_kernel(int n, int np, int ne_ctas, const double* __restrict__ epart
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     const int q = blockIdx.x * 32 + warp;
     if (lane == 0 && q < n2) {
-      const int f = q / n + n * (q % n);   // focke(x,b), column-major
+      const int f = lean ? q : q / n + n * (q % n);   // focke(x,b), column-major
       focke[f] = accumulate ? focke[f] + v : v;
     }
     return;
@@ -1041,28 +1065,33 @@ cudaError_t launch_gam4_factored(int ne, int np, const double* gee,
   unsigned* counter = reinterpret_cast<unsigned*>(evals + p2);
   // Threads beyond the n^2 elements of a tile share its proton pairs, so small
   // n takes wide CTAs too (n = 12: seven groups of 144; 256 threads, one group
-  // walking all pairs, were 2.5x slower).  But one CTA of that width fills an SM,
-  // whose memory and FP64 phases then wait for each other, and from n = 33 its
-  // loops over the n^2 elements take a second, nearly empty turn: 640 threads
-  // there, so that two CTAs share an SM.  The backward kernel (128 registers)
-  // has two of 256 threads up to n = 48, by their shared memory, which pays
-  // while its sums over proton pairs, which want all 16 warps, are short: up to
-  // np = 5, where the narrow forward pays from n = 23 too.  Whole calls, us,
-  // (1024, 512), (640, 512), (640, 256) threads:
-  //   n = 24, np = 3   247  235  200     n = 33, np = 3  1093  992  840
-  //   n = 24, np = 10  472  404  443     n = 33, np = 6  1266 1092 1042
-  //   n = 28, np = 3   478  456  406     n = 36, np = 6  1666 1515 1577
-  //   n = 28, np = 10  823  856  834     n = 40, np = 1  2127 2052 1883
-  //   n = 30, np = 8   783  797  774     n = 40, np = 10 3594 3272 3326
-  //   n = 32, np = 5   882  844  789     n = 49, np = 3  5458 5222 5353
-  // The results do not depend on the choice.
-  const bool two = np <= 5 && n > 22 && n <= 48;
-  const int tforward = two || n > 32 ? 640 : kForwardThreads;
-  const int tbackward = two ? 256 : kBackwardThreads;
+  // walking all pairs, were 2.5x slower).  Beyond n = 22 there is one group, and
+  // one wide CTA fills an SM, whose memory and FP64 phases then wait for each
+  // other (and from n = 33 its loops over the n^2 elements take a second, nearly
+  // empty turn): CTAs of which two share an SM are the better ones.  The forward
+  // kernel has them with 640 threads; the backward one, by its 128 registers,
+  // with 256, and with the three tiles of LEAN up to n = 64 (six: n = 48).  That
+  // pays while its sums over proton pairs, which want all 16 warps, are short,
+  // up to np = 5.  Whole calls, us, threads (1024, 512) with six tiles / (640, 256)
+  // with six / (640, 512) LEAN / (640, 256) LEAN:
+  //   n = 24, np = 1   244  192  235  194    n = 40, np = 1  2129 1886 2071 1880
+  //   n = 24, np = 10  473  377  409  377    n = 40, np = 6  2546 2403 2385 2392
+  //   n = 30, np = 4   677  567  646  561    n = 40, np = 10 3595 3327 3272 3302
+  //   n = 30, np = 10  997 1010 1027 1000    n = 50, np = 2  5992 5901 5832 5374
+  //   n = 33, np = 1   912  759  863  759    n = 60, np = 1 13573 13458 12933 12069
+  //   n = 33, np = 10 1882 1471 1534 1461    n = 60, np = 10 20268 23020 18470 18396
+  //   n = 36, np = 6  1670 1580 1511 1567    n = 64, np = 4 19749 19432 18067 17967
+  // Six tiles stay below n = 23 (n = 12, np = 8: 45.6 us, LEAN 47.7).  The results
+  // do not depend on the choice.
+  const bool lean = n > 22, few = lean && np <= 5;
+  const int tforward = few || n > 32 ? 640 : kForwardThreads;
+  const int tbackward = few ? 256 : kBackwardThreads;
+  const auto backward = lean ? gam4f_backward_kernel<true> : gam4f_backward_kernel<false>;
   const size_t tile = (size_t)n * (n | 1);
-  const size_t smf = sizeof(double) * (3 * tile + kForwardThreads), smb = sizeof(double) * 6 * tile;
+  const size_t smf = sizeof(double) * (3 * tile + kForwardThreads);
+  const size_t smb = sizeof(double) * (lean ? 3 : 6) * tile;
   for (const auto& k : {std::make_pair((const void*)gam4f_forward_kernel, smf),
-                        std::make_pair((const void*)gam4f_backward_kernel, smb)})
+                        std::make_pair((const void*)backward, smb)})
     if (k.second > 48 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(k.first, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)k.second);
@@ -1070,10 +1099,10 @@ cudaError_t launch_gam4_factored(int ne, int np, const double* gee,
     }
   gam4f_forward_kernel<<<dim3(n2, 2), tforward, smf, s>>>(n, np, gee, g2s, DE, DP, HG, Gp, HE, Ep, counter);
   traces_kernel<<<dim3(grid_for(6LL * n2, 128), 2), 128, 0, s>>>(n, Gp, Ep, PT);
-  gam4f_backward_kernel<<<n2, tbackward, smb, s>>>(n, np, g2s, DE, HG, Gp, HE, Ep, PT, epart, fpart);
+  backward<<<n2, tbackward, smb, s>>>(n, np, g2s, DE, HG, Gp, HE, Ep, PT, epart, fpart);
   const int ne_ctas = (n2 + 31) / 32;
   gam4f_reduce_kernel<<<ne_ctas + (int)((p2 + 31) / 32), 1024, 0, s>>>(
-      n, np, ne_ctas, epart, fpart, DP, accumulate, focke, fockp, evals, counter, E);
+      n, np, ne_ctas, lean, epart, fpart, DP, accumulate, focke, fockp, evals, counter, E);
   return cudaGetLastError();
 }
 
