@@ -109,10 +109,12 @@ __global__ void weights_open_kernel(int ne, const double* __restrict__ DA,
 
 // NC classes; USED: bit c = class c has weights.  Threads (j, q): ket j of the
 // row, q strides the pairs (u,v).  CTA y of a (p, i1, i2) takes its share of i3
-// and writes a partial row of its own.  W null (NC = 2): the weights are formed
-// here, of flags fa and fb.
-template <int NC, unsigned USED>
-__global__ void __launch_bounds__(kThreads)
+// and writes a partial row of its own.  FORM (NC = 2): the weights are formed
+// here, of flags fa and fb, and W is not read.  Eight CTAs an SM, six with FORM:
+// with 40 registers for 32, ne = 12, np = 4 took 611 us for 601; with all that
+// FORM would take, ne = 7, np = 2 57 for 48.
+template <int NC, unsigned USED, bool FORM>
+__global__ void __launch_bounds__(kThreads, FORM ? 6 : 8)
 rank3_kernel(int ne, const double* __restrict__ G, const double* __restrict__ W,
              const double* __restrict__ DA, const double* __restrict__ DB, unsigned fa,
              unsigned fb, double* __restrict__ part, double* __restrict__ ppart) {
@@ -143,9 +145,7 @@ rank3_kernel(int ne, const double* __restrict__ G, const double* __restrict__ W,
       const int x = (int)dv((unsigned)xy), y = xy - x * ne;
       sG[x * pt0 + y * pt1 + z] = __ldg(g0 + (long long)x * n4 + (long long)y * n2 + i3 * ne + z);
     }
-    bool formed = false;
-    if constexpr (NC == 2) formed = !W;
-    if (formed) {
+    if constexpr (FORM) {
       for (int k = threadIdx.x; k < NC * n2; k += blockDim.x) {
         const int c = k >= n2, uv = k - c * n2, u = (int)dv((unsigned)uv);
         double w[3];
@@ -205,7 +205,7 @@ rank3_kernel(int ne, const double* __restrict__ G, const double* __restrict__ W,
   }
 }
 
-template <int NC, unsigned USED>
+template <int NC, unsigned USED, bool FORM>
 cudaError_t launch_t(int ne, long long nipjp, int split, const double* G, const double* W,
                      const double* DA, const double* DB, unsigned fa, unsigned fb, double* part,
                      double* ppart, cudaStream_t s) {
@@ -215,11 +215,11 @@ cudaError_t launch_t(int ne, long long nipjp, int split, const double* G, const 
   const int bs = lanes * ne, pt1 = ne | 1, pt0 = (pt1 * ne) | 1;
   const size_t smem = sizeof(double) * ((size_t)pt0 * ne + 3 * NC * (size_t)ne * ne + bs);
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(rank3_kernel<NC, USED>,
+    cudaError_t e = cudaFuncSetAttribute(rank3_kernel<NC, USED, FORM>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  rank3_kernel<NC, USED><<<dim3((unsigned)(nipjp * ne * ne), split), bs, smem, s>>>(
+  rank3_kernel<NC, USED, FORM><<<dim3((unsigned)(nipjp * ne * ne), split), bs, smem, s>>>(
       ne, G, W, DA, DB, fa, fb, part, ppart);
   return cudaGetLastError();
 }
@@ -245,7 +245,7 @@ int rank3_split(int ne, long long nipjp) {
 cudaError_t launch_rank3_closed(int ne, long long nipjp, const double* G, const double* W,
                                 double* part, cudaStream_t s) {
   if (ne < 1 || ne > 28 || nipjp < 1) return cudaErrorInvalidValue;
-  return launch_t<1, 1u>(ne, nipjp, 1, G, W, nullptr, nullptr, 0u, 0u, part, nullptr, s);
+  return launch_t<1, 1u, false>(ne, nipjp, 1, G, W, nullptr, nullptr, 0u, 0u, part, nullptr, s);
 }
 
 cudaError_t launch_rank3_open(int ne, long long nipjp, const double* G, const double* DA,
@@ -253,19 +253,15 @@ cudaError_t launch_rank3_open(int ne, long long nipjp, const double* G, const do
                               double* ppart, cudaStream_t s) {
   if (ne < 1 || ne > 28 || nipjp < 1) return cudaErrorInvalidValue;
   const int n = rank3_split(ne, nipjp);
-  if (n > 1 && ne <= kFormNE) {
-    W = nullptr;
-  } else {
-    weights_open_kernel<<<wgrid(2LL * ne * ne * ne * ne), 256, 0, s>>>(ne, DA, DB, fa, fb, W);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  switch ((fa ? 1u : 0u) | (fb ? 2u : 0u)) {
-    case 0: return launch_t<2, 0u>(ne, nipjp, n, G, W, DA, DB, fa, fb, part, ppart, s);
-    case 1: return launch_t<2, 1u>(ne, nipjp, n, G, W, DA, DB, fa, fb, part, ppart, s);
-    case 2: return launch_t<2, 2u>(ne, nipjp, n, G, W, DA, DB, fa, fb, part, ppart, s);
-    default: return launch_t<2, 3u>(ne, nipjp, n, G, W, DA, DB, fa, fb, part, ppart, s);
-  }
+  const unsigned used = (fa ? 1u : 0u) | (fb ? 2u : 0u);
+#define R3(U, F) launch_t<2, U, F>(ne, nipjp, n, G, W, DA, DB, fa, fb, part, ppart, s)
+  if (n > 1 && ne <= kFormNE)
+    return used == 3u ? R3(3u, true) : used == 2u ? R3(2u, true) : used == 1u ? R3(1u, true) : R3(0u, true);
+  weights_open_kernel<<<wgrid(2LL * ne * ne * ne * ne), 256, 0, s>>>(ne, DA, DB, fa, fb, W);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  return used == 3u ? R3(3u, false) : used == 2u ? R3(2u, false) : used == 1u ? R3(1u, false) : R3(0u, false);
+#undef R3
 }
 
 }  // namespace neoxc
