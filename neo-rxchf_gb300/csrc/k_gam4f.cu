@@ -542,11 +542,11 @@ gam4f_backward_kernel(int n, int np, const double* __restrict__ g2s,
   extern __shared__ double sm[];
   const int n2 = n * n, np2 = np * np, ld = n | 1, tl = n * ld;
   const long long n4 = (long long)n2 * n2;
-  double* sW = sm;             // Wp(a,x,c,y)
+  double* sDE = sm;
+  double* sW = LEAN ? sm : sDE + tl;   // Wp(a,x,c,y)
   double* sX = sW + tl;        // Wp(a,x,c,y) + Wp(c,y,a,x)
   double* sY = sX + tl;        // the same of Vp
-  double* sDE = sY + tl;
-  double* sHG = sDE + tl;      // [b][y]
+  double* sHG = sY + tl;       // [b][y]
   double* sHE = sHG + tl;
   __shared__ double sST[8];
   const int a = blockIdx.x / n, c = blockIdx.x - a * n;
