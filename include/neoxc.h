@@ -79,7 +79,12 @@ int neoxc_calc_gam_ee(int64_t nebf, int64_t npebf, int64_t ngee,
                       const double* ELCEX, const int64_t* ELCAM,
                       const double* ELCBFC, double* GAM_ee);
 
-/* gam2_IC1_OMP.f:2-212 GAM2_IC1 -> GM2ICR, GM2sICR (pair-symmetrised) */
+/* gam2_IC1_OMP.f:2-212 GAM2_IC1 -> GM2ICR, GM2sICR (pair-symmetrised).
+ * Every gam_2 build (this one, RXCHF-ne's, the direct one, the solves') takes
+ * device scratch beside its tensors, in chunks of proton pairs of about
+ * 256 MiB; one proton pair is the least: about 24 q r bytes with
+ * q = nebf (nebf + 1) / 2 and r the primitive pairs of those q pairs (three
+ * primitives each: 160 MB at nebf = 40, 2.3 GB at nebf = 80). */
 int neoxc_gam2_ic1(int64_t Nchunks, int64_t nebf, int64_t npebf, int64_t npbf,
                    int64_t ng2, int64_t ng2prm, int64_t nat, int64_t ngtg1,
                    double pmass, const double* cat, const double* zan,
@@ -104,7 +109,8 @@ int neoxc_gam3_ic1(int64_t Nchunks, int64_t nebf, int64_t npebf, int64_t npbf,
                    const double* NUCBFC, double* GM3ICR);
 /* GAM3_IC1 with options (no reference counterpart for the options):
  * NEOXC_SCF_MIXED computes the four-particle terms with FP32 tables and
- * FP64 Boys function, seeds and sums; NEOXC_SCF_SCREEN skips primitive
+ * FP64 Boys function, seeds and sums (what that gains and costs: at
+ * neoxc_xchf_scf below); NEOXC_SCF_SCREEN skips primitive
  * (bra, ket) pairs whose Schwarz-type estimate is below 1e-12.  seconds
  * (optional) receives the device time of the build (CUDA events, the copy
  * to GM3ICR excluded). */
@@ -417,6 +423,10 @@ int neoxc_dev_gam4_fock_factored_tc(void* stream, int64_t ne, int64_t np,
  * NEOXC_SCF_MIXED (no reference counterpart) evaluates the gam_3 primitive
  * integrals with FP32 McMurchie-Davidson recursions (FP64 Boys function,
  * FP64 sums over primitives and geminal pairs); everything else stays FP64.
+ * It gains little: about 7 % of a solve with s functions only, nothing to 10 %
+ * with p functions of one or two primitives, and with longer contractions it
+ * is slower than FP64 (nebf = 12 s/p of 3 primitives, npbf = 8: 52 s for 47),
+ * at 1e-7 Eh of error: measure before choosing it.
  * NEOXC_SCF_MIXED_GAM2 is accepted and changes nothing: the gam_2 build is
  * FP64 (faster than its earlier FP32-first form; gam_1 is FP64 as well).
  *   DE (in: initial electronic density, e.g. from guessCE; out: converged)

@@ -5,7 +5,7 @@
 // XC1_G4_MD.f:796-1125 (G4_MD_xgVeeg), :1559-1978 (G4_MD_xgVepg).
 //
 // xcalc_GAM3_MD's integrand is gVEE + gHEg + gVEEg1/2 + 2 gVEEg2 (:964).
-// Its separable terms are contracted once per system in k_md.cu (W1 x
+// Its separable terms are contracted once per system in k_gam2.cu (W1 x
 // GAM_ee + W3 x Hcore); what remains per primitive 8-tuple is
 //   g4part = sum_kl b_k b_l (2 G4Vee(e1,e2,e3,p) - G4Vep(e1,e2,e3,p))
 // (:846, :930).  Two structural facts make it cheap on the GPU:

@@ -1,11 +1,16 @@
 // md_math_body.cuh -- McMurchie-Davidson geminal integrals, written for the
 // GPU and usable as plain C++ (every function is __host__ __device__).
-// Included by md_math.cuh (real = double, namespace md: the FP64 path that
-// matches the reference) and md_math32.cuh (real = float, namespace md32:
-// the mixed-precision path).  In both instances the Boys function, the
-// seeds (-alpha)^m F_m(T) and the final Hermite-Coulomb sum are FP64; md32's
-// Gaussian-product set-up, Hermite and derivative tables and the Hermite
-// folds are FP32 (the mixed gam_3 build).
+// Included by md_math.cuh (real = double, namespace md: the precision of the
+// reference) and md_math32.cuh (real = float, namespace md32).  In both
+// instances the Boys function, the seeds (-alpha)^m F_m(T) and the final
+// Hermite-Coulomb sum are FP64; md32's Gaussian-product set-up, Hermite and
+// derivative tables and the Hermite folds are FP32.
+// The kernels take from here the Boys function and its sums, the Gaussian
+// products, Hermite coefficients and Gaussian derivatives, and the two-centre
+// overlap, kinetic and nuclear attraction integrals (gfke, gfvec, ovl1d); the
+// geminal integrals that they evaluate are those of g2_threebody.cuh and
+// g3_fatbra.cuh.  The element-wise geminal integrals below (g2_*, g3_*, g4_*,
+// gfvee, pgike1) and all of md32 are what the host checks compare those with.
 //
 // The reference evaluates each primitive integral as a 9- or 12-deep loop
 // over Hermite indices, and inside every iteration re-derives the Boys'
@@ -696,54 +701,6 @@ NX_BIG real g3_vxc(const G3& s, const real* C) {
   }
   const real alpha = tv3, T = alpha * R2;
   return g3_coulomb(s, C0, C3, bf, bg, bh, T, alpha, Rv);
-}
-
-// G3_MD_xgVxCg for nat classical centres at once (cat: 3 x nat bohr):
-// the Hermite vectors W_d do not depend on the attracting centre, so they
-// are folded once and only the Coulomb sum runs per centre; out[ia] equals
-// g3_vxc(s, C_ia).
-NX_BIG void g3_vxc_multi(const G3& s, int nat, const double* cat, real* out) {
-  const real s1 = s.S1, s2 = s.S2, g = s.gam12;
-  const real p1 = s.pr[0].p, p2 = s.pr[1].p, c1 = s.C1, c2 = s.C2;
-  const real tv1 = s2 + g;
-  const real tv2 = s1 * s2 + s1 * g + s2 * g;
-  const real tv3 = tv2 / tv1;
-  const real x = kPiT / tv1;
-  const real C3 = sqrt(x * x * x) * (R_(2.0) * kPiT / tv3);
-  const real C0 = pow(kPiT / s.xsum, R_(1.5));
-  const real bf = (s1 * s2 + s1 * g) / tv2 * (p1 / (p1 + c1));
-  const real bg = (s2 * g) / tv2 * (p2 / (p2 + c2));
-  const real bh = (s1 * s2 + s1 * g) / tv2 * (c1 / (p1 + c1)) +
-                    (s2 * g) / tv2 * (c2 / (p2 + c2));
-  const real alpha = tv3;
-  bool all_s = true;
-  for (int i = 0; i < 3; i++)
-    for (int d = 0; d < 3; d++) all_s = all_s && s.T[i][d] == 0;
-  real W[3][LTOT + 1];
-  int n[3] = {0, 0, 0};
-  real w = R_(1.0);
-  if (all_s) {
-    for (int d = 0; d < 3; d++) {
-      const real wd = ((s.pr[0].K[d] * s.pr[1].K[d]) * s.pr[2].K[d]) * s.D[d][0];
-      w = d == 0 ? wd : w * wd;
-    }
-  } else {
-    for (int d = 0; d < 3; d++) g3_wvec(s, d, bf, bg, bh, W[d], &n[d]);
-  }
-  for (int ia = 0; ia < nat; ia++) {
-    real Rv[3], R2 = R_(0.0);
-    for (int d = 0; d < 3; d++) {
-      real sm = ((s1 * s2 + s1 * g) / tv2) * s.Sm1[d] + ((s2 * g) / tv2) * s.Sm2[d];
-      Rv[d] = sm - (real)cat[3 * ia + d];
-      R2 += Rv[d] * Rv[d];
-    }
-    const real T = alpha * R2;
-    if (all_s) {
-      out[ia] = C0 * C3 * (w * (real)boys_sum(0, T, 0.0, [](int) { return 1.0; }));
-    } else {
-      out[ia] = C0 * C3 * contract_wr(W[0], n[0], W[1], n[1], W[2], n[2], T, alpha, Rv);
-    }
-  }
 }
 
 // G3_MD_xgVeeg (XC1_G3_MD.f:1376-1675): 1/|r1 - r2|
