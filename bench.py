@@ -404,7 +404,7 @@ def open_shell_section(neoxc, torch, dev, stream):
     the device; NAE = NBE = 2.  The tensor is read once (algorithmic bytes,
     reported against HBM), but the bound is the FP64 pipe: ncu shows 90 %
     FP64-pipe activity and 3.5 % DRAM for rank 3
-    (profiles/spin_kernel_rank3_open_shell.md)."""
+    (profiles/kernels_ncu.md)."""
     f64 = torch.float64
     peak = read_hbm_peak()
     out = {"api": "neoxc_dev_xcuhf_omg (device)", "peak_gbs": peak}

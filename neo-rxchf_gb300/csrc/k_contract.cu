@@ -172,7 +172,7 @@ __global__ void eg2_kernel(int ne, int np, const double* __restrict__ DE,
 // dots over its lanes by a transposing butterfly (one addition per row instead
 // of five).  Measured there: 7.75 ms with a CTA of 256 threads per row and a
 // tree per row, 6.5 ms with register columns but barriers every eight rows,
-// 3.7 ms so (96 % of the FP64 pipe).
+// 3.7 ms so (95 % of the FP64 pipe).
 constexpr int kOmgRows = 8, kOmgCols = 10, kOmgWarps = 2;
 
 // Columns a lane holds: as many as fit, in panels of even size.
