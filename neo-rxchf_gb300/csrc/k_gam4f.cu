@@ -282,9 +282,9 @@ constexpr int kMixChunk = 64;
 constexpr int kDpShared = 12288;   // np^2 up to this: DP staged in shared memory
 
 // G[r] = sum_p DP(p) GAM_2s[p][r]  (DP column-major, p = ip*np + jp as above);
-// two consecutive elements per thread (16-byte loads) when every row p * n4
-// stays 16-byte aligned, i.e. n4 even.
-__global__ void dp_contract_mixed_kernel(long long n4, int np, const double* __restrict__ g2s,
+// vec: two consecutive elements per thread (16-byte loads), for a 16-byte
+// aligned table whose rows p * n4 stay so, i.e. n4 even.
+__global__ void dp_contract_mixed_kernel(long long n4, int np, bool vec, const double* __restrict__ g2s,
                          const double* __restrict__ DP, double* __restrict__ G) {
   extern __shared__ float sdp[];   // [np*np] in the loop order of g2s, if staged
   const int np2 = np * np;
@@ -295,7 +295,7 @@ __global__ void dp_contract_mixed_kernel(long long n4, int np, const double* __r
       sdp[p] = tc::narrow_f64(DP[ip + np * jp]);
     }
   __syncthreads();
-  const long long nv = (n4 & 1) ? n4 : n4 / 2;
+  const long long nv = vec ? n4 / 2 : n4;
   // one item a thread: a grid-strided loop of four and a quarter rounds left
   // the last one three quarters empty
   const long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -304,7 +304,7 @@ __global__ void dp_contract_mixed_kernel(long long n4, int np, const double* __r
     for (int p0 = 0; p0 < np2; p0 += kMixChunk) {
       const int p1 = p0 + kMixChunk < np2 ? p0 + kMixChunk : np2;
       float a0 = 0.0f, a1 = 0.0f;
-      if (n4 & 1) {
+      if (!vec) {
 #pragma unroll 8
         for (int p = p0; p < p1; p++) {
           const float d = staged ? sdp[p] : tc::narrow_f64(DP[(p / np) + np * (p % np)]);
@@ -322,7 +322,7 @@ __global__ void dp_contract_mixed_kernel(long long n4, int np, const double* __r
       acc0 += (double)a0;
       acc1 += (double)a1;
     }
-    if (n4 & 1) {
+    if (!vec) {
       G[v] = acc0;
     } else {
       G[2 * v] = acc0;
@@ -1160,9 +1160,10 @@ cudaError_t launch_gam4_factored_tc(int ne, int np, const double* gee,
     return tc_gemm(in, n, n3, DE, n, n, n, n, ea, out, n, 0, err, s);
   };
   // 1. G = DP . GAM_2s (FP32 products, HBM)
-  const long long nv = (n4 & 1) ? n4 : n4 / 2;
+  const bool vec = !(n4 & 1) && !((uintptr_t)g2s & 15);
+  const long long nv = vec ? n4 / 2 : n4;
   dp_contract_mixed_kernel<<<(unsigned)((nv + 255) / 256), 256, np * np <= kDpShared ? sizeof(float) * np * np : 0, s>>>(
-      n4, np, g2s, DP, buf[0]);
+      n4, np, vec, g2s, DP, buf[0]);
   // 2. H_G, G' and H_E, E'
   TRY(last_f(buf[0], buf[1]));                                        // H_G
   pair_swap_kernel<<<tgrid, tblk, 0, s>>>((int)n2, buf[1], 0.0, buf[2]);
